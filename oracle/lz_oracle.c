@@ -126,17 +126,23 @@ void lzo_sgemm36(const float* U, const float* V, float* M, int C, int K) {
         const float* u = U + (size_t)t * C * K;
         const float* v = V + (size_t)t * C * LZO_P;
         float* m = M + (size_t)t * K * LZO_P;
-        memset(m, 0, sizeof(float) * (size_t)K * LZO_P);
-        for (int c = 0; c < C; c++) {
-            const float* vrow = v + (size_t)c * LZO_P;
-            const float* urow = u + (size_t)c * K;
-            for (int k = 0; k < K; k++) {
-                const float uk = urow[k];
-                float* mrow = m + (size_t)k * LZO_P;
-                for (int p = 0; p < LZO_P; p++) {
-                    mrow[p] += uk * vrow[p];
+        /* c ascending for every output, as a plain triple loop would add them;
+         * eight rows at a time, so that their sums stay in the nearest cache. */
+        for (int k0 = 0; k0 < K; k0 += 8) {
+            const int rows = K - k0 < 8 ? K - k0 : 8;
+            float acc[8][LZO_P];
+            memset(acc, 0, sizeof(acc));
+            for (int c = 0; c < C; c++) {
+                const float* vrow = v + (size_t)c * LZO_P;
+                const float* urow = u + (size_t)c * K + k0;
+                for (int r = 0; r < rows; r++) {
+                    const float uk = urow[r];
+                    for (int p = 0; p < LZO_P; p++) {
+                        acc[r][p] += uk * vrow[p];
+                    }
                 }
             }
+            memcpy(m + (size_t)k0 * LZO_P, acc, sizeof(float) * (size_t)rows * LZO_P);
         }
     }
 }
