@@ -435,7 +435,7 @@ __global__ void __launch_bounds__(kDcThreads, 1) conv_direct_kernel(
         }
     } else if (warp == 1) {
         // ------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = (1u << 4) | (OperandFormat<T>::value << 7) |
                                    (OperandFormat<T>::value << 10) |
                                    (static_cast<uint32_t>(Kp >> 3) << 17) |
@@ -465,8 +465,11 @@ __global__ void __launch_bounds__(kDcThreads, 1) conv_direct_kernel(
                         const uint64_t b_desc = umma_desc_sw128(b_base + stage * kBStageBytes);
 #pragma unroll
                         for (int k = 0; k < kChunkK / 16; ++k) {
-                            tcgen05_mma_f16(d_tmem, a_desc + 2u * k, b_desc + 2u * k, idesc,
-                                            (c > 0 || tap > 0 || k > 0) ? 1u : 0u);
+                            if (k == 0 && c == 0 && tap == 0) {
+                                tcgen05_mma_f16<false>(d_tmem, a_desc, b_desc, idesc);
+                            } else {
+                                tcgen05_mma_f16<true>(d_tmem, a_desc + 2u * k, b_desc + 2u * k, idesc);
+                            }
                         }
                         tcgen05_commit(bempty_bar(stage));
                         if (++stage == kBStages) { stage = 0; phase ^= 1u; }

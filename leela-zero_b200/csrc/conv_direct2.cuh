@@ -81,23 +81,25 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
         "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(leader_bar)
         : "memory");
 }
+template <bool kAccumulate>
 __device__ __forceinline__ void tcgen05_mma_f16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                                     uint32_t idesc, uint32_t accumulate) {
+                                                     uint32_t idesc) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "n"(kAccumulate ? 1 : 0)
         : "memory");
 }
-// The same with e5m2 / e4m3 operands (K = 32 per instruction: again 32 bytes of every row).
+// The same with e5m2 / e4m3 operands (K = 32 per instruction: again 32 bytes of
+// every row), always into a running accumulator.
 __device__ __forceinline__ void tcgen05_mma_f8_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                                    uint32_t idesc, uint32_t accumulate) {
+                                                    uint32_t idesc) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "n"(1)
         : "memory");
 }
 // Arrive, once the pair's MMAs issued so far have retired, on the barrier at
@@ -358,7 +360,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kDcThreads, 1) conv_
         }
     } else if (warp == 1) {
         // ------------------------------------------------ MMA issuer (leader CTA only)
-        if (lane == 0 && leader) {
+        if (leader && elect_one()) {
             const uint32_t idesc = (1u << 4) | (OperandFormat<T>::value << 7) |
                                    (OperandFormat<T>::value << 10) |
                                    (static_cast<uint32_t>(n_slice >> 3) << 17) |
@@ -386,7 +388,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kDcThreads, 1) conv_
                     if (!ok) break;
                     tcgen05_fence_after();
                     const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * kMaxN);
-                    uint32_t accum = 0u;
                     for (int c = 0; c < kchunks && ok; ++c) {
                         ok = mbar_wait(wfull_bar(wb), wphase, abort_flag, err, kErrD2MmaFull);
                         if (!ok) break;
@@ -403,14 +404,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kDcThreads, 1) conv_
                             if (f8) {
 #pragma unroll
                                 for (int k = 0; k < 4; ++k) {
-                                    tcgen05_mma_f8_pair(d_tmem, a_desc + 2u * k, b_desc + 2u * k, idesc8, 1u);
+                                    tcgen05_mma_f8_pair(d_tmem, a_desc + 2u * k, b_desc + 2u * k, idesc8);
                                 }
                             } else {
-                                tcgen05_mma_f16_pair(d_tmem, a_desc, b_desc, idesc, accum);
-                                accum = 1u;
+                                if (tap == 0 && c == 0) tcgen05_mma_f16_pair<false>(d_tmem, a_desc, b_desc, idesc);
+                                else tcgen05_mma_f16_pair<true>(d_tmem, a_desc, b_desc, idesc);
 #pragma unroll
                                 for (int k = 1; k < kChunkK / 16; ++k) {
-                                    tcgen05_mma_f16_pair(d_tmem, a_desc + 2u * k, b_desc + 2u * k, idesc, 1u);
+                                    tcgen05_mma_f16_pair<true>(d_tmem, a_desc + 2u * k, b_desc + 2u * k, idesc);
                                 }
                             }
                             tcgen05_commit_pair(bempty_bar(stage));
@@ -451,13 +452,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kDcThreads, 1) conv_
                                 if (kPlanes == 3 && c >= fchunks) {
 #pragma unroll
                                     for (int k = 0; k < 4; ++k) {
-                                        tcgen05_mma_f8_pair(d_tmem, a_desc + 2u * k, b_desc + 2u * k, idesc8, 1u);
+                                        tcgen05_mma_f8_pair(d_tmem, a_desc + 2u * k, b_desc + 2u * k, idesc8);
                                     }
                                 } else {
 #pragma unroll
                                     for (int k = 0; k < kChunkK / 16; ++k) {
-                                        tcgen05_mma_f16_pair(d_tmem, a_desc + 2u * k, b_desc + 2u * k, idesc,
-                                                             (c > 0 || tap > 0 || k > 0) ? 1u : 0u);
+                                        if (k == 0 && c == 0 && tap == 0) {
+                                            tcgen05_mma_f16_pair<false>(d_tmem, a_desc, b_desc, idesc);
+                                        } else {
+                                            tcgen05_mma_f16_pair<true>(d_tmem, a_desc + 2u * k, b_desc + 2u * k, idesc);
+                                        }
                                     }
                                 }
                             }

@@ -234,14 +234,15 @@ __global__ void __launch_bounds__(kDcThreads, 1) conv_ksplit_kernel(
         }
     } else if (warp == 1) {
         // ------------------------------------------------ MMA issuer (pair leaders)
-        if (lane == 0 && h == 0) {
+        if (h == 0 && elect_one()) {
             const uint32_t idesc = (1u << 4) | (OperandFormat<T>::value << 7) |
                                    (OperandFormat<T>::value << 10) |
                                    (static_cast<uint32_t>(Kp >> 3) << 17) |
                                    (static_cast<uint32_t>(kPairM >> 4) << 24);
             bool ok = mbar_wait(wfull_bar, 0u, abort_flag, err, kErrD3MmaFull);
-            for (int tap = 0; tap < kTaps && ok; ++tap) {
-                ok = mbar_wait(bfull_bar(tap), 0u, abort_flag, err, kErrD3MmaFull);
+#pragma unroll
+            for (int tap = 0; tap < kTaps; ++tap) {
+                ok = ok && mbar_wait(bfull_bar(tap), 0u, abort_flag, err, kErrD3MmaFull);
                 if (!ok) break;
                 tcgen05_fence_after();
                 const int row0 = kWinPad + (tap / 3 - 1) * kCellsPerRow + (tap % 3 - 1);
@@ -249,8 +250,8 @@ __global__ void __launch_bounds__(kDcThreads, 1) conv_ksplit_kernel(
                 const uint64_t b_desc = umma_desc_sw128(w_base + tap * kWStageBytes);
 #pragma unroll
                 for (int k = 0; k < kChunkK / 16; ++k) {
-                    tcgen05_mma_f16_pair(tmem_base, a_desc + 2u * k, b_desc + 2u * k, idesc,
-                                         (tap > 0 || k > 0) ? 1u : 0u);
+                    if (tap == 0 && k == 0) tcgen05_mma_f16_pair<false>(tmem_base, a_desc, b_desc, idesc);
+                    else tcgen05_mma_f16_pair<true>(tmem_base, a_desc + 2u * k, b_desc + 2u * k, idesc);
                 }
                 if (pass2) tcgen05_commit_to_pair(bempty_bar(tap), lead);
             }
@@ -260,8 +261,9 @@ __global__ void __launch_bounds__(kDcThreads, 1) conv_ksplit_kernel(
                                         (static_cast<uint32_t>(Kp >> 3) << 17) |
                                         (static_cast<uint32_t>(kPairM >> 4) << 24);
                 ok = mbar_wait(wfull2_bar, 0u, abort_flag, err, kErrD3MmaFull);
-                for (int tap = 0; tap < kTaps && ok; ++tap) {
-                    ok = mbar_wait(bfull_bar(tap), 1u, abort_flag, err, kErrD3MmaFull);
+#pragma unroll
+                for (int tap = 0; tap < kTaps; ++tap) {
+                    ok = ok && mbar_wait(bfull_bar(tap), 1u, abort_flag, err, kErrD3MmaFull);
                     if (!ok) break;
                     tcgen05_fence_after();
                     const int row0 = kWinPad + (tap / 3 - 1) * kCellsPerRow + (tap % 3 - 1);
@@ -269,7 +271,7 @@ __global__ void __launch_bounds__(kDcThreads, 1) conv_ksplit_kernel(
                     const uint64_t b_desc = umma_desc_sw128(w_base + tap * kWStageBytes);
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
-                        tcgen05_mma_f8_pair(tmem_base, a_desc + 2u * k, b_desc + 2u * k, idesc8, 1u);
+                        tcgen05_mma_f8_pair(tmem_base, a_desc + 2u * k, b_desc + 2u * k, idesc8);
                     }
                 }
             }

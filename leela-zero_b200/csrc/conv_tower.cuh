@@ -180,7 +180,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kDcThreads, 1) conv_
         }
     } else if (warp == 1) {
         // ------------------------------------------------ MMA issuer (leader CTA only)
-        if (lane == 0 && leader) {
+        if (leader && elect_one()) {
             const uint32_t idesc = (1u << 4) | (OperandFormat<T>::value << 7) |
                                    (OperandFormat<T>::value << 10) |
                                    (static_cast<uint32_t>(Kp >> 3) << 17) |
@@ -204,7 +204,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kDcThreads, 1) conv_
                     if (!ok) break;
                     tcgen05_fence_after();
                     const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * kMaxN);
-                    uint32_t accum = 0u;
                     for (int c = 0; c < kchunks && ok; ++c) {
                         ok = mbar_wait(wfull_bar(wb), wphase, abort_flag, err, kErrTowerMmaFull);
                         if (!ok) break;
@@ -221,14 +220,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kDcThreads, 1) conv_
                             if (f8) {
 #pragma unroll
                                 for (int kk = 0; kk < 4; ++kk) {
-                                    tcgen05_mma_f8_pair(d_tmem, a_desc + 2u * kk, b_desc + 2u * kk, idesc8, 1u);
+                                    tcgen05_mma_f8_pair(d_tmem, a_desc + 2u * kk, b_desc + 2u * kk, idesc8);
                                 }
                             } else {
-                                tcgen05_mma_f16_pair(d_tmem, a_desc, b_desc, idesc, accum);
-                                accum = 1u;
+                                if (tap == 0 && c == 0) tcgen05_mma_f16_pair<false>(d_tmem, a_desc, b_desc, idesc);
+                                else tcgen05_mma_f16_pair<true>(d_tmem, a_desc, b_desc, idesc);
 #pragma unroll
                                 for (int kk = 1; kk < kChunkK / 16; ++kk) {
-                                    tcgen05_mma_f16_pair(d_tmem, a_desc + 2u * kk, b_desc + 2u * kk, idesc, 1u);
+                                    tcgen05_mma_f16_pair<true>(d_tmem, a_desc + 2u * kk, b_desc + 2u * kk, idesc);
                                 }
                             }
                             tcgen05_commit_pair(bempty_bar(stage));

