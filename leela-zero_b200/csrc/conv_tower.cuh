@@ -1,22 +1,43 @@
-// The whole residual tower of a large batch in ONE launch.
+// The whole residual tower of a batch in ONE launch.
 //
-// conv_direct2.cuh runs a layer per launch; what a launch pays once (turnover
-// of the CTAs on the SMs, barrier and tensor-memory set-up, the first operands'
-// round trip, the last tile's epilogue, which nothing overlaps) is about 6 us
-// of an 87 us layer.  Here the CTA pairs stay: every pair owns the same range
-// of 256-cell tiles in every layer and walks the layers in one loop, its TMA
-// ring, its two accumulators and its epilogue pipeline running on across layer
-// boundaries.  Layers depend on each other tile by tile through the flags of
-// conv_direct2.cuh (a tile of layer l+1 reads tiles i-1, i, i+1 of layer l);
-// since the tiles that are waited for belong to other pairs of the SAME launch,
-// all pairs must be resident at once: the kernel is launched cooperatively,
-// and the host falls back to the launch-per-layer path where that is refused.
+// conv_direct2.cuh runs a layer per launch.  A launch pays once for the turnover
+// between dependent kernels, for the first operands' round trip and for the last
+// tile's epilogue: measured 7-10 us per layer, where the MMAs of one position's
+// layer take 3 us and those of 32 positions 7.  Here the CTA pairs stay and walk
+// through all layers.
 //
-// Per layer the kernel reads a TowerLayer record from global memory: the weight
-// tensor maps (used in place by the TMA unit), batch-norm vectors, which of the
-// two activation buffers it reads and writes, chunk counts and plane switches.
-// Everything else (window addressing, descriptors, epilogue arithmetic, bounded
-// waits) is that of conv_direct2_kernel's whole-tile path.
+// Work units.  A position is three row tiles of 128 cells (cells 20 .. 403 of its
+// 400-cell block: 384 rows for 361 cells); two consecutive row tiles make the
+// 256-row tile of a CTA pair, and its output channels are cut into nsplit slices
+// of N = Kp / nsplit.  Unit u of a layer is (tile u / nsplit, slice u % nsplit).
+// The units of all layers form one sequence, layer after layer, which the pairs
+// take round robin: with fewer units per layer than pairs, every unit has a pair
+// of its own; with more, a pair goes on to its next unit, of this layer or the
+// next one, without a layer boundary that everybody waits at, so that a layer of
+// 102 units costs 102 / 74 rounds and not two.
+//
+// Dependencies.  A row tile of layer l+1 reads, through its window, the row tiles
+// i-1, i, i+1 of its own position in layer l.  Every epilogue warp adds one to
+// the counter of its (layer, tile) once its stores have completed; the producer
+// that wants to load a window polls the counters of the tiles it reads.  The same
+// wait orders the writes: the rows a unit of layer l+1 overwrites were last read
+// by exactly those tiles of layer l.  Units depend only on units before them in
+// the sequence and every pair works through its own units in order, so with all
+// pairs resident (cooperative launch) the oldest unfinished unit can always run.
+//
+// Roles (12 warps): warp 0 polls the counters and loads activation windows, warp
+// 2 loads weights, which depend on nobody and so run ahead as far as the ring
+// allows (at the next layer's weights while this layer waits for its inputs),
+// warp 1 issues the MMAs, warps 4-11 are the epilogue of conv_direct2.cuh.
+//
+// What bounds it: with one or two units per pair the chain MMAs -> epilogue ->
+// stores -> counters -> windows (about 5,000 cycles besides the MMAs: 1,600 for
+// the stores to complete, 2,000 for the counter to arrive and be seen, 1,000 for
+// the first window); with more units per pair the tensor pipe, and over seconds
+// the power cap.
+//
+// Every wait is bounded; a thread that gives up sets the CTA's abort flag, all
+// roles leave their loops, tensor memory is freed and the kernel returns.
 #pragma once
 #include "conv_direct2.cuh"
 
@@ -28,14 +49,14 @@ using namespace dc;
 using namespace dc2;
 
 struct alignas(64) TowerLayer {
-    CUtensorMap tmW;            // weights [9*Kp][Cin'], box 64 x Kp/2
-    CUtensorMap tmWl;           // e5m2 weights (byte map), box 128 x Kp/2; any valid map if unused
+    CUtensorMap tmW;            // weights [9][Kp][Cin'], box 64 x N/2 x taps per stage
+    CUtensorMap tmWl;           // e5m2 weights (byte map), box 128 x N/2 x taps per stage; any valid map if unused
     const float* mean;          // batch norm, Kp entries each
     const float* invstd;
     int in_sel;                 // 0: network input cells, 1: X, 2: H
     int out_sel;                // 1: X, 2: H
-    int kchunks;                // chunks of the reduction in total (fp16 ones first, then e5m2 ones)
-    int fchunks;                // fp16 chunks among them
+    int kchunks;                // chunks of the reduction in total (16-bit ones first, then e5m2 ones)
+    int fchunks;                // 16-bit chunks among them
     int achunks;                // 64-channel chunks the activation tensor has
     int has_res;                // add X (the block's input) before the ReLU
     int res_lo;                 // the residual carries an e5m2 plane to add as well
@@ -44,39 +65,130 @@ struct alignas(64) TowerLayer {
     int pad;
 };
 
+constexpr int kTowerThreads = 384;
+constexpr int kTowerEpiWarp = 4;                        // first epilogue warp
+constexpr int kTilesPerPos128 = 3;                      // row tiles of one position
+constexpr int kTowerWins = 4;                           // activation windows in flight
+constexpr uint32_t kTowerRingBytes = 112 * 1024;        // weight ring
+constexpr int kTowerMaxStages = 14;
+constexpr uint32_t kTowerOperandBytes = kTowerWins * kWinBytes + kTowerRingBytes;
+constexpr uint32_t kTowerSmemBytes =
+    kTowerOperandBytes + 8 * kStageOutBytes + 8 * kMaxN * 4 /* bn, per warp */ + kBarBytes + 1024;
+static_assert(kTowerSmemBytes <= 227 * 1024, "shared memory of one CTA");
+constexpr int kDepRing = 8;                             // units the window loads can be ahead of the epilogue, rounded up
+constexpr unsigned long long kTileWaitLimitNs = 1000000000ull;
+
 constexpr int kErrTowerProducer = 501;
 constexpr int kErrTowerMmaAcc = 502;
 constexpr int kErrTowerMmaFull = 503;
 constexpr int kErrTowerEpilogue = 504;
-constexpr uint32_t kTowerSmemBytes = kD2SmemBytes + 2 * kMaxN * 4;   // a second set of batch-norm constants
+constexpr int kErrTowerTiles = 505;
+
+// Weight taps per ring stage for an N of n_slice channels: a stage should hold
+// some 8-16 KB, else the waits and commits around it outweigh its MMAs (a
+// 32-row half slice is 4 KB a tap: three taps, 525 cycles of MMAs).
+__host__ __device__ inline int tower_taps_per_stage(int n_slice) { return n_slice <= 64 ? 3 : 1; }
+__host__ __device__ inline int tower_stage_bytes(int n_slice) {
+    return tower_taps_per_stage(n_slice) * (n_slice / 2) * 128;
+}
+// First cell of row tile i.
+__host__ __device__ inline int tower_tile_row(int i) {
+    return (i / kTilesPerPos128) * kCellsPerPos + kCellsPerRow + (i % kTilesPerPos128) * kTileM;
+}
+
+__device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void red_release_gpu_add(uint32_t* p, uint32_t v) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2,
+                                                 uint32_t leader_bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
+        "[%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(leader_bar)
+        : "memory");
+}
+// A whole warp waits until every lane's counter (null: none) has reached target.
+__device__ __forceinline__ bool tiles_wait(const uint32_t* counter, uint32_t target, volatile int* abort_flag,
+                                           int* err) {
+    unsigned long long t0 = 0;
+    long long c0 = 0;
+    for (uint32_t spin = 0;; ++spin) {
+        const bool ready = counter == nullptr || ld_acquire_gpu(counter) >= target;
+        if (__all_sync(0xffffffffu, ready)) return true;
+        if ((spin & 63u) == 0u) {
+            if (spin == 0) {
+                t0 = globaltimer_ns();
+                c0 = clock64();
+            }
+            const bool late = globaltimer_ns() - t0 > kTileWaitLimitNs &&
+                              static_cast<unsigned long long>(clock64() - c0) > kTileWaitLimitNs;
+            if (__any_sync(0xffffffffu, late || *abort_flag != 0)) {
+                if (late) {
+                    *abort_flag = 1;
+                    atomicCAS(err, 0, kErrTowerTiles);
+                }
+                return false;
+            }
+        }
+    }
+}
+// Residual rows come from L2: this kernel's other CTAs rewrite them layer by layer.
+template <typename T>
+__device__ __forceinline__ void load_residual_l2(uint4 (&v)[4], const T* src, bool use) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        v[i] = use ? __ldcg(reinterpret_cast<const uint4*>(src) + i) : make_uint4(0u, 0u, 0u, 0u);
+    }
+}
+__device__ __forceinline__ void load_residual8_l2(uint4 (&v)[2], const unsigned char* src, bool use) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        v[i] = use ? __ldcg(reinterpret_cast<const uint4*>(src) + i) : make_uint4(0u, 0u, 0u, 0u);
+    }
+}
+// The units of one pair: g = first, first + step, ... below units * n_layers.
+struct UnitWalk {
+    int layer, u, units, step;
+    __device__ __forceinline__ UnitWalk(int first, int units_, int step_)
+        : layer(0), u(first), units(units_), step(step_) {}
+    __device__ __forceinline__ void next() {
+        u += step;
+        while (u >= units) {
+            u -= units;
+            ++layer;
+        }
+    }
+};
 
 // tmIN, tmX, tmH : activation windows (box 64 x kWinRows); tmXl, tmHl : their
 // e5m2 planes (byte maps, box 128 x kWinRows); tmXo, tmHo : output tiles (box
 // 32 x 32, 64-byte swizzle).  X, H : the two activation tensors (residual reads,
-// byte-plane stores), ldr elements of T / out_pitch bytes per cell row, q_rows
-// rows.  flags, counts : [n_layers][tile_cap] words each (conv_direct2.cuh),
-// run : the number of this tower run.
+// byte-plane stores), ldr elements of T / out_pitch bytes per cell row.  ntiles
+// row tiles (three per position), nsplit slices.  counts : [n_layers][tile_cap]
+// words, zero when the kernel starts; counts_next : the same for the next run on
+// this context, cleared here.
 template <typename T, int kPlanes>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kDcThreads, 1) conv_tower_kernel(
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTowerThreads, 1) conv_tower_kernel(
     const __grid_constant__ CUtensorMap tmIN, const __grid_constant__ CUtensorMap tmX,
     const __grid_constant__ CUtensorMap tmH, const __grid_constant__ CUtensorMap tmXl,
     const __grid_constant__ CUtensorMap tmHl, const __grid_constant__ CUtensorMap tmXo,
     const __grid_constant__ CUtensorMap tmHo, const TowerLayer* __restrict__ layers, int n_layers,
-    T* X, T* H, int Q, int Kp, int npairs, int ldr, int out_pitch, int q_rows, uint32_t* flags,
-    uint32_t* counts, int tile_cap, uint32_t run, int* err) {
+    T* X, T* H, int ntiles, int Kp, int nsplit, int ldr, int out_pitch, uint32_t* counts,
+    uint32_t* counts_next, int tile_cap, int* err) {
     extern __shared__ unsigned char smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
     unsigned char* smem = smem_raw + (base - raw);
-    constexpr int nwin = kWinBufs;
-    constexpr int nstages = kB2Stages;
     const uint32_t win_base = base;
-    const uint32_t b_base = base + static_cast<uint32_t>(nwin) * kWinBytes;
-    unsigned char* stage_out = smem + kOperand2Bytes;
-    // batch-norm constants of two layers: the epilogue may still be in layer l
-    // while nothing else is, and each warp refills the half it reads itself
-    float* s_const = reinterpret_cast<float*>(stage_out + 8 * kStageOutBytes);   // [2][scale | bias][kMaxN]
-    unsigned char* bar_mem = stage_out + 8 * kStageOutBytes + 4 * kMaxN * 4;
+    const uint32_t b_base = base + kTowerWins * kWinBytes;
+    unsigned char* stage_out = smem + kTowerOperandBytes;
+    float* s_bn = reinterpret_cast<float*>(stage_out + 8 * kStageOutBytes);      // per warp: scale[128], bias[128]
+    unsigned char* bar_mem = stage_out + 8 * kStageOutBytes + 8 * kMaxN * 4;
     const uint32_t bars = smem_u32(bar_mem);
     auto bfull_bar = [&](int s) { return bars + 8u * (0 + s); };      // leader's are used
     auto bempty_bar = [&](int s) { return bars + 8u * (16 + s); };    // both CTAs
@@ -84,19 +196,26 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kDcThreads, 1) conv_
     auto wempty_bar = [&](int w) { return bars + 8u * (36 + w); };    // both
     auto tfull_bar = [&](int a) { return bars + 8u * (40 + a); };     // both
     auto tempty_bar = [&](int a) { return bars + 8u * (42 + a); };    // leader's
-    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bar_mem + 8 * 44);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(bar_mem + 8 * 44 + 8);
+    auto dep_bar = [&](int d) { return bars + 8u * (48 + d); };       // own CTA's producer -> epilogue
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bar_mem + 8 * 56);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(bar_mem + 8 * 56 + 8);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();
     const bool leader = rank == 0;
+    const int n_slice = Kp / nsplit;          // MMA N
+    const int half_n = n_slice >> 1;          // weight rows each CTA stages per tap
+    const int tps = tower_taps_per_stage(n_slice);
+    const uint32_t stage_bytes = static_cast<uint32_t>(tower_stage_bytes(n_slice));
+    const int fit = static_cast<int>(kTowerRingBytes / stage_bytes);
+    const int nstages = fit < kTowerMaxStages ? fit : kTowerMaxStages;
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < kB2Stages; i++) {
+        for (int i = 0; i < kTowerMaxStages; i++) {
             mbar_init(bfull_bar(i), 2);      // one arrive.expect_tx per CTA of the pair
             mbar_init(bempty_bar(i), 1);
         }
-        for (int i = 0; i < nwin; i++) {
+        for (int i = 0; i < kTowerWins; i++) {
             mbar_init(wfull_bar(i), 2);
             mbar_init(wempty_bar(i), 1);
         }
@@ -104,9 +223,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kDcThreads, 1) conv_
             mbar_init(tfull_bar(a), 1);
             mbar_init(tempty_bar(a), 16);    // 8 epilogue warps in each CTA
         }
+        for (int d = 0; d < kDepRing; d++) mbar_init(dep_bar(d), 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    for (int i = blockIdx.x * kTowerThreads + threadIdx.x; i < n_layers * tile_cap; i += gridDim.x * kTowerThreads) {
+        counts_next[i] = 0u;
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -120,60 +243,91 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kDcThreads, 1) conv_
     cluster_sync_all();          // the peer's barriers are initialised before anyone signals them
     tcgen05_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    const int nclusters = gridDim.x >> 1, cid = blockIdx.x >> 1;
-    const int tile_begin = static_cast<int>(static_cast<long long>(cid) * npairs / nclusters);
-    const int tile_end = static_cast<int>(static_cast<long long>(cid + 1) * npairs / nclusters);
-    const int ntiles = tile_end - tile_begin;
-    const bool reorder = ntiles <= kMaxOrder;
-    auto tile_of = [&](int k) { return tile_begin + (reorder ? middle_out(k, ntiles) : k); };
-    const int half_n = Kp >> 1;               // weight rows each CTA stages per tap
+    const int npairs = (ntiles + 1) >> 1;
+    const int units = npairs * nsplit;
+    const int cid = blockIdx.x >> 1, step = gridDim.x >> 1;
+    // counter value of a finished tile: 8 epilogue warps in each CTA, per slice
+    const uint32_t complete = 16u * static_cast<uint32_t>(nsplit);
+    // this CTA's row tile of unit u (the last pair of an odd count works on a copy
+    // of the last tile and stores nothing)
+    auto tile_of = [&](int pair) {
+        const int t = 2 * pair + static_cast<int>(rank);
+        return t < ntiles ? t : ntiles - 1;
+    };
 
     if (warp == 0) {
-        // ------------------------------------------------ TMA producer (both CTAs)
-        if (lane == 0) {
-            int stage = 0, wb = 0;
-            uint32_t phase = 0, wphase = 0;
+        // ------------------------------------------------ activation windows (both CTAs)
+        const uint32_t lead_bars = map_to_cta(bars, 0);
+        int wb = 0, dep = 0;              // the ring position is the elected lane's
+        uint32_t wphase = 0;
+        for (UnitWalk w(cid, units, step); w.layer < n_layers; w.next()) {
+            const TowerLayer* tl = layers + w.layer;
+            const int kchunks = tl->kchunks, fchunks = tl->fchunks, achunks = tl->achunks;
+            const CUtensorMap* in_map = tl->in_sel == 0 ? &tmIN : (tl->in_sel == 1 ? &tmX : &tmH);
+            const CUtensorMap* in_lo = tl->in_sel == 2 ? &tmHl : &tmXl;
+            const int pair = w.u / nsplit;
+            const int tile = tile_of(pair);
+            if (w.layer > 0) {
+                // the tiles this window reaches: its own pair's two, and the neighbour
+                // pair's where the neighbouring row tile belongs to the same position
+                const uint32_t* row = counts + static_cast<size_t>(w.layer - 1) * tile_cap;
+                const uint32_t* mine = nullptr;
+                if (lane == 0) mine = row + pair;
+                if (lane == 1) {
+                    const int part = tile % kTilesPerPos128;
+                    const int other = part == 0 ? tile + 1 : tile - 1;          // a row tile on either side ...
+                    mine = row + (other >> 1);
+                }
+                if (lane == 2) {
+                    const int part = tile % kTilesPerPos128;
+                    const int other = part == kTilesPerPos128 - 1 ? tile - 1 : tile + 1;
+                    mine = row + (other >> 1);
+                }
+                if (!tiles_wait(mine, complete, abort_flag, err)) break;
+            }
             bool ok = true;
-            const uint32_t btx = static_cast<uint32_t>(half_n) * 128u;
-            for (int li = 0; li < n_layers && ok; ++li) {
-                const TowerLayer* tl = layers + li;
-                const int kchunks = tl->kchunks, fchunks = tl->fchunks, achunks = tl->achunks;
-                const CUtensorMap* in_map = tl->in_sel == 0 ? &tmIN : (tl->in_sel == 1 ? &tmX : &tmH);
-                const CUtensorMap* in_lo = tl->in_sel == 2 ? &tmHl : &tmXl;
-                const uint32_t* flags_in = li > 0 ? flags + static_cast<size_t>(li - 1) * tile_cap : nullptr;
-                for (int k = 0; k < ntiles && ok; ++k) {
-                    const int pair = tile_of(k);
-                    const int m0 = pair * kPairM + static_cast<int>(rank) * kTileM;
-                    const int wrow0 = static_cast<int>(rank) * half_n;
-                    if (flags_in != nullptr) {
-                        // the window of this tile reaches into the tiles on either side
-                        for (int t = pair - 1; t <= pair + 1 && ok; ++t) {
-                            if (t >= 0 && t < npairs) ok = flag_wait(flags_in + t, run, abort_flag, err);
-                        }
+            if (elect_one()) {
+                // what those tiles' epilogues stored is read below by TMA (async proxy)
+                asm volatile("fence.proxy.async;" ::: "memory");
+                mbar_arrive(dep_bar(dep));
+                const int m0 = tower_tile_row(tile);
+                for (int c = 0; c < kchunks; ++c) {
+                    ok = mbar_wait(wempty_bar(wb), wphase ^ 1u, abort_flag, err, kErrTowerProducer);
+                    if (!ok) break;
+                    const uint32_t wf = lead_bars + (wfull_bar(wb) - bars);
+                    mbar_expect_tx_cluster(wf, kWinBytes);
+                    const bool low8 = kPlanes == 3 && c >= fchunks;     // e5m2 chunk: byte coordinates
+                    tma_load_2d_pair(win_base + wb * kWinBytes, low8 ? in_lo : in_map,
+                                     low8 ? (c - fchunks) * 128 : (c < achunks ? c : c - achunks) * kChunkK,
+                                     m0 - kWinPad, wf);
+                    if (++wb == kTowerWins) { wb = 0; wphase ^= 1u; }
+                }
+            }
+            if (!__all_sync(0xffffffffu, ok)) break;
+            if (++dep == kDepRing) dep = 0;
+        }
+    } else if (warp == 2) {
+        // ------------------------------------------------ weights (both CTAs)
+        if (elect_one()) {
+            const uint32_t lead_bars = map_to_cta(bars, 0);
+            int stage = 0;
+            uint32_t phase = 0;
+            bool ok = true;
+            for (UnitWalk w(cid, units, step); w.layer < n_layers && ok; w.next()) {
+                const TowerLayer* tl = layers + w.layer;
+                const int kchunks = tl->kchunks, fchunks = tl->fchunks;
+                const int wrow0 = (w.u % nsplit) * n_slice + static_cast<int>(rank) * half_n;
+                for (int c = 0; c < kchunks && ok; ++c) {
+                    const bool low8 = kPlanes == 3 && c >= fchunks;
+                    const CUtensorMap* wmap = low8 ? &tl->tmWl : &tl->tmW;
+                    const int wcol = low8 ? (c - fchunks) * 128 : c * kChunkK;
+                    for (int tap = 0; tap < 9; tap += tps) {
+                        ok = mbar_wait(bempty_bar(stage), phase ^ 1u, abort_flag, err, kErrTowerProducer);
                         if (!ok) break;
-                        // what those tiles' epilogues stored is read below by TMA (async proxy)
-                        asm volatile("fence.proxy.async;" ::: "memory");
-                    }
-                    for (int c = 0; c < kchunks && ok; ++c) {
-                        ok = mbar_wait(wempty_bar(wb), wphase ^ 1u, abort_flag, err, kErrTowerProducer);
-                        if (!ok) break;
-                        const uint32_t wf = map_to_cta(wfull_bar(wb), 0);
-                        mbar_expect_tx_cluster(wf, kWinBytes);
-                        const bool low8 = kPlanes == 3 && c >= fchunks;     // e5m2 chunk: byte coordinates
-                        const int wcol = low8 ? (c - fchunks) * 128 : c * kChunkK;
-                        tma_load_2d_pair(win_base + wb * kWinBytes, low8 ? in_lo : in_map,
-                                         low8 ? wcol : (c < achunks ? c : c - achunks) * kChunkK,
-                                         m0 - kWinPad, wf);
-                        if (++wb == nwin) { wb = 0; wphase ^= 1u; }
-                        for (int tap = 0; tap < 9; ++tap) {
-                            ok = mbar_wait(bempty_bar(stage), phase ^ 1u, abort_flag, err, kErrTowerProducer);
-                            if (!ok) break;
-                            const uint32_t bf = map_to_cta(bfull_bar(stage), 0);
-                            mbar_expect_tx_cluster(bf, btx);
-                            tma_load_2d_pair(b_base + stage * kB2StageBytes, low8 ? &tl->tmWl : &tl->tmW, wcol,
-                                             tap * Kp + wrow0, bf);
-                            if (++stage == nstages) { stage = 0; phase ^= 1u; }
-                        }
+                        const uint32_t bf = lead_bars + 8u * static_cast<uint32_t>(stage);
+                        mbar_expect_tx_cluster(bf, stage_bytes);
+                        tma_load_3d_pair(b_base + stage * stage_bytes, wmap, wcol, wrow0, tap, bf);
+                        if (++stage == nstages) { stage = 0; phase ^= 1u; }
                     }
                 }
             }
@@ -181,89 +335,105 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kDcThreads, 1) conv_
     } else if (warp == 1) {
         // ------------------------------------------------ MMA issuer (leader CTA only)
         if (leader && elect_one()) {
-            const uint32_t idesc = (1u << 4) | (OperandFormat<T>::value << 7) |
-                                   (OperandFormat<T>::value << 10) |
-                                   (static_cast<uint32_t>(Kp >> 3) << 17) |
+            const uint32_t shape = (static_cast<uint32_t>(n_slice >> 3) << 17) |
                                    (static_cast<uint32_t>(kPairM >> 4) << 24);
+            const uint32_t idesc = (1u << 4) | (OperandFormat<T>::value << 7) | (OperandFormat<T>::value << 10) | shape;
             // e5m2 x e5m2 -> fp32 for the chunks of an e5m2 activation plane
-            const uint32_t idesc8 = (1u << 4) | (1u << 7) | (1u << 10) |
-                                    (static_cast<uint32_t>(Kp >> 3) << 17) |
-                                    (static_cast<uint32_t>(kPairM >> 4) << 24);
+            const uint32_t idesc8 = (1u << 4) | (1u << 7) | (1u << 10) | shape;
             int stage = 0, wb = 0;
             uint32_t phase = 0, wphase = 0;
             bool ok = true;
             int local = 0;
+            // descriptors are a constant plus an address in 16-byte units
             const uint64_t dbase = umma_desc_sw128(0);
             const uint32_t win16 = (win_base & 0x3FFFFu) >> 4, b16 = (b_base & 0x3FFFFu) >> 4;
-            for (int li = 0; li < n_layers && ok; ++li) {
-                const int kchunks = layers[li].kchunks, fchunks = layers[li].fchunks;
-                for (int k = 0; k < ntiles && ok; ++k, ++local) {
-                    const int acc = local & 1;
-                    const uint32_t accphase = (local >> 1) & 1u;
-                    ok = mbar_wait(tempty_bar(acc), accphase ^ 1u, abort_flag, err, kErrTowerMmaAcc);
+            const uint32_t stage16 = stage_bytes >> 4, tap16 = static_cast<uint32_t>(half_n) * 8u;
+            for (UnitWalk w(cid, units, step); w.layer < n_layers && ok; w.next(), ++local) {
+                const int kchunks = layers[w.layer].kchunks, fchunks = layers[w.layer].fchunks;
+                const int acc = local & 1;
+                ok = mbar_wait(tempty_bar(acc), ((local >> 1) & 1u) ^ 1u, abort_flag, err, kErrTowerMmaAcc);
+                if (!ok) break;
+                tcgen05_fence_after();
+                const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * kMaxN);
+                for (int c = 0; c < kchunks && ok; ++c) {
+                    ok = mbar_wait(wfull_bar(wb), wphase, abort_flag, err, kErrTowerMmaFull);
                     if (!ok) break;
-                    tcgen05_fence_after();
-                    const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * kMaxN);
-                    for (int c = 0; c < kchunks && ok; ++c) {
-                        ok = mbar_wait(wfull_bar(wb), wphase, abort_flag, err, kErrTowerMmaFull);
-                        if (!ok) break;
-                        const uint64_t a_win = dbase + (win16 + static_cast<uint32_t>(wb) * (kWinBytes >> 4));
-                        const bool f8 = kPlanes == 3 && c >= fchunks;
+                    const uint64_t a_win = dbase + (win16 + static_cast<uint32_t>(wb) * (kWinBytes >> 4));
+                    const bool f8 = kPlanes == 3 && c >= fchunks;
+                    uint64_t b_desc = 0;
+                    int left = 0;                    // taps left in the current stage
 #pragma unroll
-                        for (int tap = 0; tap < 9; ++tap) {
+                    for (int tap = 0; tap < 9; ++tap) {
+                        if (left == 0) {
                             ok = mbar_wait(bfull_bar(stage), phase, abort_flag, err, kErrTowerMmaFull);
                             if (!ok) break;
-                            // rows (24 + 20 dy + dx) .. of the window, 8 sixteen-byte units each
-                            const uint64_t a_desc =
-                                a_win + static_cast<uint32_t>((kWinPad + (tap / 3 - 1) * kCellsPerRow + (tap % 3 - 1)) * 8);
-                            const uint64_t b_desc = dbase + (b16 + static_cast<uint32_t>(stage) * (kB2StageBytes >> 4));
-                            if (f8) {
+                            tcgen05_fence_after();
+                            b_desc = dbase + (b16 + static_cast<uint32_t>(stage) * stage16);
+                            left = tps;
+                        }
+                        // rows (24 + 20 dy + dx) .. of the window, 8 sixteen-byte units each
+                        const uint64_t a_desc =
+                            a_win + static_cast<uint32_t>((kWinPad + (tap / 3 - 1) * kCellsPerRow + (tap % 3 - 1)) * 8);
+                        if (f8) {
 #pragma unroll
-                                for (int kk = 0; kk < 4; ++kk) {
-                                    tcgen05_mma_f8_pair(d_tmem, a_desc + 2u * kk, b_desc + 2u * kk, idesc8);
-                                }
-                            } else {
-                                if (tap == 0 && c == 0) tcgen05_mma_f16_pair<false>(d_tmem, a_desc, b_desc, idesc);
-                                else tcgen05_mma_f16_pair<true>(d_tmem, a_desc, b_desc, idesc);
-#pragma unroll
-                                for (int kk = 1; kk < kChunkK / 16; ++kk) {
-                                    tcgen05_mma_f16_pair<true>(d_tmem, a_desc + 2u * kk, b_desc + 2u * kk, idesc);
-                                }
+                            for (int k = 0; k < 4; ++k) {
+                                tcgen05_mma_f8_pair(d_tmem, a_desc + 2u * k, b_desc + 2u * k, idesc8);
                             }
+                        } else {
+                            if (tap == 0 && c == 0) tcgen05_mma_f16_pair<false>(d_tmem, a_desc, b_desc, idesc);
+                            else tcgen05_mma_f16_pair<true>(d_tmem, a_desc, b_desc, idesc);
+#pragma unroll
+                            for (int k = 1; k < kChunkK / 16; ++k) {
+                                tcgen05_mma_f16_pair<true>(d_tmem, a_desc + 2u * k, b_desc + 2u * k, idesc);
+                            }
+                        }
+                        b_desc += tap16;
+                        if (--left == 0) {
                             tcgen05_commit_pair(bempty_bar(stage));
                             if (++stage == nstages) { stage = 0; phase ^= 1u; }
                         }
-                        if (!ok) break;
-                        tcgen05_commit_pair(wempty_bar(wb));
-                        if (++wb == nwin) { wb = 0; wphase ^= 1u; }
                     }
                     if (!ok) break;
-                    tcgen05_commit_pair(tfull_bar(acc));
+                    tcgen05_commit_pair(wempty_bar(wb));
+                    if (++wb == kTowerWins) { wb = 0; wphase ^= 1u; }
                 }
+                if (!ok) break;
+                tcgen05_commit_pair(tfull_bar(acc));
             }
         }
-    } else {
-        // ------------------------------------------------ epilogue (warps 2..9, both CTAs)
-        const int qd = warp & 3;
-        const int ncols = Kp >> 1;               // channels this warp converts per tile
-        const int wcol = ((warp - 2) >> 2) * ncols;
-        unsigned char* stg_ptr = stage_out + (warp - 2) * kStageOutBytes;
+    } else if (warp >= kTowerEpiWarp) {
+        // ------------------------------------------------ epilogue (warps 4..11, both CTAs)
+        const int ew = warp - kTowerEpiWarp;
+        const int qd = warp & 3;                 // tensor-memory lane quadrant
+        const int ncols = n_slice >> 1;          // channels this warp converts per unit
+        const int wcol = (ew >> 2) * ncols;
+        unsigned char* stg_ptr = stage_out + ew * kStageOutBytes;
         const uint32_t stg = smem_u32(stg_ptr);
         unsigned char* stg_row = stg_ptr + lane * 64;
-        int local = 0;
-        bool alive = true;
-        for (int li = 0; li < n_layers && alive; ++li) {
-            const TowerLayer* tl = layers + li;
-            // this warp's half of the layer's batch-norm constants (four warps write
-            // the same values into the same half; each reads back what it wrote)
-            float* s_scale = s_const + (li & 1) * 2 * kMaxN;
-            float* s_bias = s_scale + kMaxN;
-            for (int i = wcol + lane; i < wcol + ncols; i += 32) {
-                const float is = tl->invstd[i];
-                s_scale[i] = is;
-                s_bias[i] = -tl->mean[i] * is;
+        float* s_scale = s_bn + ew * 2 * (kMaxN / 2);
+        float* s_bias = s_scale + kMaxN / 2;
+        int local = 0, dep = 0, bn_layer = -1, bn_col = -1;
+        uint32_t dphase = 0;
+        for (UnitWalk w(cid, units, step); w.layer < n_layers; w.next(), ++local) {
+            const TowerLayer* tl = layers + w.layer;
+            const int pair = w.u / nsplit;
+            const bool live = 2 * pair + static_cast<int>(rank) < ntiles;
+            const int col0 = (w.u % nsplit) * n_slice + wcol;      // first output channel of this warp
+            const int acc = local & 1;
+            const int row0 = tower_tile_row(tile_of(pair)) + qd * 32;
+            const int q = row0 + lane;
+            const bool interior = q % kCellsPerRow != 0 && (q / kCellsPerRow) % 20 != 0;
+            // batch-norm constants of this warp's channels, before anything is waited for
+            if (bn_layer != w.layer || bn_col != col0) {
+                for (int i = lane; i < ncols; i += 32) {
+                    const float is = tl->invstd[col0 + i];
+                    s_scale[i] = is;
+                    s_bias[i] = -tl->mean[col0 + i] * is;
+                }
+                bn_layer = w.layer;
+                bn_col = col0;
+                __syncwarp();
             }
-            __syncwarp();
             const CUtensorMap* out_map = tl->out_sel == 1 ? &tmXo : &tmHo;
             T* out_base = tl->out_sel == 1 ? X : H;
             const T* res = tl->has_res ? X : nullptr;
@@ -273,93 +443,98 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kDcThreads, 1) conv_
             unsigned char* out_hi8 = tl->out_hi8 ? reinterpret_cast<unsigned char*>(out_base) +
                                                        static_cast<size_t>(Kp) * (sizeof(T) + 1)
                                                  : nullptr;
-            uint32_t* flags_out = flags + static_cast<size_t>(li) * tile_cap;
-            uint32_t* counts_out = counts + static_cast<size_t>(li) * tile_cap;
-            for (int k = 0; k < ntiles; ++k, ++local) {
-                const int pair = tile_of(k);
-                const int col0 = wcol;                      // first output channel of this warp
-                const int acc = local & 1;
-                const uint32_t accphase = (local >> 1) & 1u;
-                const int row0 = pair * kPairM + static_cast<int>(rank) * kTileM + qd * 32;
-                const int q = row0 + lane;
-                const bool interior = cell_is_interior(q, Q);
-                // one lane polls, the others sleep at the warp barrier
-                bool ok = true;
-                if (lane == 0) ok = mbar_wait(tfull_bar(acc), accphase, abort_flag, err, kErrTowerEpilogue);
-                ok = __shfl_sync(0xffffffffu, ok, 0);
-                if (!ok) { alive = false; break; }
-                tcgen05_fence_after();
-                const bool use_res = (res != nullptr) && interior;
-                constexpr bool e5 = kPlanes == 3;
-                const T* rrow = res + static_cast<size_t>(q) * ldr + col0;
-                // e5m2 plane of the same row: Kp bytes after the Kp 16-bit channels
-                const unsigned char* erow =
-                    reinterpret_cast<const unsigned char*>(res + static_cast<size_t>(q) * ldr + Kp) + col0;
-                const uint32_t taddr0 = tmem_base + (static_cast<uint32_t>(qd * 32) << 16) +
-                                        static_cast<uint32_t>(acc * kMaxN + wcol);
-                uint32_t ra[32], rb[32];
-                uint4 va[4], vb[4], ea[2], eb[2];
-                auto emit = [&](const uint32_t (&r)[32], const uint4 (&v)[4], const uint4 (&e)[2], int col) {
+            constexpr bool two = kPlanes == 2;
+            constexpr bool e5 = kPlanes == 3;
+            const bool use_res = (res != nullptr) && interior && live;
+            const T* rrow = res + static_cast<size_t>(q) * ldr + col0;
+            // e5m2 plane of the same row: Kp bytes after the Kp 16-bit channels
+            const unsigned char* erow =
+                reinterpret_cast<const unsigned char*>(res + static_cast<size_t>(q) * ldr + Kp) + col0;
+            uint32_t ra[32], rb[32];
+            uint4 va[4], vb[4], la[4], lb[4], ea[2], eb[2];
+            // the residual is final once this unit's inputs are: fetch it behind the MMAs
+            bool ok = true;
+            if (lane == 0) ok = mbar_wait(dep_bar(dep), dphase, abort_flag, err, kErrTowerEpilogue);
+            ok = __shfl_sync(0xffffffffu, ok, 0);
+            if (!ok) break;
+            if (++dep == kDepRing) { dep = 0; dphase ^= 1u; }
+            load_residual_l2(va, rrow, use_res);
+            if constexpr (two) load_residual_l2(la, rrow + Kp, use_res);
+            if constexpr (e5) load_residual8_l2(ea, erow, use_res && res_lo);
+            // one lane polls, the others sleep at the warp barrier
+            if (lane == 0) ok = mbar_wait(tfull_bar(acc), (local >> 1) & 1u, abort_flag, err, kErrTowerEpilogue);
+            ok = __shfl_sync(0xffffffffu, ok, 0);
+            if (!ok) break;
+            tcgen05_fence_after();
+            const uint32_t taddr0 =
+                tmem_base + (static_cast<uint32_t>(qd * 32) << 16) + static_cast<uint32_t>(acc * kMaxN + wcol);
+            // batch-norm etc. of the 32-channel chunk at column j of this warp, and its store(s)
+            auto emit = [&](const uint32_t (&r)[32], const uint4 (&v)[4], const uint4 (&l)[4],
+                            const uint4 (&e)[2], int j) {
+                const int col = col0 + j;
+                wait_staged_tile_read(lane);
+                if constexpr (e5) {
+                    uint32_t lo[8], h8[8];
+                    epilogue_chunk_e5m2<T>(r, v, e, s_scale + j, s_bias + j, use_res, interior, stg_row, lane,
+                                           lo, h8, out_hi8 != nullptr);
+                    if (live) {
+                        store_staged_tile(out_map, stg, col, row0, lane);
+                        const size_t off = static_cast<size_t>(q) * out_pitch + col;
+                        if (out_lo != nullptr) {
+                            uint4* dst = reinterpret_cast<uint4*>(out_lo + off);
+                            dst[0] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                            dst[1] = make_uint4(lo[4], lo[5], lo[6], lo[7]);
+                        }
+                        if (out_hi8 != nullptr) {
+                            uint4* dst = reinterpret_cast<uint4*>(out_hi8 + off);
+                            dst[0] = make_uint4(h8[0], h8[1], h8[2], h8[3]);
+                            dst[1] = make_uint4(h8[4], h8[5], h8[6], h8[7]);
+                        }
+                    }
+                } else if constexpr (!two) {
+                    epilogue_chunk<T>(r, v, s_scale + j, s_bias + j, use_res, interior, stg_row, lane);
+                    if (live) store_staged_tile(out_map, stg, col, row0, lane);
+                } else {
+                    uint32_t lo[16];
+                    epilogue_chunk_x2<T>(r, v, l, s_scale + j, s_bias + j, use_res, interior, stg_row, lane, lo);
+                    if (live) store_staged_tile(out_map, stg, col, row0, lane);
                     wait_staged_tile_read(lane);
-                    if constexpr (e5) {
-                        uint32_t lo[8], h8[8];
-                        epilogue_chunk_e5m2<T>(r, v, e, s_scale + col, s_bias + col, use_res, interior, stg_row,
-                                               lane, lo, h8, out_hi8 != nullptr);
-                        store_staged_tile(out_map, stg, col, row0, lane);
-                        if (q < q_rows) {
-                            const size_t off = static_cast<size_t>(q) * out_pitch + col;
-                            if (out_lo != nullptr) {
-                                uint4* dst = reinterpret_cast<uint4*>(out_lo + off);
-                                dst[0] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-                                dst[1] = make_uint4(lo[4], lo[5], lo[6], lo[7]);
-                            }
-                            if (out_hi8 != nullptr) {
-                                uint4* dst = reinterpret_cast<uint4*>(out_hi8 + off);
-                                dst[0] = make_uint4(h8[0], h8[1], h8[2], h8[3]);
-                                dst[1] = make_uint4(h8[4], h8[5], h8[6], h8[7]);
-                            }
-                        }
-                    } else {
-                        epilogue_chunk<T>(r, v, s_scale + col, s_bias + col, use_res, interior, stg_row, lane);
-                        store_staged_tile(out_map, stg, col, row0, lane);
-                    }
-                };
-                load_residual(va, rrow, use_res);
-                if constexpr (e5) load_residual8(ea, erow, use_res && res_lo);
-                LZB_TMEM_LD32(ra, taddr0);
-                for (int j = 0; j < ncols; j += 64) {
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    const bool more = j + 32 < ncols;
-                    if (more) {
-                        load_residual(vb, rrow + j + 32, use_res);
-                        if constexpr (e5) load_residual8(eb, erow + j + 32, use_res && res_lo);
-                        LZB_TMEM_LD32(rb, taddr0 + j + 32);
-                    }
-                    emit(ra, va, ea, col0 + j);
-                    if (more) {
-                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                        if (j + 64 < ncols) {
-                            load_residual(va, rrow + j + 64, use_res);
-                            if constexpr (e5) load_residual8(ea, erow + j + 64, use_res && res_lo);
-                            LZB_TMEM_LD32(ra, taddr0 + j + 64);
-                        }
-                        emit(rb, vb, eb, col0 + j + 32);
-                    }
+                    stage_low_plane(lo, stg_row, lane);
+                    if (live) store_staged_tile(out_map, stg, Kp + col, row0, lane);
                 }
-                tcgen05_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(map_to_cta(tempty_bar(acc), 0));
-                // this warp's part of the tile is in memory: its TMA stores have
-                // completed, its lanes' direct stores are fenced; then count it
-                if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-                __threadfence();
-                __syncwarp();
-                if (lane == 0) {
-                    asm volatile("fence.proxy.async;" ::: "memory");
-                    const uint32_t before = atom_acq_rel_gpu_add(counts_out + pair, 1u);
-                    if ((before & (kFlagArrivals - 1u)) == kFlagArrivals - 1u) st_release_gpu(flags_out + pair, run);
+            };
+            LZB_TMEM_LD32(ra, taddr0);
+            for (int j = 0; j < ncols; j += 64) {
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                const bool more = j + 32 < ncols;
+                if (more) {
+                    load_residual_l2(vb, rrow + j + 32, use_res);
+                    if constexpr (two) load_residual_l2(lb, rrow + Kp + j + 32, use_res);
+                    if constexpr (e5) load_residual8_l2(eb, erow + j + 32, use_res && res_lo);
+                    LZB_TMEM_LD32(rb, taddr0 + j + 32);
+                }
+                emit(ra, va, la, ea, j);
+                if (more) {
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if (j + 64 < ncols) {
+                        load_residual_l2(va, rrow + j + 64, use_res);
+                        if constexpr (two) load_residual_l2(la, rrow + Kp + j + 64, use_res);
+                        if constexpr (e5) load_residual8_l2(ea, erow + j + 64, use_res && res_lo);
+                        LZB_TMEM_LD32(ra, taddr0 + j + 64);
+                    }
+                    emit(rb, vb, lb, eb, j + 32);
                 }
             }
+            tcgen05_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(map_to_cta(tempty_bar(acc), 0));
+            // this warp's part of the tile is in memory: its TMA stores have completed,
+            // its lanes' byte-plane stores are handed to the async proxy; the release
+            // covers what the other lanes stored before the warp barrier
+            if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+            asm volatile("fence.proxy.async;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) red_release_gpu_add(counts + static_cast<size_t>(w.layer) * tile_cap + pair, 1u);
         }
         if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     }

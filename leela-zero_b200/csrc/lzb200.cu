@@ -18,8 +18,8 @@
 
 #include <cstdio>
 #include <cstdlib>
+#include <algorithm>
 #include <atomic>
-#include <chrono>
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -28,7 +28,6 @@
 
 #include "conv_direct.cuh"
 #include "conv_direct2.cuh"
-#include "conv_direct3.cuh"
 #include "conv_tower.cuh"
 #include "gemm_simt.cuh"
 #include "gemm_tcgen05.cuh"
@@ -118,6 +117,31 @@ int make_map_2d(CUtensorMap* map, int precision, void* base, uint64_t rows, uint
     return LZB_OK;
 }
 
+// 3-D map over weights [9 taps][rows][cols] of 16-bit elements (precision < 0:
+// bytes), box box_cols x box_rows x box_taps under the 128-byte swizzle: the rows
+// of several taps in one load.
+int make_weight_map(CUtensorMap* map, int precision, void* base, uint64_t rows, uint64_t cols, uint32_t box_cols,
+                    uint32_t box_rows, uint32_t box_taps) {
+    EncodeTiledFn fn = encode_tiled_fn();
+    if (!fn) return fail(LZB_ERR_CUDA, "cuTensorMapEncodeTiled entry point not available");
+    const uint64_t elt = precision < 0 ? 1 : 2;
+    const cuuint64_t dims[3] = {cols, rows, 9};
+    const cuuint64_t strides[2] = {cols * elt, cols * rows * elt};
+    const cuuint32_t box[3] = {box_cols, box_rows, box_taps};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    const CUtensorMapDataType dt =
+        precision < 0 ? CU_TENSOR_MAP_DATA_TYPE_UINT8
+                      : (precision == LZB_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
+                                               : CU_TENSOR_MAP_DATA_TYPE_FLOAT16);
+    CUresult r = fn(map, dt, 3, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) {
+        return fail(LZB_ERR_CUDA, "cuTensorMapEncodeTiled failed with code " + std::to_string((int)r));
+    }
+    return LZB_OK;
+}
+
 struct Layer {
     void* U = nullptr;          // [36][Kp][cin_p] storage type
     float* mean = nullptr;      // [Kp]
@@ -171,18 +195,13 @@ struct lzb_pipe {
     bool wsplit = false;        // weights carried as hi + lo planes as well (LZB_FP16_X3)
     int elt = 2;        // bytes per stored element
     int sm_count = 0;
-    // Reduction-split kernel (conv_direct3.cuh): most tiles one launch may have
-    // (clusters of 2 * chunks CTAs that can be resident at once), per chunk
-    // count 2..4; 0 = not used.
-    int ksplit_max_tiles[5] = {0, 0, 0, 0, 0};
     std::vector<Layer> layers;
-    // per-layer records of the one-launch tower kernel (conv_tower.cuh), on the
-    // device; null where that kernel does not apply
-    lzb::dct::TowerLayer* tower_table = nullptr;
-    bool tower_refused = false;         // a cooperative launch of it failed once: not tried again
-    // contexts on this pipe (their streams are asked whether they are busy)
-    std::mutex ctx_mutex;
-    std::vector<lzb_ctx*> contexts;
+    // One-launch tower (conv_tower.cuh): per-layer records on the device for each
+    // number of channel slices (null: not a valid one), and how many CTA pairs of
+    // the kernel are resident at once (0: not used).
+    lzb::dct::TowerLayer* tower_table[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
+    int tower_pairs = 0;
+    std::atomic<bool> tower_refused{false};      // a cooperative launch of it failed once: not tried again
     float* head_w = nullptr;   // [3][Cp] fp32
     bool head_convs = false;
     bool finalized = false;
@@ -200,15 +219,11 @@ struct lzb_ctx {
     float *d_in = nullptr, *d_pol = nullptr, *d_val = nullptr;
     float *d_policy = nullptr, *d_winrate = nullptr;
     unsigned int* d_packed = nullptr;   // bit-packed input planes [max_batch][18][12]
-    // per-tile completion words of the direct path, [2][layers][tile_cap] (the run
-    // that completed a tile last, then the arrival counters), and the number of
-    // tower runs so far (see conv_direct2.cuh); null: not used
-    uint32_t* tile_flags = nullptr;
+    // One-launch tower: arrival counters of the tiles, two sets of [layers][tile_cap]
+    // words used in turn (a run clears the other set); null: a launch per layer
+    uint32_t* tile_counts = nullptr;
     int tile_cap = 0;
     uint32_t tower_runs = 0;
-    bool tile_flags_always = false;     // asked for by LZB_TILE_FLAGS=1: also while other contexts are busy
-    bool tower_kernel = false;          // LZB_TOWER_KERNEL=1: all layers of a large batch in one launch
-    std::atomic<long long> last_tower_ns{0};   // when this context last enqueued a tower (steady clock)
     int* d_err = nullptr;
     int* h_err = nullptr;  // pinned
     CUtensorMap tmV_first, tmV;
@@ -423,55 +438,13 @@ int run_tower(lzb_ctx* c, const float* in_dev, int nb, float* pol_dev, float* va
 template <typename T>
 int launch_conv_direct(lzb_ctx* c, const Layer& L, int nb, const CUtensorMap& tm_in,
                        const CUtensorMap& tm_out, const T* res, const CUtensorMap* tm_in_lo = nullptr,
-                       void* out = nullptr, const uint32_t* flags_in = nullptr,
-                       uint32_t* flags_out = nullptr, uint32_t* counts_out = nullptr,
-                       uint32_t flag_target = 0) {
+                       void* out = nullptr) {
     lzb_pipe* p = c->pipe;
     const int Q = static_cast<int>(dc::cells_for(nb));
     if (p->pairs) {
         const int npairs = (Q + dc2::kPairM - 1) / dc2::kPairM;
         const int max_clusters = p->sm_count / 2;
-        // Few tiles (small batches) and a tower layer: split the reduction of
-        // each tile over the pairs of one cluster.
         const int kchunks = L.cinw / tc::kChunkK;
-        if ((p->aplanes == 1 || p->aplanes == 3) && kchunks >= 2 && kchunks <= dc3::kMaxSplit &&
-            p->Cp == kchunks * dc3::kGroupCols && L.lchunks <= kchunks && npairs <= p->ksplit_max_tiles[kchunks]) {
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(npairs * 2 * kchunks);
-            cfg.blockDim = dim3(dc::kDcThreads);
-            cfg.dynamicSmemBytes = dc3::kD3SmemBytes;
-            cfg.stream = c->stream;
-            cudaLaunchAttribute attr[2];
-            attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-            attr[0].val.programmaticStreamSerializationAllowed = 1;
-            attr[1].id = cudaLaunchAttributeClusterDimension;
-            attr[1].val.clusterDim.x = 2 * kchunks;
-            attr[1].val.clusterDim.y = 1;
-            attr[1].val.clusterDim.z = 1;
-            cfg.attrs = attr;
-            cfg.numAttrs = 2;
-            cudaError_t le;
-            {
-                LaunchScope scope(c, kClassContraction);
-                auto kernel = dc3::conv_ksplit_kernel<T, 1>;
-                if constexpr (std::is_same<T, __half>::value) {     // the two-plane mode is fp16 only
-                    if (p->aplanes == 3 && (L.out_lo || L.lchunks > 0)) kernel = dc3::conv_ksplit_kernel<T, 3>;
-                }
-                const CUtensorMap& in_lo = tm_in_lo ? *tm_in_lo : tm_in;
-                const CUtensorMap& w_lo = L.Wd8 ? L.tmW8[1] : L.tmW2[1];
-                unsigned char* out_lo =
-                    (L.out_lo && out) ? static_cast<unsigned char*>(out) + (size_t)p->Cp * p->elt : nullptr;
-                unsigned char* out_hi8 =
-                    (L.out_hi8 && out) ? static_cast<unsigned char*>(out) + (size_t)p->Cp * (p->elt + 1) : nullptr;
-                le = cudaLaunchKernelEx(&cfg, kernel, tm_in, L.tmW2[1], tm_out, res,
-                                        (const float*)L.mean, (const float*)L.invstd, Q, p->Cp, kchunks,
-                                        c->d_err, in_lo, w_lo, L.lchunks, p->row_bytes() / p->elt, out_lo,
-                                        out_hi8, p->row_bytes(), c->Qa, L.achunks);
-            }
-            LZB_CUDA(le);
-            LZB_CUDA(cudaGetLastError());
-            return LZB_OK;
-        }
         // Small batches: cut the output channels of each tile into slices so that
         // the layer spreads over more SMs (one slice per CTA pair).
         int nsplit = 1;
@@ -520,9 +493,7 @@ int launch_conv_direct(lzb_ctx* c, const Layer& L, int nb, const CUtensorMap& tm
             le = cudaLaunchKernelEx(&cfg, kernel, tm_in, L.tmW2[nsplit], tm_out, res,
                                     (const float*)L.mean, (const float*)L.invstd, Q, p->Cp,
                                     kchunks + L.lchunks, npairs, nsplit, c->d_err, L.achunks, in_lo, w_lo,
-                                    ldr, out_lo, p->row_bytes(), c->Qa, kchunks, out_hi8,
-                                    nsplit == 1 ? flags_in : nullptr, nsplit == 1 ? flags_out : nullptr,
-                                    counts_out, flag_target);
+                                    ldr, out_lo, p->row_bytes(), c->Qa, kchunks, out_hi8);
         }
         LZB_CUDA(le);
         LZB_CUDA(cudaGetLastError());
@@ -541,8 +512,78 @@ int launch_conv_direct(lzb_ctx* c, const Layer& L, int nb, const CUtensorMap& tm
     return LZB_OK;
 }
 
-// One micro-batch through the tower, direct (implicit GEMM) path: one launch
-// per 3x3 layer, batch-norm / residual / ReLU in its epilogue.
+// Channel slices of a tile in the one-launch tower.  An MMA of 256 x N x 16 takes
+// 44, 65, 97, 129 cycles at N = 64, 128, 192, 256 (measured), so slices shorten a
+// unit less than they multiply their number: with units to spare they pay only
+// while pairs are idle.  Cost of a layer in cycles: one unit's MMAs plus the chain
+// between layers (some 5,000 cycles), or the pairs' share of all units' MMAs,
+// whichever is longer; the fewest slices within 3 % of the best, since every
+// slice loads the activation windows again.
+int tower_slices(const lzb_pipe* p, int npairs) {
+    auto mma_cycles = [](int n) { return n <= 64 ? 44.0 : n * 0.5 + 1.0; };
+    const double mmas = 36.0 * p->layers.back().cinw / tc::kChunkK;
+    double cost[5] = {0, 0, 0, 0, 0}, best = 1e30;
+    for (int ns = 1; ns <= 4; ns++) {
+        if (p->tower_table[ns] == nullptr) continue;
+        const double unit = mmas * mma_cycles(p->Cp / ns);
+        cost[ns] = std::max(unit + 5000.0, unit * npairs * ns / p->tower_pairs);
+        best = std::min(best, cost[ns]);
+    }
+    for (int ns = 1; ns <= 4; ns++) {
+        if (p->tower_table[ns] != nullptr && cost[ns] <= 1.03 * best) return ns;
+    }
+    return 1;
+}
+
+// All 3x3 layers of one micro-batch in one cooperative launch.  A launch that is
+// refused is reported in *refused and not an error.
+template <typename T>
+int launch_tower(lzb_ctx* c, int nb, bool* refused) {
+    lzb_pipe* p = c->pipe;
+    const int ntiles = dct::kTilesPerPos128 * nb, npairs = (ntiles + 1) / 2;
+    const int ns = tower_slices(p, npairs);
+    const int n_layers = static_cast<int>(p->layers.size());
+    const size_t words = static_cast<size_t>(n_layers) * c->tile_cap;
+    uint32_t* counts = c->tile_counts + (c->tower_runs & 1u) * words;
+    uint32_t* counts_next = c->tile_counts + ((c->tower_runs & 1u) ^ 1u) * words;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * std::min(npairs * ns, p->tower_pairs));
+    cfg.blockDim = dim3(dct::kTowerThreads);
+    cfg.dynamicSmemBytes = dct::kTowerSmemBytes;
+    cfg.stream = c->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    auto kernel = dct::conv_tower_kernel<T, 1>;
+    if (p->aplanes == 2) kernel = dct::conv_tower_kernel<T, 2>;
+    if constexpr (std::is_same<T, __half>::value) {     // the e5m2 planes accompany fp16 only
+        if (p->aplanes == 3) kernel = dct::conv_tower_kernel<T, 3>;
+    }
+    const bool bytes = p->aplanes == 3;
+    LaunchScope scope(c, kClassContraction, n_layers);
+    cudaError_t le = cudaLaunchKernelEx(
+        &cfg, kernel, c->tmIN, c->tmX, c->tmH, bytes ? c->tmXl : c->tmX, bytes ? c->tmHl : c->tmH, c->tmXo, c->tmHo,
+        (const dct::TowerLayer*)p->tower_table[ns], n_layers, static_cast<T*>(c->X), static_cast<T*>(c->H), ntiles,
+        p->Cp, ns, p->row_bytes() / p->elt, p->row_bytes(), counts, counts_next, c->tile_cap, c->d_err);
+    if (le == cudaSuccess) le = cudaGetLastError();
+    *refused = le != cudaSuccess;
+    if (*refused) {
+        // e.g. cooperative launches with clusters not available: keep to a launch per layer
+        (void)cudaGetLastError();
+        p->tower_refused = true;
+        c->launches--;
+    } else {
+        c->tower_runs++;
+    }
+    return LZB_OK;
+}
+
+// One micro-batch through the tower, direct (implicit GEMM) path: all 3x3 layers
+// in one launch, or, where the caller wants layers timed one by one
+// (lzb_ctx_profile_begin) or the one launch is not available, a launch per layer;
+// batch-norm / residual / ReLU in the epilogue either way.
 template <typename T>
 int run_tower_direct(lzb_ctx* c, const float* in_dev, int nb, float* pol_dev, float* val_dev) {
     lzb_pipe* p = c->pipe;
@@ -554,98 +595,18 @@ int run_tower_direct(lzb_ctx* c, const float* in_dev, int nb, float* pol_dev, fl
             in_dev, static_cast<T*>(c->IN), nb);
     }
     LZB_CUDA(cudaGetLastError());
-    // Per-tile dependencies between the layers (conv_direct2.cuh) where every
-    // layer of this batch runs whole tiles on CTA pairs: more tiles than half the
-    // pairs, so that neither the channel slices nor the reduction-split kernel apply.
-    const int npairs = (static_cast<int>(dc::cells_for(nb)) + dc2::kPairM - 1) / dc2::kPairM;
-    bool flags = c->tile_flags != nullptr && p->pairs && npairs <= c->tile_cap &&
-                 2 * npairs > p->sm_count / 2;
-    const long long now_ns = std::chrono::duration_cast<std::chrono::nanoseconds>(
-                                 std::chrono::steady_clock::now().time_since_epoch()).count();
-    if (flags && !c->tile_flags_always) {
-        // A launch that waits tile by tile holds its SMs while it waits.  Alone on
-        // the GPU that hides the turnover between layers (-4 % per step); beside
-        // another context's tower, whose launches would have filled those gaps
-        // anyway, it costs 4 %.  So: only while no other context of this pipe is at
-        // work, i.e. none has work in flight or has enqueued a tower in the last 100 ms.
-        std::lock_guard<std::mutex> lk(p->ctx_mutex);
-        for (lzb_ctx* other : p->contexts) {
-            if (other == c || other->stream == nullptr) continue;
-            if (now_ns - other->last_tower_ns.load(std::memory_order_relaxed) < 100000000ll ||
-                cudaStreamQuery(other->stream) == cudaErrorNotReady) {
-                flags = false;
-                break;
+    bool per_layer = c->tile_counts == nullptr || p->tower_refused || c->profiling;
+    if (!per_layer && (rc = launch_tower<T>(c, nb, &per_layer))) return rc;
+    if (per_layer) {
+        if ((rc = launch_conv_direct<T>(c, p->layers[0], nb, c->tmIN, c->tmXo, nullptr, nullptr, c->X))) return rc;
+        for (int b = 0; b < p->blocks; b++) {
+            if ((rc = launch_conv_direct<T>(c, p->layers[1 + 2 * b], nb, c->tmX, c->tmHo, nullptr, &c->tmXl,
+                                            c->H))) {
+                return rc;
             }
-        }
-        (void)cudaGetLastError();       // "not ready" is an answer, not an error
-    }
-    c->last_tower_ns.store(now_ns, std::memory_order_relaxed);
-    const uint32_t target = flags ? ++c->tower_runs : 0u;     // the number of this run
-    const size_t words = (size_t)(1 + 2 * p->blocks) * c->tile_cap;
-    auto layer_flags = [&](int layer) { return flags ? c->tile_flags + (size_t)layer * c->tile_cap : nullptr; };
-    auto layer_counts = [&](int layer) { return flags ? c->tile_flags + words + (size_t)layer * c->tile_cap : nullptr; };
-    if (flags && c->tower_kernel && p->tower_table != nullptr && !p->tower_refused) {
-        // every layer in one cooperative launch (conv_tower.cuh)
-        const int max_clusters = p->sm_count / 2;
-        const int rounds = (npairs + max_clusters - 1) / max_clusters;
-        const int clusters = (npairs + rounds - 1) / rounds;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(2 * clusters);
-        cfg.blockDim = dim3(dc::kDcThreads);
-        cfg.dynamicSmemBytes = dct::kTowerSmemBytes;
-        cfg.stream = c->stream;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeCooperative;
-        attr[0].val.cooperative = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        auto kernel = dct::conv_tower_kernel<T, 1>;
-        if constexpr (std::is_same<T, __half>::value) {
-            if (p->aplanes == 3) kernel = dct::conv_tower_kernel<T, 3>;
-        }
-        const int n_layers = static_cast<int>(p->layers.size());
-        cudaError_t le;
-        {
-            LaunchScope scope(c, kClassContraction, n_layers);
-            le = cudaLaunchKernelEx(&cfg, kernel, c->tmIN, c->tmX, c->tmH, p->aplanes == 3 ? c->tmXl : c->tmX,
-                                    p->aplanes == 3 ? c->tmHl : c->tmH, c->tmXo, c->tmHo,
-                                    (const dct::TowerLayer*)p->tower_table, n_layers, X, static_cast<T*>(c->H),
-                                    static_cast<int>(dc::cells_for(nb)), p->Cp, npairs, p->row_bytes() / p->elt,
-                                    p->row_bytes(), c->Qa, c->tile_flags, c->tile_flags + words, c->tile_cap,
-                                    target, c->d_err);
-        }
-        if (le == cudaSuccess) le = cudaGetLastError();
-        if (le != cudaSuccess) {
-            // e.g. cooperative launches with clusters not available: keep to a launch per layer
-            (void)cudaGetLastError();
-            p->tower_refused = true;
-        } else {
-            const int cells = nb * kSq;
-            {
-                LaunchScope scope(c, kClassHead);
-                dc::head_conv_cells_kernel<T><<<(cells + 7) / 8, 256, 0, c->stream>>>(
-                    X, p->head_w, p->Cp, cells, pol_dev, val_dev, p->row_bytes() / p->elt,
-                    (p->aplanes == 2 || (p->aplanes == 3 && p->layers.back().out_lo)) ? p->Cp : 0,
-                    p->aplanes == 3 ? 1 : 0);
+            if ((rc = launch_conv_direct<T>(c, p->layers[2 + 2 * b], nb, c->tmH, c->tmXo, X, &c->tmHl, c->X))) {
+                return rc;
             }
-            LZB_CUDA(cudaGetLastError());
-            return LZB_OK;
-        }
-    }
-    if ((rc = launch_conv_direct<T>(c, p->layers[0], nb, c->tmIN, c->tmXo, nullptr, nullptr, c->X, nullptr,
-                                    layer_flags(0), layer_counts(0), target))) {
-        return rc;
-    }
-    for (int b = 0; b < p->blocks; b++) {
-        if ((rc = launch_conv_direct<T>(c, p->layers[1 + 2 * b], nb, c->tmX, c->tmHo, nullptr, &c->tmXl,
-                                        c->H, layer_flags(2 * b), layer_flags(1 + 2 * b),
-                                        layer_counts(1 + 2 * b), target))) {
-            return rc;
-        }
-        if ((rc = launch_conv_direct<T>(c, p->layers[2 + 2 * b], nb, c->tmH, c->tmXo, X, &c->tmHl,
-                                        c->X, layer_flags(1 + 2 * b), layer_flags(2 + 2 * b),
-                                        layer_counts(2 + 2 * b), target))) {
-            return rc;
         }
     }
     const int cells = nb * kSq;
@@ -659,7 +620,6 @@ int run_tower_direct(lzb_ctx* c, const float* in_dev, int nb, float* pol_dev, fl
     LZB_CUDA(cudaGetLastError());
     return LZB_OK;
 }
-
 int run_tower_any(lzb_ctx* c, const float* in_dev, int nb, float* pol_dev, float* val_dev) {
     if (c->pipe->direct) {
         return c->pipe->precision == LZB_FP16
@@ -721,38 +681,27 @@ int set_smem_attrs() {
             LZB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, dc2::kD2SmemBytes));
         }
     }
-    LZB_CUDA(cudaFuncSetAttribute(dct::conv_tower_kernel<__half, 1>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, dct::kTowerSmemBytes));
-    LZB_CUDA(cudaFuncSetAttribute(dct::conv_tower_kernel<__half, 3>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, dct::kTowerSmemBytes));
-    LZB_CUDA(cudaFuncSetAttribute(dct::conv_tower_kernel<__nv_bfloat16, 1>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, dct::kTowerSmemBytes));
-    LZB_CUDA(cudaFuncSetAttribute(dc3::conv_ksplit_kernel<__half, 1>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, dc3::kD3SmemBytes));
-    LZB_CUDA(cudaFuncSetAttribute(dc3::conv_ksplit_kernel<__half, 3>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, dc3::kD3SmemBytes));
-    LZB_CUDA(cudaFuncSetAttribute(dc3::conv_ksplit_kernel<__nv_bfloat16, 1>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, dc3::kD3SmemBytes));
+    {
+        const void* variants[] = {
+            (const void*)dct::conv_tower_kernel<__half, 1>, (const void*)dct::conv_tower_kernel<__half, 2>,
+            (const void*)dct::conv_tower_kernel<__half, 3>, (const void*)dct::conv_tower_kernel<__nv_bfloat16, 1>,
+            (const void*)dct::conv_tower_kernel<__nv_bfloat16, 2>};
+        for (const void* k : variants) {
+            LZB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, dct::kTowerSmemBytes));
+        }
+    }
     return LZB_OK;
 }
 
-// How many clusters of `csize` CTAs of the reduction-split kernel fit the
-// device at once (0 if the question fails: the kernel is then not used).
-template <typename T>
-int ksplit_resident_clusters(int csize) {
+// How many CTA pairs of the one-launch tower the device holds at once (0 if the
+// question fails: it is then not used).
+int tower_resident_pairs() {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(csize);
-    cfg.blockDim = dim3(dc::kDcThreads);
-    cfg.dynamicSmemBytes = dc3::kD3SmemBytes;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = csize;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.gridDim = dim3(2);
+    cfg.blockDim = dim3(dct::kTowerThreads);
+    cfg.dynamicSmemBytes = dct::kTowerSmemBytes;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, dc3::conv_ksplit_kernel<T, 1>, &cfg) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&n, dct::conv_tower_kernel<__half, 3>, &cfg) != cudaSuccess) {
         (void)cudaGetLastError();
         return 0;
     }
@@ -1141,14 +1090,7 @@ int lzb_pipe_create(lzb_pipe** out, int device, int channels, int blocks, int pr
                           !(getenv("LZB_CONV_PAIRS") != nullptr && atoi(getenv("LZB_CONV_PAIRS")) == 0));
     p->elt = precision == LZB_FP32 ? 4 : 2;
     p->sm_count = prop.multiProcessorCount;
-    // LZB_CONV_KSPLIT=0 keeps small batches on the sliced CTA-pair kernel
-    // (cross-check and diagnostics).
-    if (p->pairs && (aplanes == 1 || aplanes == 3) && !(getenv("LZB_CONV_KSPLIT") != nullptr && atoi(getenv("LZB_CONV_KSPLIT")) == 0)) {
-        for (int k = 2; k <= dc3::kMaxSplit; k++) {
-            p->ksplit_max_tiles[k] = precision == LZB_FP16 ? ksplit_resident_clusters<__half>(2 * k)
-                                                            : ksplit_resident_clusters<__nv_bfloat16>(2 * k);
-        }
-    }
+    if (p->pairs) p->tower_pairs = tower_resident_pairs();
     p->layers.resize(1 + 2 * blocks);
     *out = p;
     return LZB_OK;
@@ -1180,7 +1122,7 @@ void lzb_pipe_destroy(lzb_pipe* p) {
         cudaFree(L.invstd);
     }
     cudaFree(p->head_w);
-    cudaFree(p->tower_table);
+    for (auto* t : p->tower_table) cudaFree(t);
     Heads& h = p->heads;
     float* hs[] = {h.bn_pol_mean, h.bn_pol_invstd, h.ip_pol_wT, h.ip_pol_b, h.bn_val_mean,
                    h.bn_val_invstd, h.ip1_val_wT, h.ip1_val_b, h.ip2_val_w, h.ip2_val_b};
@@ -1247,16 +1189,23 @@ int lzb_pipe_finalize(lzb_pipe* p) {
         if (!p->layers[l].present) return fail(LZB_ERR_ARG, "layer " + std::to_string(l) + " missing");
     }
     if (!p->head_convs) return fail(LZB_ERR_ARG, "head convolutions missing");
-    // the one-launch tower (conv_tower.cuh): CTA pairs, one or the e5m2 two-plane form
-    if (p->direct && p->pairs && (p->aplanes == 1 || p->aplanes == 3) && p->blocks > 0) {
+    // records of the one-launch tower (conv_tower.cuh), for each number of slices
+    for (int ns = 1; ns <= 4 && p->tower_pairs > 0; ns++) {
+        // a channel slice must be a multiple of 64 (two epilogue warps x 32 columns)
+        if (p->Cp % ns != 0 || (p->Cp / ns) % 64 != 0) continue;
         LZB_CUDA(enter_device(p->device));
+        const int n_slice = p->Cp / ns, tps = dct::tower_taps_per_stage(n_slice);
         std::vector<dct::TowerLayer> table(p->layers.size());
         for (size_t l = 0; l < p->layers.size(); l++) {
             const Layer& L = p->layers[l];
             dct::TowerLayer& t = table[l];
             std::memset(&t, 0, sizeof(t));
-            t.tmW = L.tmW2[1];
-            t.tmWl = L.Wd8 ? L.tmW8[1] : L.tmW2[1];
+            int rc = make_weight_map(&t.tmW, p->precision, L.Wd, p->Cp, L.cinw, 64, n_slice / 2, tps);
+            t.tmWl = t.tmW;
+            if (!rc && L.Wd8) {
+                rc = make_weight_map(&t.tmWl, -1, L.Wd8, p->Cp, (uint64_t)L.lchunks * 128, 128, n_slice / 2, tps);
+            }
+            if (rc) return rc;
             t.mean = L.mean;
             t.invstd = L.invstd;
             const bool second = l > 0 && l % 2 == 0;          // second convolution of a block
@@ -1272,8 +1221,8 @@ int lzb_pipe_finalize(lzb_pipe* p) {
             t.out_lo = (planes && L.out_lo) ? 1 : 0;
             t.out_hi8 = (planes && L.out_hi8) ? 1 : 0;
         }
-        LZB_CUDA(cudaMalloc(&p->tower_table, table.size() * sizeof(dct::TowerLayer)));
-        LZB_CUDA(cudaMemcpy(p->tower_table, table.data(), table.size() * sizeof(dct::TowerLayer),
+        LZB_CUDA(cudaMalloc(&p->tower_table[ns], table.size() * sizeof(dct::TowerLayer)));
+        LZB_CUDA(cudaMemcpy(p->tower_table[ns], table.data(), table.size() * sizeof(dct::TowerLayer),
                             cudaMemcpyHostToDevice));
     }
     p->finalized = true;
@@ -1335,20 +1284,12 @@ int lzb_ctx_create(lzb_ctx** out, lzb_pipe* p, int max_batch) {
         alloc(&c->IN, (size_t)c->Qa * 64 * p->elt);
         alloc(&c->X, (size_t)c->Qa * p->row_bytes());
         alloc(&c->H, (size_t)c->Qa * p->row_bytes());
-        // Layers of large batches depend on each other tile by tile instead of
-        // launch by launch (conv_direct2.cuh).  Measured gain: 3-4 % per step with
-        // the e5m2 planes (LZB_FP16_X2), none without them, so that mode has it by
-        // default, used while the context is alone on the GPU (run_tower_direct);
-        // LZB_TILE_FLAGS=0 / 1, read here, switches it off / always on for any mode.
+        // LZB_TILE_FLAGS=0, read here, keeps this context to a launch per layer
+        // (cross-check and diagnostics).
         const char* tf = getenv("LZB_TILE_FLAGS");
-        const bool tile_flags = tf != nullptr ? atoi(tf) == 1 : p->aplanes == 3;
-        c->tile_flags_always = tf != nullptr && atoi(tf) == 1;
-        const char* tk = getenv("LZB_TOWER_KERNEL");
-        c->tower_kernel = tk != nullptr && atoi(tk) == 1;
-        if (p->pairs && tile_flags) {
-            c->tile_cap = (c->Qa + dc2::kPairM - 1) / dc2::kPairM;
-            // two words per layer and tile: the run that completed it last, and the arrival counter
-            alloc((void**)&c->tile_flags, (size_t)2 * (1 + 2 * p->blocks) * c->tile_cap * sizeof(uint32_t));
+        if (p->tower_pairs > 0 && !(tf != nullptr && atoi(tf) == 0)) {
+            c->tile_cap = (dct::kTilesPerPos128 * c->micro_cap + 1) / 2;
+            alloc((void**)&c->tile_counts, (size_t)2 * (1 + 2 * p->blocks) * c->tile_cap * sizeof(uint32_t));
         }
     } else {
         c->micro = default_micro_batch(p, c->micro_cap);
@@ -1374,10 +1315,6 @@ int lzb_ctx_create(lzb_ctx** out, lzb_pipe* p, int max_batch) {
         return code;
     }
     *c->h_err = 0;
-    {
-        std::lock_guard<std::mutex> lk(p->ctx_mutex);
-        p->contexts.push_back(c);
-    }
     if (p->direct) {
         int rc = make_map_2d(&c->tmIN, p->precision, c->IN, (uint64_t)c->Qa, 64, dc::kWinRows);
         // 16-bit channels of a cell row (hi [+ 16-bit lo] plane) and the row pitch
@@ -1416,21 +1353,11 @@ int lzb_ctx_create(lzb_ctx** out, lzb_pipe* p, int max_batch) {
 void lzb_ctx_destroy(lzb_ctx* c) {
     if (!c) return;
     cudaSetDevice(c->pipe->device);
-    {
-        std::lock_guard<std::mutex> lk(c->pipe->ctx_mutex);
-        auto& v = c->pipe->contexts;
-        for (size_t i = 0; i < v.size(); i++) {
-            if (v[i] == c) {
-                v.erase(v.begin() + i);
-                break;
-            }
-        }
-    }
     if (c->stream) {
         cudaStreamSynchronize(c->stream);
         cudaStreamDestroy(c->stream);
     }
-    void* ptrs[] = {c->V, c->M, c->X, c->IN, c->H, c->d_in, c->d_pol, c->d_val, c->d_policy, c->d_winrate, c->d_packed, c->d_err, c->tile_flags};
+    void* ptrs[] = {c->V, c->M, c->X, c->IN, c->H, c->d_in, c->d_pol, c->d_val, c->d_policy, c->d_winrate, c->d_packed, c->d_err, c->tile_counts};
     for (void* q : ptrs) cudaFree(q);
     if (c->h_err) cudaFreeHost(c->h_err);
     delete c;
@@ -1474,11 +1401,10 @@ int lzb_ctx_sync(lzb_ctx* c) {
         const int code = *c->h_err;
         *c->h_err = 0;
         cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream);
-        if (c->tile_flags != nullptr) {
-            // an abandoned run may have left a tile's arrivals short of sixteen
-            cudaMemsetAsync(c->tile_flags, 0,
+        if (c->tile_counts != nullptr) {
+            // an abandoned run leaves its counters short
+            cudaMemsetAsync(c->tile_counts, 0,
                             (size_t)2 * (1 + 2 * c->pipe->blocks) * c->tile_cap * sizeof(uint32_t), c->stream);
-            c->tower_runs = 0;
         }
         return fail(LZB_ERR_DEVICE_WAIT,
                     "a kernel gave up a bounded wait (code " + std::to_string(code) + ")");
