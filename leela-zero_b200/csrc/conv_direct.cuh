@@ -42,6 +42,7 @@
 // layer (src/OpenCL.cpp:332-494) with one.
 #pragma once
 #include "gemm_tcgen05.cuh"
+#include "input_view.cuh"
 #include "winograd_math.cuh"
 
 namespace lzb {
@@ -554,11 +555,11 @@ __global__ void __launch_bounds__(kDcThreads, 1) conv_direct_kernel(
 // Helper kernels of the direct path (all bandwidth-trivial).
 // ---------------------------------------------------------------------------
 
-// Network input planes in[n][18][361] fp32 -> padded cell-major X0[Qa][64],
+// Network input planes -> padded cell-major X0[Qa][64],
 // channels 18..63 and halo cells zero.  One thread per (cell, channel pair).
 template <typename T>
-__global__ void __launch_bounds__(256) input_to_cells_kernel(const float* __restrict__ in,
-                                                             T* __restrict__ X0, int n) {
+__global__ void __launch_bounds__(256) input_to_cells_kernel(const InputView in, T* __restrict__ X0,
+                                                             int n) {
     using P2 = Pair<T>;
     const long long total = cells_for(n) * 32;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -568,9 +569,8 @@ __global__ void __launch_bounds__(256) input_to_cells_kernel(const float* __rest
         const int c = q % kCellsPerRow, r = q / kCellsPerRow;
         float2 v = make_float2(0.f, 0.f);
         if (c != 0 && (r % 20) != 0 && 2 * pair < kInputPlanes) {
-            const int pos = r / 20, y = r % 20 - 1, x = c - 1;
-            const float* src = in + ((size_t)pos * kInputPlanes + 2 * pair) * kSq + y * kBoard + x;
-            v = make_float2(src[0], src[kSq]);
+            const int pos = r / 20, s = (r % 20 - 1) * kBoard + c - 1;
+            v = make_float2(in.at(pos, 2 * pair, s), in.at(pos, 2 * pair + 1, s));
         }
         *reinterpret_cast<typename P2::type*>(X0 + (size_t)q * 64 + 2 * pair) = P2::from_f2(v);
     }
@@ -657,54 +657,6 @@ __global__ void weights_to_e5m2_kernel(const float* __restrict__ Wd32, unsigned 
             b = e5m2_from_float(kWLoScale * (w - __half2float(__float2half_rn(w))));
         }
         W8[i] = static_cast<unsigned char>(b);
-    }
-}
-
-// 1x1 head convolutions reading the padded cell-major layout (see
-// head_conv_kernel for the arithmetic).  One warp per board cell.
-// ldx: elements (of T) per cell row of X; lo_off > 0: activations are two
-// planes, the low one lo_off elements after the high one, stored as T or,
-// with lo_e5m2, as one e5m2 byte per channel.
-template <typename T>
-__global__ void __launch_bounds__(256) head_conv_cells_kernel(
-    const T* __restrict__ X, const float* __restrict__ w, int Cp, int cells,
-    float* __restrict__ pol, float* __restrict__ val, int ldx, int lo_off, int lo_e5m2) {
-    using P2 = Pair<T>;
-    const int lane = threadIdx.x & 31;
-    const int cell = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (cell >= cells) return;
-    const int n = cell / kSq, s = cell % kSq;
-    const T* x = X + (size_t)cell_of(n, s / kBoard, s % kBoard) * ldx;
-    float a0 = 0.f, a1 = 0.f, a2 = 0.f;
-    for (int c = 2 * lane; c < Cp; c += 64) {
-        float2 v = P2::to_f2(*reinterpret_cast<const typename P2::type*>(x + c));
-        if (lo_off > 0 && lo_e5m2) {
-            const unsigned short two =
-                *reinterpret_cast<const unsigned short*>(reinterpret_cast<const unsigned char*>(x + lo_off) + c);
-            v.x += e5m2_to_float(two);
-            v.y += e5m2_to_float(two >> 8);
-        } else if (lo_off > 0) {
-            const float2 l = P2::to_f2(*reinterpret_cast<const typename P2::type*>(x + lo_off + c));
-            v.x += l.x;
-            v.y += l.y;
-        }
-        const float2 w0 = *reinterpret_cast<const float2*>(w + c);
-        const float2 w1 = *reinterpret_cast<const float2*>(w + Cp + c);
-        const float2 w2 = *reinterpret_cast<const float2*>(w + 2 * Cp + c);
-        a0 += w0.x * v.x + w0.y * v.y;
-        a1 += w1.x * v.x + w1.y * v.y;
-        a2 += w2.x * v.x + w2.y * v.y;
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        a0 += __shfl_xor_sync(0xffffffffu, a0, off);
-        a1 += __shfl_xor_sync(0xffffffffu, a1, off);
-        a2 += __shfl_xor_sync(0xffffffffu, a2, off);
-    }
-    if (lane == 0) {
-        pol[((size_t)n * 2 + 0) * kSq + s] = a0;
-        pol[((size_t)n * 2 + 1) * kSq + s] = a1;
-        val[(size_t)n * kSq + s] = a2;
     }
 }
 

@@ -69,11 +69,12 @@ constexpr int kTowerThreads = 384;
 constexpr int kTowerEpiWarp = 4;                        // first epilogue warp
 constexpr int kTilesPerPos128 = 3;                      // row tiles of one position
 constexpr int kTowerWins = 4;                           // activation windows in flight
-constexpr uint32_t kTowerRingBytes = 112 * 1024;        // weight ring
-constexpr int kTowerMaxStages = 14;
+constexpr uint32_t kTowerRingBytes = 96 * 1024;         // weight ring
+constexpr int kTowerMaxStages = 12;
+constexpr uint32_t kTowerStageOut = kStageOutBytes + 2 * 1024;   // one epilogue warp: 16-bit tile, two byte tiles
 constexpr uint32_t kTowerOperandBytes = kTowerWins * kWinBytes + kTowerRingBytes;
 constexpr uint32_t kTowerSmemBytes =
-    kTowerOperandBytes + 8 * kStageOutBytes + 8 * kMaxN * 4 /* bn, per warp */ + kBarBytes + 1024;
+    kTowerOperandBytes + 8 * kTowerStageOut + 8 * kMaxN * 4 /* bn, per warp */ + kBarBytes + 1024;
 static_assert(kTowerSmemBytes <= 227 * 1024, "shared memory of one CTA");
 constexpr int kDepRing = 8;                             // units the window loads can be ahead of the epilogue, rounded up
 constexpr unsigned long long kTileWaitLimitNs = 1000000000ull;
@@ -137,6 +138,15 @@ __device__ __forceinline__ bool tiles_wait(const uint32_t* counter, uint32_t tar
         }
     }
 }
+// One lane hands a staged tile to the TMA engine (after store_staged_tile's fence).
+__device__ __forceinline__ void store_tile(const CUtensorMap* map, uint32_t src, int col, int row) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(
+            reinterpret_cast<uint64_t>(map)),
+        "r"(col), "r"(row), "r"(src)
+        : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
 // Residual rows come from L2: this kernel's other CTAs rewrite them layer by layer.
 template <typename T>
 __device__ __forceinline__ void load_residual_l2(uint4 (&v)[4], const T* src, bool use) {
@@ -167,18 +177,21 @@ struct UnitWalk {
 
 // tmIN, tmX, tmH : activation windows (box 64 x kWinRows); tmXl, tmHl : their
 // e5m2 planes (byte maps, box 128 x kWinRows); tmXo, tmHo : output tiles (box
-// 32 x 32, 64-byte swizzle).  X, H : the two activation tensors (residual reads,
-// byte-plane stores), ldr elements of T / out_pitch bytes per cell row.  ntiles
-// row tiles (three per position), nsplit slices.  counts : [n_layers][tile_cap]
-// words, zero when the kernel starts; counts_next : the same for the next run on
-// this context, cleared here.
+// 32 x 32, 64-byte swizzle), tmXlo, tmHlo : byte-plane output tiles (box 32 x 32,
+// the e5m2 plane from byte 0, the hi8 plane from byte Kp).  X, H : the two
+// activation tensors, ldr elements of T per cell row.  input : the network input, converted here into IN (64 channels of T per cell row,
+// channels 24 .. 63 zero beforehand).  ntiles row tiles (three per position),
+// nsplit slices.  counts : [n_layers + 1][tile_cap] words, row l for the tiles
+// layer l reads, zero when the kernel starts; counts_next : the same for the next
+// run on this context, cleared here.
 template <typename T, int kPlanes>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTowerThreads, 1) conv_tower_kernel(
     const __grid_constant__ CUtensorMap tmIN, const __grid_constant__ CUtensorMap tmX,
     const __grid_constant__ CUtensorMap tmH, const __grid_constant__ CUtensorMap tmXl,
     const __grid_constant__ CUtensorMap tmHl, const __grid_constant__ CUtensorMap tmXo,
-    const __grid_constant__ CUtensorMap tmHo, const TowerLayer* __restrict__ layers, int n_layers,
-    T* X, T* H, int ntiles, int Kp, int nsplit, int ldr, int out_pitch, uint32_t* counts,
+    const __grid_constant__ CUtensorMap tmHo, const __grid_constant__ CUtensorMap tmXlo,
+    const __grid_constant__ CUtensorMap tmHlo, const TowerLayer* __restrict__ layers, int n_layers,
+    const InputView input, T* IN, T* X, T* H, int ntiles, int Kp, int nsplit, int ldr, uint32_t* counts,
     uint32_t* counts_next, int tile_cap, int* err) {
     extern __shared__ unsigned char smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
@@ -187,8 +200,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTowerThreads, 1) co
     const uint32_t win_base = base;
     const uint32_t b_base = base + kTowerWins * kWinBytes;
     unsigned char* stage_out = smem + kTowerOperandBytes;
-    float* s_bn = reinterpret_cast<float*>(stage_out + 8 * kStageOutBytes);      // per warp: scale[128], bias[128]
-    unsigned char* bar_mem = stage_out + 8 * kStageOutBytes + 8 * kMaxN * 4;
+    float* s_bn = reinterpret_cast<float*>(stage_out + 8 * kTowerStageOut);      // per warp: scale[128], bias[128]
+    unsigned char* bar_mem = stage_out + 8 * kTowerStageOut + 8 * kMaxN * 4;
     const uint32_t bars = smem_u32(bar_mem);
     auto bfull_bar = [&](int s) { return bars + 8u * (0 + s); };      // leader's are used
     auto bempty_bar = [&](int s) { return bars + 8u * (16 + s); };    // both CTAs
@@ -200,6 +213,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTowerThreads, 1) co
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bar_mem + 8 * 56);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(bar_mem + 8 * 56 + 8);
 
+    // the head kernel may be placed on SMs this kernel leaves free; it waits for the
+    // end of this one before it reads anything
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();
     const bool leader = rank == 0;
@@ -228,7 +244,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTowerThreads, 1) co
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    for (int i = blockIdx.x * kTowerThreads + threadIdx.x; i < n_layers * tile_cap; i += gridDim.x * kTowerThreads) {
+    for (int i = blockIdx.x * kTowerThreads + threadIdx.x; i < (n_layers + 1) * tile_cap; i += gridDim.x * kTowerThreads) {
         counts_next[i] = 0u;
     }
     if (warp == 1) {
@@ -267,29 +283,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTowerThreads, 1) co
             const CUtensorMap* in_lo = tl->in_sel == 2 ? &tmHl : &tmXl;
             const int pair = w.u / nsplit;
             const int tile = tile_of(pair);
-            if (w.layer > 0) {
-                // the tiles this window reaches: its own pair's two, and the neighbour
-                // pair's where the neighbouring row tile belongs to the same position
-                const uint32_t* row = counts + static_cast<size_t>(w.layer - 1) * tile_cap;
-                const uint32_t* mine = nullptr;
-                if (lane == 0) mine = row + pair;
-                if (lane == 1) {
-                    const int part = tile % kTilesPerPos128;
-                    const int other = part == 0 ? tile + 1 : tile - 1;          // a row tile on either side ...
-                    mine = row + (other >> 1);
-                }
-                if (lane == 2) {
-                    const int part = tile % kTilesPerPos128;
-                    const int other = part == kTilesPerPos128 - 1 ? tile - 1 : tile + 1;
-                    mine = row + (other >> 1);
-                }
-                if (!tiles_wait(mine, complete, abort_flag, err)) break;
-            }
+            // the row tiles this window reaches: its own and, within the position, one
+            // on either side, each counted with its pair
+            const uint32_t* row = counts + static_cast<size_t>(w.layer) * tile_cap;
+            const int part = tile % kTilesPerPos128;
+            const uint32_t* mine = nullptr;
+            if (lane == 0) mine = row + pair;
+            if (lane == 1 && part > 0) mine = row + ((tile - 1) >> 1);
+            if (lane == 2 && part < kTilesPerPos128 - 1) mine = row + ((tile + 1) >> 1);
+            if (!tiles_wait(mine, complete, abort_flag, err)) break;
             bool ok = true;
             if (elect_one()) {
-                // what those tiles' epilogues stored is read below by TMA (async proxy)
-                asm volatile("fence.proxy.async;" ::: "memory");
                 mbar_arrive(dep_bar(dep));
+                // what was counted above is read below by TMA (async proxy)
+                asm volatile("fence.proxy.async.global;" ::: "memory");
                 const int m0 = tower_tile_row(tile);
                 for (int c = 0; c < kchunks; ++c) {
                     ok = mbar_wait(wempty_bar(wb), wphase ^ 1u, abort_flag, err, kErrTowerProducer);
@@ -407,11 +414,37 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTowerThreads, 1) co
         const int qd = warp & 3;                 // tensor-memory lane quadrant
         const int ncols = n_slice >> 1;          // channels this warp converts per unit
         const int wcol = (ew >> 2) * ncols;
-        unsigned char* stg_ptr = stage_out + ew * kStageOutBytes;
+        unsigned char* stg_ptr = stage_out + ew * kTowerStageOut;
         const uint32_t stg = smem_u32(stg_ptr);
         unsigned char* stg_row = stg_ptr + lane * 64;
         float* s_scale = s_bn + ew * 2 * (kMaxN / 2);
         float* s_bias = s_scale + kMaxN / 2;
+        if (ew < 4) {
+            // network input: this CTA's row tile of every pair it starts with, 32 cells a
+            // warp; counted like a layer's tiles (two CTAs x four warps x 2 nsplit)
+            for (int pair = cid; pair < npairs; pair += step) {
+                const int t = 2 * pair + static_cast<int>(rank);
+                if (t < ntiles) {
+                    const int q = tower_tile_row(t) + ew * 32 + lane;
+                    const int c = q % kCellsPerRow, r = (q / kCellsPerRow) % 20;
+                    const bool inside = c != 0 && r != 0;
+                    const int s = (r - 1) * kBoard + c - 1;
+                    uint32_t o[12];
+#pragma unroll
+                    for (int k = 0; k < 12; ++k) {
+                        const bool use = inside && 2 * k < kInputPlanes;
+                        o[k] = pack2(T(), use ? input.at(t / kTilesPerPos128, 2 * k, s) : 0.f,
+                                     use ? input.at(t / kTilesPerPos128, 2 * k + 1, s) : 0.f);
+                    }
+                    uint4* dst = reinterpret_cast<uint4*>(IN + static_cast<size_t>(q) * 64);
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) dst[k] = make_uint4(o[4 * k], o[4 * k + 1], o[4 * k + 2], o[4 * k + 3]);
+                }
+                asm volatile("fence.proxy.async;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) red_release_gpu_add(counts + pair, 2u * static_cast<uint32_t>(nsplit));
+            }
+        }
         int local = 0, dep = 0, bn_layer = -1, bn_col = -1;
         uint32_t dphase = 0;
         for (UnitWalk w(cid, units, step); w.layer < n_layers; w.next(), ++local) {
@@ -435,14 +468,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTowerThreads, 1) co
                 __syncwarp();
             }
             const CUtensorMap* out_map = tl->out_sel == 1 ? &tmXo : &tmHo;
-            T* out_base = tl->out_sel == 1 ? X : H;
+            const CUtensorMap* out_bytes = tl->out_sel == 1 ? &tmXlo : &tmHlo;
             const T* res = tl->has_res ? X : nullptr;
-            const bool res_lo = tl->res_lo != 0;
-            unsigned char* out_lo =
-                tl->out_lo ? reinterpret_cast<unsigned char*>(out_base) + static_cast<size_t>(Kp) * sizeof(T) : nullptr;
-            unsigned char* out_hi8 = tl->out_hi8 ? reinterpret_cast<unsigned char*>(out_base) +
-                                                       static_cast<size_t>(Kp) * (sizeof(T) + 1)
-                                                 : nullptr;
+            const bool res_lo = tl->res_lo != 0, out_lo = tl->out_lo != 0, out_hi8 = tl->out_hi8 != 0;
             constexpr bool two = kPlanes == 2;
             constexpr bool e5 = kPlanes == 3;
             const bool use_res = (res != nullptr) && interior && live;
@@ -476,20 +504,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTowerThreads, 1) co
                 if constexpr (e5) {
                     uint32_t lo[8], h8[8];
                     epilogue_chunk_e5m2<T>(r, v, e, s_scale + j, s_bias + j, use_res, interior, stg_row, lane,
-                                           lo, h8, out_hi8 != nullptr);
+                                           lo, h8, out_hi8);
+                    // byte tiles beside the 16-bit one: 32 cells x 32 bytes each
+                    uint4* row = reinterpret_cast<uint4*>(stg_ptr + kStageOutBytes + lane * 32);
+                    if (out_lo) {
+                        row[0] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                        row[1] = make_uint4(lo[4], lo[5], lo[6], lo[7]);
+                    }
+                    if (out_hi8) {
+                        row[64] = make_uint4(h8[0], h8[1], h8[2], h8[3]);
+                        row[65] = make_uint4(h8[4], h8[5], h8[6], h8[7]);
+                    }
                     if (live) {
                         store_staged_tile(out_map, stg, col, row0, lane);
-                        const size_t off = static_cast<size_t>(q) * out_pitch + col;
-                        if (out_lo != nullptr) {
-                            uint4* dst = reinterpret_cast<uint4*>(out_lo + off);
-                            dst[0] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-                            dst[1] = make_uint4(lo[4], lo[5], lo[6], lo[7]);
-                        }
-                        if (out_hi8 != nullptr) {
-                            uint4* dst = reinterpret_cast<uint4*>(out_hi8 + off);
-                            dst[0] = make_uint4(h8[0], h8[1], h8[2], h8[3]);
-                            dst[1] = make_uint4(h8[4], h8[5], h8[6], h8[7]);
-                        }
+                        if (lane == 0 && out_lo) store_tile(out_bytes, stg + kStageOutBytes, col, row0);
+                        if (lane == 0 && out_hi8) store_tile(out_bytes, stg + kStageOutBytes + 1024, Kp + col, row0);
                     }
                 } else if constexpr (!two) {
                     epilogue_chunk<T>(r, v, s_scale + j, s_bias + j, use_res, interior, stg_row, lane);
@@ -528,13 +557,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTowerThreads, 1) co
             tcgen05_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(map_to_cta(tempty_bar(acc), 0));
-            // this warp's part of the tile is in memory: its TMA stores have completed,
-            // its lanes' byte-plane stores are handed to the async proxy; the release
-            // covers what the other lanes stored before the warp barrier
-            if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-            asm volatile("fence.proxy.async;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) red_release_gpu_add(counts + static_cast<size_t>(w.layer) * tile_cap + pair, 1u);
+            // this warp's part of the tile is in memory once its TMA stores have
+            // completed; nothing else wrote it, so no proxy fence is needed on this side
+            if (lane == 0) {
+                asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+                red_release_gpu_add(counts + static_cast<size_t>(w.layer + 1) * tile_cap + pair, 1u);
+            }
         }
         if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     }

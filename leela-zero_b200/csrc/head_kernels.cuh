@@ -1,22 +1,39 @@
-// The network heads after the two 1x1 convolutions, finished on the device:
-//   policy: batch-norm + ReLU on 2 planes -> FC 722 -> 362 -> softmax
-//   value : batch-norm + ReLU on 1 plane  -> FC 361 -> 256 ReLU -> FC 256 -> 1
-//           -> (1 + tanh) / 2
-// This is the arithmetic Network::get_output_internal runs on the CPU for every
-// evaluation (src/Network.cpp:833-851, innerproduct :609-637, softmax :693-712).
-// FC matrices are kept transposed ([in][out]) so that neighbouring threads read
-// neighbouring weights.  One CLUSTER per position: the inputs of the first
-// fully connected layer are cut into one slice per CTA (a single CTA walking
-// all 722 rows of the 1 MB policy matrix took 34 us whatever the batch size);
-// the partial sums are written into the first CTA's shared memory
-// (st.shared::cluster), which adds them in slice order and finishes the head.
+// The network heads, from the last activations to policy and winrate in one launch:
+//   policy: 1x1 conv to 2 planes, batch-norm + ReLU -> FC 722 -> 362 -> softmax
+//   value : 1x1 conv to 1 plane,  batch-norm + ReLU -> FC 361 -> 256 ReLU
+//           -> FC 256 -> 1 -> (1 + tanh) / 2
+// This is the arithmetic of the convolutions in CPUPipe::forward
+// (src/CPUPipe.cpp:301-350) and of what Network::get_output_internal runs on the
+// CPU for every evaluation (src/Network.cpp:833-851, innerproduct :609-637,
+// softmax :693-712).
+//
+// One CLUSTER of eight CTAs per position (or per group of positions).  Each CTA
+// owns 46 of the 361 cells in all three planes: it computes the 1x1 convolutions
+// of its cells, which are then exactly its slice of the inputs of both fully
+// connected layers, and sends the partial sums of their outputs to the shared
+// memory of the CTA that finishes a head (policy: the first, value: the second),
+// which adds them in slice order.
+//
+// What bounds it is latency.  A thread owns one (plane, output) pair, 46 weights;
+// it has them in registers before it waits for the tower, so that after the tower
+// only the activations (L2), two block barriers and one cluster barrier remain.
+// As separate launches (1x1 convolutions, policy head, value head), with the weights
+// fetched four at a time behind the activations, the heads of one position took
+// 25 us; together with the copies that followed them they were a third of a small
+// evaluation.  With more positions than clusters fit the GPU at once a cluster
+// takes several and reads the 1.4 MB of weights once for all of them.
 #pragma once
+#include "conv_direct.cuh"
 #include "winograd_math.cuh"
 
 namespace lzb {
 
 constexpr int kMoves = 362;
 constexpr int kValueHidden = 256;
+constexpr int kHeadCtas = 8;                                    // CTAs per cluster
+constexpr int kHeadCells = (kSq + kHeadCtas - 1) / kHeadCtas;   // 46 cells per CTA
+constexpr int kHeadThreads = 992;                               // 362 + 362 + 256 (plane, output) pairs
+static_assert(kHeadThreads >= 2 * kMoves + kValueHidden && kHeadThreads % 32 == 0, "a thread per pair");
 
 __device__ __forceinline__ float block_reduce(float v, float* scratch, bool is_max) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -32,19 +49,15 @@ __device__ __forceinline__ float block_reduce(float v, float* scratch, bool is_m
     for (int i = 1; i < nw; i++) r = is_max ? fmaxf(r, scratch[i]) : r + scratch[i];
     return r;
 }
-
-constexpr int kPolicySlices = 8;     // CTAs per position in policy_head_kernel
-constexpr int kValueSlices = 4;      // ... in value_head_kernel
-
 __device__ __forceinline__ uint32_t head_cluster_rank() {
     uint32_t r;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
     return r;
 }
-// store into the shared memory of CTA 0 of the cluster, at the offset `local` has here
-__device__ __forceinline__ void store_to_first_cta(float* local, float v) {
+// store into the shared memory of CTA `rank` of the cluster, at the offset `local` has here
+__device__ __forceinline__ void store_to_cta(float* local, uint32_t rank, float v) {
     uint32_t addr = static_cast<uint32_t>(__cvta_generic_to_shared(local)), remote;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(0u));
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
     asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(v) : "memory");
 }
 __device__ __forceinline__ void head_cluster_sync() {
@@ -52,86 +65,166 @@ __device__ __forceinline__ void head_cluster_sync() {
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// grid kPolicySlices * n (clusters of kPolicySlices), block 384.
-// pol[n][2][361] raw planes -> policy[n][362].
-__global__ void __cluster_dims__(kPolicySlices, 1, 1) __launch_bounds__(384) policy_head_kernel(
-    const float* __restrict__ pol, const float* __restrict__ bn_mean,
-    const float* __restrict__ bn_invstd, const float* __restrict__ wT /*[722][362]*/,
-    const float* __restrict__ bias, float inv_temp, float* __restrict__ policy) {
-    constexpr int kRows = (2 * kSq + kPolicySlices - 1) / kPolicySlices;   // FC inputs per slice
-    __shared__ float x[kRows];
-    __shared__ float part[kPolicySlices][kMoves];       // used in the first CTA of the cluster
-    __shared__ float scratch[12];
-    const int n = blockIdx.x / kPolicySlices;
-    const int slice = static_cast<int>(head_cluster_rank());
-    const int i0 = slice * kRows;
-    const int rows = (2 * kSq - i0) < kRows ? (2 * kSq - i0) : kRows;
-    for (int r = threadIdx.x; r < rows; r += blockDim.x) {
-        const int i = i0 + r, c = i / kSq;
-        const float v = nf_mul(bn_invstd[c], nf_add(pol[(size_t)n * 2 * kSq + i], -bn_mean[c]));
-        x[r] = fmaxf(v, 0.f);
+// The three 1x1 convolutions of one cell by one warp: channels two per lane, 64
+// apart, added up the lanes.  Activations are rows of ldx elements; lo_off > 0:
+// two planes, the low one lo_off elements after the high one, stored as T or, with
+// lo_e5m2, as one e5m2 byte per channel.  w: [3][Cp].
+template <typename T>
+__device__ __forceinline__ float3 head_conv_cell(const T* x, const float* __restrict__ w, int Cp, int lo_off,
+                                                 int lo_e5m2, int lane) {
+    using P2 = Pair<T>;
+    float a0 = 0.f, a1 = 0.f, a2 = 0.f;
+    for (int c = 2 * lane; c < Cp; c += 64) {
+        float2 v = P2::to_f2(*reinterpret_cast<const typename P2::type*>(x + c));
+        if (lo_off > 0 && lo_e5m2) {
+            const unsigned short two =
+                *reinterpret_cast<const unsigned short*>(reinterpret_cast<const unsigned char*>(x + lo_off) + c);
+            v.x += dc::e5m2_to_float(two);
+            v.y += dc::e5m2_to_float(two >> 8);
+        } else if (lo_off > 0) {
+            const float2 l = P2::to_f2(*reinterpret_cast<const typename P2::type*>(x + lo_off + c));
+            v.x += l.x;
+            v.y += l.y;
+        }
+        const float2 w0 = *reinterpret_cast<const float2*>(w + c);
+        const float2 w1 = *reinterpret_cast<const float2*>(w + Cp + c);
+        const float2 w2 = *reinterpret_cast<const float2*>(w + 2 * Cp + c);
+        a0 += w0.x * v.x + w0.y * v.y;
+        a1 += w1.x * v.x + w1.y * v.y;
+        a2 += w2.x * v.x + w2.y * v.y;
     }
-    __syncthreads();
-    const int o = threadIdx.x;
-    if (o < kMoves) {
-        float acc = 0.f;
-        const float* w = wT + (size_t)i0 * kMoves + o;
-#pragma unroll 4
-        for (int r = 0; r < rows; r++) acc = fmaf(w[(size_t)r * kMoves], x[r], acc);
-        store_to_first_cta(&part[slice][o], acc);
-    }
-    __syncthreads();                  // every warp whole again before the aligned cluster barrier
-    head_cluster_sync();              // all partial sums are in the first CTA
-    if (slice != 0) return;
-    float logit = -INFINITY;
-    if (o < kMoves) {
-        float acc = 0.f;
 #pragma unroll
-        for (int s2 = 0; s2 < kPolicySlices; s2++) acc += part[s2][o];
-        logit = bias[o] + acc;
+    for (int off = 16; off > 0; off >>= 1) {
+        a0 += __shfl_xor_sync(0xffffffffu, a0, off);
+        a1 += __shfl_xor_sync(0xffffffffu, a1, off);
+        a2 += __shfl_xor_sync(0xffffffffu, a2, off);
     }
-    const float mx = block_reduce(logit, scratch, true);
-    const float e = (o < kMoves) ? expf((logit - mx) * inv_temp) : 0.f;
-    const float denom = block_reduce(e, scratch, false);
-    if (o < kMoves) policy[(size_t)n * kMoves + o] = e / denom;
+    return make_float3(a0, a1, a2);
+}
+// Row of board cell s of position n: padded cell-major layout (conv_direct.cuh), or
+// 361 dense rows per position (the Winograd pipeline).
+template <bool kCells>
+__device__ __forceinline__ size_t head_row(int n, int s) {
+    if (kCells) return static_cast<size_t>(dc::cell_of(n, s / kBoard, s % kBoard));
+    return static_cast<size_t>(n) * kSq + s;
 }
 
-// grid kValueSlices * n (clusters of kValueSlices), block 256.
-// val[n][361] raw plane -> winrate[n].
-__global__ void __cluster_dims__(kValueSlices, 1, 1) __launch_bounds__(256) value_head_kernel(
-    const float* __restrict__ val, const float* __restrict__ bn_mean,
-    const float* __restrict__ bn_invstd, const float* __restrict__ w1T /*[361][256]*/,
-    const float* __restrict__ b1, const float* __restrict__ w2, const float* __restrict__ b2,
-    float* __restrict__ winrate) {
-    constexpr int kRows = (kSq + kValueSlices - 1) / kValueSlices;
-    __shared__ float x[kRows];
-    __shared__ float part[kValueSlices][kValueHidden];  // used in the first CTA of the cluster
-    __shared__ float scratch[8];
-    const int n = blockIdx.x / kValueSlices;
-    const int slice = static_cast<int>(head_cluster_rank());
-    const int i0 = slice * kRows;
-    const int rows = (kSq - i0) < kRows ? (kSq - i0) : kRows;
-    for (int r = threadIdx.x; r < rows; r += blockDim.x) {
-        const float v = nf_mul(bn_invstd[0], nf_add(val[(size_t)n * kSq + i0 + r], -bn_mean[0]));
-        x[r] = fmaxf(v, 0.f);
+// Raw head planes pol[n][2][361], val[n][361] (which may be page-locked host memory):
+// 32 board cells per CTA, four per warp, written as whole rows of 128 bytes.
+// err_out, if given, receives *err.
+template <typename T, bool kCells>
+__global__ void __launch_bounds__(256) head_planes_kernel(const T* X, const float* __restrict__ w, int Cp, int n,
+                                                          float* __restrict__ pol, float* __restrict__ val, int ldx,
+                                                          int lo_off, int lo_e5m2, const int* err, int* err_out) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (err_out != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *err_out = *err;
+    __shared__ float out[3][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int first = blockIdx.x * 32;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const int cell = first + warp * 4 + k;
+        if (cell >= n * kSq) break;
+        const float3 r = head_conv_cell<T>(X + head_row<kCells>(cell / kSq, cell % kSq) * ldx, w, Cp, lo_off,
+                                           lo_e5m2, lane);
+        if (lane == 0) {
+            out[0][warp * 4 + k] = r.x;
+            out[1][warp * 4 + k] = r.y;
+            out[2][warp * 4 + k] = r.z;
+        }
     }
     __syncthreads();
-    const int j = threadIdx.x;
-    {
-        float acc = 0.f;
-        const float* w = w1T + (size_t)i0 * kValueHidden + j;
-#pragma unroll 4
-        for (int r = 0; r < rows; r++) acc = fmaf(w[(size_t)r * kValueHidden], x[r], acc);
-        store_to_first_cta(&part[slice][j], acc);
+    const int cell = first + lane;
+    if (warp < 3 && cell < n * kSq) {
+        const int pos = cell / kSq, s = cell % kSq;
+        if (warp < 2) pol[((size_t)pos * 2 + warp) * kSq + s] = out[warp][lane];
+        else val[(size_t)pos * kSq + s] = out[2][lane];
     }
-    head_cluster_sync();
-    if (slice != 0) return;
-    float acc = 0.f;
+}
+
+struct HeadWeights {
+    const float *bn_pol_mean, *bn_pol_invstd, *ip_pol_wT /*[722][362]*/, *ip_pol_b, *bn_val_mean, *bn_val_invstd,
+        *ip1_val_wT /*[361][256]*/, *ip1_val_b, *ip2_val_w, *ip2_val_b;
+};
+
+// grid: clusters of kHeadCtas, each takes positions first, first + clusters, ...
+template <typename T, bool kCells>
+__global__ void __cluster_dims__(kHeadCtas, 1, 1) __launch_bounds__(kHeadThreads)
+    heads_kernel(const T* X, const float* __restrict__ w, int Cp, int n, int ldx, int lo_off, int lo_e5m2,
+                 const HeadWeights h, float inv_temp, float* __restrict__ policy, float* __restrict__ winrate,
+                 const int* err, int* err_out) {
+    __shared__ float x[3][kHeadCells];
+    __shared__ float part_pol[2 * kHeadCtas][kMoves];       // used in the first CTA of the cluster
+    __shared__ float part_val[kHeadCtas][kValueHidden];     // ... in the second
+    __shared__ float scratch[32];
+    const int rank = static_cast<int>(head_cluster_rank());
+    const int s0 = rank * kHeadCells;
+    const int cells = (kSq - s0) < kHeadCells ? (kSq - s0) : kHeadCells;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, warps = kHeadThreads / 32;
+    // this thread's plane and output, and its weights
+    const int plane = t < kMoves ? 0 : (t < 2 * kMoves ? 1 : 2);
+    const int o = t - plane * kMoves;
+    const bool owns = plane < 2 || o < kValueHidden;
+    const int outs = plane < 2 ? kMoves : kValueHidden;
+    const float* wsrc = plane < 2 ? h.ip_pol_wT + (size_t)(plane * kSq + s0) * kMoves + o
+                                  : h.ip1_val_wT + (size_t)s0 * kValueHidden + o;
+    constexpr int kHeld = 26;        // weights held in registers; the rest come from L1 / L2 later
+    float wr[kHeld];
 #pragma unroll
-    for (int s2 = 0; s2 < kValueSlices; s2++) acc += part[s2][j];
-    const float h = fmaxf(b1[j] + acc, 0.f);
-    const float s = block_reduce(w2[j] * h, scratch, false);
-    if (j == 0) winrate[n] = (1.0f + tanhf(b2[0] + s)) / 2.0f;
+    for (int i = 0; i < kHeld; i++) wr[i] = owns ? wsrc[i * outs] : 0.f;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (err_out != nullptr && blockIdx.x == 0 && t == 0) *err_out = *err;
+    for (int pos = blockIdx.x / kHeadCtas; pos < n; pos += gridDim.x / kHeadCtas) {
+        for (int s = warp; s < cells; s += warps) {
+            const float3 r = head_conv_cell<T>(X + head_row<kCells>(pos, s0 + s) * ldx, w, Cp, lo_off, lo_e5m2, lane);
+            if (lane < 3) {
+                const float raw = lane == 0 ? r.x : (lane == 1 ? r.y : r.z);
+                const float m = lane < 2 ? h.bn_pol_mean[lane] : h.bn_val_mean[0];
+                const float is = lane < 2 ? h.bn_pol_invstd[lane] : h.bn_val_invstd[0];
+                x[lane][s] = fmaxf(nf_mul(is, nf_add(raw, -m)), 0.f);
+            }
+        }
+        __syncthreads();
+        if (owns) {
+            const float* xp = x[plane];
+            float acc = 0.f;
+#pragma unroll
+            for (int i = 0; i < kHeld; i++) acc = fmaf(wr[i], xp[i], acc);
+#pragma unroll 8
+            for (int i = kHeld; i < cells; i++) acc = fmaf(wsrc[i * outs], xp[i], acc);
+            if (plane < 2) store_to_cta(&part_pol[2 * rank + plane][o], 0, acc);
+            else store_to_cta(&part_val[rank][o], 1, acc);
+        }
+        __syncthreads();                  // every warp whole again before the aligned cluster barrier
+        head_cluster_sync();              // all partial sums have arrived
+        if (rank == 0) {
+            float logit = -INFINITY;
+            if (t < kMoves) {
+                float acc = 0.f;
+#pragma unroll
+                for (int k = 0; k < 2 * kHeadCtas; k++) acc += part_pol[k][t];
+                logit = h.ip_pol_b[t] + acc;
+            }
+            const float mx = block_reduce(logit, scratch, true);
+            const float e = t < kMoves ? expf((logit - mx) * inv_temp) : 0.f;
+            const float denom = block_reduce(e, scratch, false);
+            if (t < kMoves) policy[(size_t)pos * kMoves + t] = e / denom;
+        } else if (rank == 1) {
+            float v = 0.f;
+            if (t < kValueHidden) {
+                float acc = 0.f;
+#pragma unroll
+                for (int k = 0; k < kHeadCtas; k++) acc += part_val[k][t];
+                v = h.ip2_val_w[t] * fmaxf(h.ip1_val_b[t] + acc, 0.f);
+            }
+            const float sum = block_reduce(v, scratch, false);
+            if (t == 0) winrate[pos] = (1.0f + tanhf(h.ip2_val_b[0] + sum)) / 2.0f;
+        }
+        if (pos + static_cast<int>(gridDim.x / kHeadCtas) < n) {
+            __syncthreads();
+            head_cluster_sync();          // the sums are read: the next position may overwrite them
+        }
+    }
 }
 
 }  // namespace lzb

@@ -32,6 +32,8 @@
 #include "gemm_simt.cuh"
 #include "gemm_tcgen05.cuh"
 #include "head_kernels.cuh"
+#include "input_view.cuh"
+#include "pack_planes.h"
 #include "transform_kernels.cuh"
 
 namespace {
@@ -66,6 +68,7 @@ inline int round_up(int v, int m) { return (v + m - 1) / m * m; }
 constexpr int kXformSmem = lzb::kBoardCells * 32 * 8;   // fp32 board of one position x 64 channels
 constexpr int kMaxMicroBatch = 256;      // rows of V/M allocated: 25 * 256 = 6400
 constexpr int kDefaultMicroBatch = 64;
+constexpr int kMaxStaged = 1024;         // positions of a host call staged at a time
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
                                   const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
@@ -216,10 +219,14 @@ struct lzb_ctx {
     int Pa = 0;            // rows of V and M (multiple of 128)
     cudaStream_t stream = nullptr;
     void *V = nullptr, *M = nullptr, *X = nullptr;
-    float *d_in = nullptr, *d_pol = nullptr, *d_val = nullptr;
-    float *d_policy = nullptr, *d_winrate = nullptr;
-    unsigned int* d_packed = nullptr;   // bit-packed input planes [max_batch][18][12]
-    // One-launch tower: arrival counters of the tiles, two sets of [layers][tile_cap]
+    // host calls: positions and results on either side of the bus, stage_cap positions
+    int stage_cap = 0;
+    float* d_in = nullptr;              // fp32 planes (positions that are not 0 / 1)
+    unsigned int* d_packed = nullptr;   // bit planes [18][12]
+    float* d_out = nullptr;             // results, out0 then out1 (see Job)
+    unsigned int* h_packed = nullptr;   // page-locked
+    float* h_out = nullptr;             // page-locked
+    // One-launch tower: arrival counters of the tiles, two sets of [layers + 1][tile_cap]
     // words used in turn (a run clears the other set); null: a launch per layer
     uint32_t* tile_counts = nullptr;
     int tile_cap = 0;
@@ -233,6 +240,7 @@ struct lzb_ctx {
     CUtensorMap tmIN, tmX, tmH;      // window loads
     CUtensorMap tmXo, tmHo;          // 32 x 32 output stores
     CUtensorMap tmXl, tmHl;          // e5m2 planes of X and H: 128-byte windows (LZB_FP16_X2)
+    CUtensorMap tmXlo, tmHlo;        // ... and their 32 x 32 output stores
     long long launches = 0;
     // per-launch timing (diagnostics): event pairs tagged with a kernel class
     bool profiling = false;
@@ -401,9 +409,65 @@ int launch_xform(lzb_ctx* c, const Layer& L, int nb, const T* R, T* X_out, T* V)
     return LZB_OK;
 }
 
+// What an evaluation reads and where its results go (device-accessible pointers:
+// device memory or page-locked host memory).
+struct Job {
+    InputView in;
+    bool heads;                   // policy and winrate, else raw planes
+    float *out0, *out1;           // pol [n][2][361], val [n][361]  or  policy [n][362], winrate [n]
+    float inv_temp;
+    int* err_out;                 // receives the error word with the results, or null
+    Job from(int pos) const {
+        Job j = *this;
+        j.in = in.from(pos);
+        j.out0 += static_cast<size_t>(pos) * (heads ? LZB_MOVES : LZB_POL_FLOATS);
+        j.out1 += static_cast<size_t>(pos) * (heads ? 1 : LZB_VAL_FLOATS);
+        return j;
+    }
+};
+
+// The last launch of an evaluation: 1x1 head convolutions, and the heads where the
+// job wants them.  Programmatic launch: its blocks are placed as soon as there is
+// room (the tower leaves SMs free in small batches) and fetch their weights while
+// the tower still runs.
+template <typename T, bool kCells>
+int launch_heads(lzb_ctx* c, const Job& job, int nb, int ldx, int lo_off, int lo_e5m2) {
+    lzb_pipe* p = c->pipe;
+    cudaLaunchConfig_t cfg = {};
+    cfg.stream = c->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const T* X = static_cast<const T*>(c->X);
+    cudaError_t le;
+    {
+        LaunchScope scope(c, kClassHead);
+        if (job.heads) {
+            const Heads& h = p->heads;
+            const HeadWeights hw = {h.bn_pol_mean, h.bn_pol_invstd, h.ip_pol_wT, h.ip_pol_b, h.bn_val_mean,
+                                    h.bn_val_invstd, h.ip1_val_wT, h.ip1_val_b, h.ip2_val_w, h.ip2_val_b};
+            // one CTA per SM: more positions than clusters fit share a cluster's weights
+            cfg.gridDim = dim3(kHeadCtas * std::min(nb, p->sm_count / kHeadCtas));
+            cfg.blockDim = dim3(kHeadThreads);
+            le = cudaLaunchKernelEx(&cfg, heads_kernel<T, kCells>, X, (const float*)p->head_w, p->Cp, nb, ldx, lo_off,
+                                    lo_e5m2, hw, job.inv_temp, job.out0, job.out1, (const int*)c->d_err, job.err_out);
+        } else {
+            cfg.gridDim = dim3((nb * kSq + 31) / 32);
+            cfg.blockDim = dim3(256);
+            le = cudaLaunchKernelEx(&cfg, head_planes_kernel<T, kCells>, X, (const float*)p->head_w, p->Cp, nb,
+                                    job.out0, job.out1, ldx, lo_off, lo_e5m2, (const int*)c->d_err, job.err_out);
+        }
+    }
+    LZB_CUDA(le);
+    LZB_CUDA(cudaGetLastError());
+    return LZB_OK;
+}
+
 // One micro-batch (nb positions, device pointers) through the whole tower.
 template <typename T>
-int run_tower(lzb_ctx* c, const float* in_dev, int nb, float* pol_dev, float* val_dev) {
+int run_tower(lzb_ctx* c, const Job& job, int nb) {
     lzb_pipe* p = c->pipe;
     const int P = nb * kTilesPerPos;
     T* V = static_cast<T*>(c->V);
@@ -411,7 +475,7 @@ int run_tower(lzb_ctx* c, const float* in_dev, int nb, float* pol_dev, float* va
     int rc;
     {
         LaunchScope scope(c, kClassInput);
-        first_in_transform_kernel<T><<<(P + 7) / 8, 256, 0, c->stream>>>(in_dev, V, c->Pa, P);
+        first_in_transform_kernel<T><<<(P + 7) / 8, 256, 0, c->stream>>>(job.in, V, c->Pa, P);
     }
     LZB_CUDA(cudaGetLastError());
     if ((rc = contraction<T>(c, p->layers[0], P, true))) return rc;
@@ -425,14 +489,7 @@ int run_tower(lzb_ctx* c, const float* in_dev, int nb, float* pol_dev, float* va
         const bool last = (b + 1 == p->blocks);
         if ((rc = launch_xform<T>(c, l2, nb, X, X, last ? nullptr : V))) return rc;
     }
-    const int cells = nb * kSq;
-    {
-        LaunchScope scope(c, kClassHead);
-        head_conv_kernel<T><<<(cells + 7) / 8, 256, 0, c->stream>>>(X, p->head_w, p->Cp, cells,
-                                                                     pol_dev, val_dev);
-    }
-    LZB_CUDA(cudaGetLastError());
-    return LZB_OK;
+    return launch_heads<T, false>(c, job, nb, p->Cp, 0, 0);
 }
 
 template <typename T>
@@ -538,12 +595,12 @@ int tower_slices(const lzb_pipe* p, int npairs) {
 // All 3x3 layers of one micro-batch in one cooperative launch.  A launch that is
 // refused is reported in *refused and not an error.
 template <typename T>
-int launch_tower(lzb_ctx* c, int nb, bool* refused) {
+int launch_tower(lzb_ctx* c, const InputView& in, int nb, bool* refused) {
     lzb_pipe* p = c->pipe;
     const int ntiles = dct::kTilesPerPos128 * nb, npairs = (ntiles + 1) / 2;
     const int ns = tower_slices(p, npairs);
     const int n_layers = static_cast<int>(p->layers.size());
-    const size_t words = static_cast<size_t>(n_layers) * c->tile_cap;
+    const size_t words = static_cast<size_t>(n_layers + 1) * c->tile_cap;
     uint32_t* counts = c->tile_counts + (c->tower_runs & 1u) * words;
     uint32_t* counts_next = c->tile_counts + ((c->tower_runs & 1u) ^ 1u) * words;
     cudaLaunchConfig_t cfg = {};
@@ -565,8 +622,8 @@ int launch_tower(lzb_ctx* c, int nb, bool* refused) {
     LaunchScope scope(c, kClassContraction, n_layers);
     cudaError_t le = cudaLaunchKernelEx(
         &cfg, kernel, c->tmIN, c->tmX, c->tmH, bytes ? c->tmXl : c->tmX, bytes ? c->tmHl : c->tmH, c->tmXo, c->tmHo,
-        (const dct::TowerLayer*)p->tower_table[ns], n_layers, static_cast<T*>(c->X), static_cast<T*>(c->H), ntiles,
-        p->Cp, ns, p->row_bytes() / p->elt, p->row_bytes(), counts, counts_next, c->tile_cap, c->d_err);
+        bytes ? c->tmXlo : c->tmXo, bytes ? c->tmHlo : c->tmHo, (const dct::TowerLayer*)p->tower_table[ns], n_layers, in, static_cast<T*>(c->IN), static_cast<T*>(c->X),
+        static_cast<T*>(c->H), ntiles, p->Cp, ns, p->row_bytes() / p->elt, counts, counts_next, c->tile_cap, c->d_err);
     if (le == cudaSuccess) le = cudaGetLastError();
     *refused = le != cudaSuccess;
     if (*refused) {
@@ -585,19 +642,18 @@ int launch_tower(lzb_ctx* c, int nb, bool* refused) {
 // (lzb_ctx_profile_begin) or the one launch is not available, a launch per layer;
 // batch-norm / residual / ReLU in the epilogue either way.
 template <typename T>
-int run_tower_direct(lzb_ctx* c, const float* in_dev, int nb, float* pol_dev, float* val_dev) {
+int run_tower_direct(lzb_ctx* c, const Job& job, int nb) {
     lzb_pipe* p = c->pipe;
     T* X = static_cast<T*>(c->X);
     int rc;
-    {
-        LaunchScope scope(c, kClassInput);
-        dc::input_to_cells_kernel<T><<<p->sm_count * 4, 256, 0, c->stream>>>(
-            in_dev, static_cast<T*>(c->IN), nb);
-    }
-    LZB_CUDA(cudaGetLastError());
     bool per_layer = c->tile_counts == nullptr || p->tower_refused || c->profiling;
-    if (!per_layer && (rc = launch_tower<T>(c, nb, &per_layer))) return rc;
+    if (!per_layer && (rc = launch_tower<T>(c, job.in, nb, &per_layer))) return rc;
     if (per_layer) {
+        {
+            LaunchScope scope(c, kClassInput);
+            dc::input_to_cells_kernel<T><<<p->sm_count * 4, 256, 0, c->stream>>>(job.in, static_cast<T*>(c->IN), nb);
+        }
+        LZB_CUDA(cudaGetLastError());
         if ((rc = launch_conv_direct<T>(c, p->layers[0], nb, c->tmIN, c->tmXo, nullptr, nullptr, c->X))) return rc;
         for (int b = 0; b < p->blocks; b++) {
             if ((rc = launch_conv_direct<T>(c, p->layers[1 + 2 * b], nb, c->tmX, c->tmHo, nullptr, &c->tmXl,
@@ -609,28 +665,18 @@ int run_tower_direct(lzb_ctx* c, const float* in_dev, int nb, float* pol_dev, fl
             }
         }
     }
-    const int cells = nb * kSq;
-    {
-        LaunchScope scope(c, kClassHead);
-        dc::head_conv_cells_kernel<T><<<(cells + 7) / 8, 256, 0, c->stream>>>(
-            X, p->head_w, p->Cp, cells, pol_dev, val_dev, p->row_bytes() / p->elt,
-            (p->aplanes == 2 || (p->aplanes == 3 && p->layers.back().out_lo)) ? p->Cp : 0,
-            p->aplanes == 3 ? 1 : 0);
-    }
-    LZB_CUDA(cudaGetLastError());
-    return LZB_OK;
+    return launch_heads<T, true>(c, job, nb, p->row_bytes() / p->elt,
+                                 (p->aplanes == 2 || (p->aplanes == 3 && p->layers.back().out_lo)) ? p->Cp : 0,
+                                 p->aplanes == 3 ? 1 : 0);
 }
-int run_tower_any(lzb_ctx* c, const float* in_dev, int nb, float* pol_dev, float* val_dev) {
+
+int run_tower_any(lzb_ctx* c, const Job& job, int nb) {
+    const bool half = c->pipe->precision == LZB_FP16;
     if (c->pipe->direct) {
-        return c->pipe->precision == LZB_FP16
-                   ? run_tower_direct<__half>(c, in_dev, nb, pol_dev, val_dev)
-                   : run_tower_direct<__nv_bfloat16>(c, in_dev, nb, pol_dev, val_dev);
+        return half ? run_tower_direct<__half>(c, job, nb) : run_tower_direct<__nv_bfloat16>(c, job, nb);
     }
-    switch (c->pipe->precision) {
-        case LZB_FP32: return run_tower<float>(c, in_dev, nb, pol_dev, val_dev);
-        case LZB_FP16: return run_tower<__half>(c, in_dev, nb, pol_dev, val_dev);
-        default: return run_tower<__nv_bfloat16>(c, in_dev, nb, pol_dev, val_dev);
-    }
+    if (c->pipe->precision == LZB_FP32) return run_tower<float>(c, job, nb);
+    return half ? run_tower<__half>(c, job, nb) : run_tower<__nv_bfloat16>(c, job, nb);
 }
 
 int check_ctx(lzb_ctx* c, int n) {
@@ -731,7 +777,7 @@ int debug_conv_direct_t(lzb_ctx* c, int layer, const float* in, int n, const flo
     T* H = static_cast<T*>(c->H);
     guard(cudaMemcpyAsync(stage, in, sizeof(float) * in_floats, cudaMemcpyHostToDevice, c->stream), "copy in");
     if (layer == 0) {
-        dc::input_to_cells_kernel<T><<<512, 256, 0, c->stream>>>(stage, static_cast<T*>(c->IN), n);
+        dc::input_to_cells_kernel<T><<<512, 256, 0, c->stream>>>(InputView{stage, nullptr}, static_cast<T*>(c->IN), n);
     } else {
         dc::nchw_to_cells_kernel<T><<<512, 256, 0, c->stream>>>(stage, H, n, C, p->Cp);
     }
@@ -772,7 +818,7 @@ int debug_conv_t(lzb_ctx* c, int layer, const float* in, int n, const float* res
     };
     if (layer == 0) {
         guard(cudaMemcpyAsync(stage, in, sizeof(float) * n * LZB_IN_FLOATS, cudaMemcpyHostToDevice, c->stream), "copy in");
-        first_in_transform_kernel<T><<<(P + 7) / 8, 256, 0, c->stream>>>(stage, V, c->Pa, P);
+        first_in_transform_kernel<T><<<(P + 7) / 8, 256, 0, c->stream>>>(InputView{stage, nullptr}, V, c->Pa, P);
     } else {
         guard(cudaMemcpyAsync(stage, in, sizeof(float) * plane_floats, cudaMemcpyHostToDevice, c->stream), "copy in");
         nchw_to_nhwc_kernel<T><<<512, 256, 0, c->stream>>>(stage, X, n, C, p->Cp);
@@ -1289,7 +1335,7 @@ int lzb_ctx_create(lzb_ctx** out, lzb_pipe* p, int max_batch) {
         const char* tf = getenv("LZB_TILE_FLAGS");
         if (p->tower_pairs > 0 && !(tf != nullptr && atoi(tf) == 0)) {
             c->tile_cap = (dct::kTilesPerPos128 * c->micro_cap + 1) / 2;
-            alloc((void**)&c->tile_counts, (size_t)2 * (1 + 2 * p->blocks) * c->tile_cap * sizeof(uint32_t));
+            alloc((void**)&c->tile_counts, (size_t)2 * (2 + 2 * p->blocks) * c->tile_cap * sizeof(uint32_t));
         }
     } else {
         c->micro = default_micro_batch(p, c->micro_cap);
@@ -1299,14 +1345,17 @@ int lzb_ctx_create(lzb_ctx** out, lzb_pipe* p, int max_batch) {
         alloc(&c->M, vm);
         alloc(&c->X, (size_t)c->micro_cap * kSq * p->Cp * p->elt);
     }
-    alloc((void**)&c->d_in, (size_t)max_batch * LZB_IN_FLOATS * sizeof(float));
-    alloc((void**)&c->d_pol, (size_t)max_batch * LZB_POL_FLOATS * sizeof(float));
-    alloc((void**)&c->d_val, (size_t)max_batch * LZB_VAL_FLOATS * sizeof(float));
-    alloc((void**)&c->d_policy, (size_t)max_batch * LZB_MOVES * sizeof(float));
-    alloc((void**)&c->d_winrate, (size_t)max_batch * sizeof(float));
-    alloc((void**)&c->d_packed, (size_t)max_batch * LZB_PACKED_WORDS * sizeof(unsigned int));
+    c->stage_cap = std::min(max_batch, kMaxStaged);
+    const size_t out_floats = (size_t)c->stage_cap * (LZB_POL_FLOATS + LZB_VAL_FLOATS);
+    alloc((void**)&c->d_in, (size_t)c->stage_cap * LZB_IN_FLOATS * sizeof(float));
+    alloc((void**)&c->d_packed, (size_t)c->stage_cap * LZB_PACKED_WORDS * sizeof(unsigned int));
+    alloc((void**)&c->d_out, out_floats * sizeof(float));
     alloc((void**)&c->d_err, sizeof(int));
     if (e == cudaSuccess) e = cudaMallocHost((void**)&c->h_err, sizeof(int));
+    if (e == cudaSuccess) {
+        e = cudaMallocHost((void**)&c->h_packed, (size_t)c->stage_cap * LZB_PACKED_WORDS * sizeof(unsigned int));
+    }
+    if (e == cudaSuccess) e = cudaMallocHost((void**)&c->h_out, out_floats * sizeof(float));
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) {
         const int code = (e == cudaErrorMemoryAllocation) ? LZB_ERR_NOMEM : LZB_ERR_CUDA;
@@ -1333,6 +1382,9 @@ int lzb_ctx_create(lzb_ctx** out, lzb_pipe* p, int max_batch) {
             const uint64_t lb = (uint64_t)p->Cp * (p->wlo_layers > 1 ? 2 : 1);
             if (!rc) rc = make_map_2d(&c->tmXl, -1, xl, (uint64_t)c->Qa, lb, dc::kWinRows, 128, sw128, pitch);
             if (!rc) rc = make_map_2d(&c->tmHl, -1, hl, (uint64_t)c->Qa, lb, dc::kWinRows, 128, sw128, pitch);
+            const CUtensorMapSwizzle sw0 = CU_TENSOR_MAP_SWIZZLE_NONE;
+            if (!rc) rc = make_map_2d(&c->tmXlo, -1, xl, (uint64_t)c->Qa, lb, 32, 32, sw0, pitch);
+            if (!rc) rc = make_map_2d(&c->tmHlo, -1, hl, (uint64_t)c->Qa, lb, 32, 32, sw0, pitch);
         }
         if (rc) {
             lzb_ctx_destroy(c);
@@ -1357,9 +1409,12 @@ void lzb_ctx_destroy(lzb_ctx* c) {
         cudaStreamSynchronize(c->stream);
         cudaStreamDestroy(c->stream);
     }
-    void* ptrs[] = {c->V, c->M, c->X, c->IN, c->H, c->d_in, c->d_pol, c->d_val, c->d_policy, c->d_winrate, c->d_packed, c->d_err, c->tile_counts};
+    void* ptrs[] = {c->V, c->M, c->X, c->IN, c->H, c->d_in, c->d_packed, c->d_out, c->d_err, c->tile_counts};
     for (void* q : ptrs) cudaFree(q);
-    if (c->h_err) cudaFreeHost(c->h_err);
+    void* pinned[] = {c->h_err, c->h_packed, c->h_out};
+    for (void* q : pinned) {
+        if (q) cudaFreeHost(q);
+    }
     delete c;
 }
 
@@ -1377,19 +1432,131 @@ long long lzb_ctx_launch_count(const lzb_ctx* c) { return c ? c->launches : 0; }
 
 void* lzb_ctx_stream(lzb_ctx* c) { return c ? (void*)c->stream : nullptr; }
 
+namespace {
+// Enqueue n positions, cut into micro-batches.
+int enqueue(lzb_ctx* c, const Job& job, int n) {
+    for (int off = 0; off < n; off += c->micro) {
+        const int nb = (n - off) < c->micro ? (n - off) : c->micro;
+        const int rc = run_tower_any(c, job.from(off), nb);
+        if (rc) return rc;
+    }
+    return LZB_OK;
+}
+
+int check_heads(lzb_ctx* c, float softmax_temp) {
+    if (!c->pipe->heads.present) return fail(LZB_ERR_ARG, "head weights were not pushed");
+    if (!(softmax_temp > 0.f)) return fail(LZB_ERR_ARG, "softmax temperature must be positive");
+    return LZB_OK;
+}
+
+// The error word has reached the host: clear what an abandoned run left behind.
+int collect_error(lzb_ctx* c) {
+    if (*c->h_err == 0) return LZB_OK;
+    const int code = *c->h_err;
+    *c->h_err = 0;
+    cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream);
+    if (c->tile_counts != nullptr) {
+        cudaMemsetAsync(c->tile_counts, 0, (size_t)2 * (2 + 2 * c->pipe->blocks) * c->tile_cap * sizeof(uint32_t),
+                        c->stream);
+    }
+    return fail(LZB_ERR_DEVICE_WAIT, "a kernel gave up a bounded wait (code " + std::to_string(code) + ")");
+}
+
+// Page-locked memory the GPU can address directly?
+bool gpu_visible(const void* ptr) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, ptr) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeHost && a.devicePointer == ptr;
+}
+
+// A blocking evaluation of host buffers: positions as fp32 planes or as bits, and
+// out0 / out1 as in Job.  Positions go over the bus as bits whenever their values
+// are 0 and 1 (864 bytes instead of 26 KB).  A copy engine operation costs 5-8 us
+// however few bytes it moves, so up to kDirectPositions the kernels read the bits
+// from and write the results to page-locked memory themselves; the error word comes
+// back the same way.  Larger batches are copied, straight from and to the caller's
+// buffers where those are page-locked, else through the context's own.
+constexpr int kDirectPositions = 32;
+
+int run_host(lzb_ctx* c, const float* planes, const unsigned int* packed, int n, bool heads, float softmax_temp,
+             float* out0, float* out1) {
+    int rc = check_ctx(c, n);
+    if (rc) return rc;
+    if (heads && (rc = check_heads(c, softmax_temp))) return rc;
+    if ((!planes && !packed) || !out0 || !out1) return fail(LZB_ERR_ARG, "null buffer");
+    LZB_CUDA(enter_device(c->pipe->device));
+    const int w0 = heads ? LZB_MOVES : LZB_POL_FLOATS, w1 = heads ? 1 : LZB_VAL_FLOATS;
+    for (int off = 0; off < n; off += c->stage_cap) {
+        const int m = std::min(c->stage_cap, n - off);
+        Job job = {};
+        job.heads = heads;
+        job.inv_temp = heads ? 1.0f / softmax_temp : 1.0f;
+        job.err_out = c->h_err;
+        const unsigned int* bits = c->h_packed;
+        if (packed) {
+            const unsigned int* src = packed + (size_t)off * LZB_PACKED_WORDS;
+            if (m > kDirectPositions && gpu_visible(src)) bits = src;
+            else std::memcpy(c->h_packed, src, (size_t)m * LZB_PACKED_WORDS * sizeof(unsigned int));
+        } else {
+            for (int i = 0; i < m && bits; i++) {
+                if (!pack_position(planes + (size_t)(off + i) * LZB_IN_FLOATS,
+                                   c->h_packed + (size_t)i * LZB_PACKED_WORDS)) {
+                    bits = nullptr;
+                }
+            }
+        }
+        if (bits == nullptr) {
+            LZB_CUDA(cudaMemcpyAsync(c->d_in, planes + (size_t)off * LZB_IN_FLOATS,
+                                     (size_t)m * LZB_IN_FLOATS * sizeof(float), cudaMemcpyHostToDevice, c->stream));
+            job.in.f32 = c->d_in;
+        } else if (m <= kDirectPositions) {
+            job.in.bits = bits;
+        } else {
+            LZB_CUDA(cudaMemcpyAsync(c->d_packed, bits, (size_t)m * LZB_PACKED_WORDS * sizeof(unsigned int),
+                                     cudaMemcpyHostToDevice, c->stream));
+            job.in.bits = c->d_packed;
+        }
+        float *to0 = out0 + (size_t)off * w0, *to1 = out1 + (size_t)off * w1;
+        const size_t n0 = (size_t)m * w0, n1 = (size_t)m * w1;
+        const bool direct = m <= kDirectPositions;
+        job.out0 = direct ? c->h_out : c->d_out;
+        job.out1 = job.out0 + n0;
+        if ((rc = enqueue(c, job, m))) return rc;
+        bool staged = true;
+        if (!direct) {
+            staged = !(gpu_visible(to0) && gpu_visible(to1));
+            if (staged) {
+                LZB_CUDA(cudaMemcpyAsync(c->h_out, c->d_out, (n0 + n1) * sizeof(float), cudaMemcpyDeviceToHost,
+                                         c->stream));
+            } else {
+                LZB_CUDA(cudaMemcpyAsync(to0, c->d_out, n0 * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
+                LZB_CUDA(cudaMemcpyAsync(to1, c->d_out + n0, n1 * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
+            }
+        }
+        LZB_CUDA(cudaStreamSynchronize(c->stream));
+        if ((rc = collect_error(c))) return rc;
+        if (staged) {
+            std::memcpy(to0, c->h_out, n0 * sizeof(float));
+            std::memcpy(to1, c->h_out + n0, n1 * sizeof(float));
+        }
+    }
+    return LZB_OK;
+}
+}  // namespace
+
 int lzb_ctx_forward_device(lzb_ctx* c, const float* in_dev, int n, float* pol_dev, float* val_dev) {
     int rc = check_ctx(c, n);
     if (rc) return rc;
     if (!in_dev || !pol_dev || !val_dev) return fail(LZB_ERR_ARG, "null buffer");
     LZB_CUDA(enter_device(c->pipe->device));
-    for (int off = 0; off < n; off += c->micro) {
-        const int nb = (n - off) < c->micro ? (n - off) : c->micro;
-        rc = run_tower_any(c, in_dev + (size_t)off * LZB_IN_FLOATS, nb,
-                           pol_dev + (size_t)off * LZB_POL_FLOATS,
-                           val_dev + (size_t)off * LZB_VAL_FLOATS);
-        if (rc) return rc;
-    }
-    return LZB_OK;
+    Job job = {};
+    job.in.f32 = in_dev;
+    job.out0 = pol_dev;
+    job.out1 = val_dev;
+    return enqueue(c, job, n);
 }
 
 int lzb_ctx_sync(lzb_ctx* c) {
@@ -1397,77 +1564,41 @@ int lzb_ctx_sync(lzb_ctx* c) {
     LZB_CUDA(enter_device(c->pipe->device));
     LZB_CUDA(cudaMemcpyAsync(c->h_err, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     LZB_CUDA(cudaStreamSynchronize(c->stream));
-    if (*c->h_err != 0) {
-        const int code = *c->h_err;
-        *c->h_err = 0;
-        cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream);
-        if (c->tile_counts != nullptr) {
-            // an abandoned run leaves its counters short
-            cudaMemsetAsync(c->tile_counts, 0,
-                            (size_t)2 * (1 + 2 * c->pipe->blocks) * c->tile_cap * sizeof(uint32_t), c->stream);
-        }
-        return fail(LZB_ERR_DEVICE_WAIT,
-                    "a kernel gave up a bounded wait (code " + std::to_string(code) + ")");
-    }
-    return LZB_OK;
+    return collect_error(c);
 }
 
 int lzb_ctx_forward(lzb_ctx* c, const float* in, int n, float* pol, float* val) {
-    int rc = check_ctx(c, n);
-    if (rc) return rc;
-    if (!in || !pol || !val) return fail(LZB_ERR_ARG, "null buffer");
-    LZB_CUDA(enter_device(c->pipe->device));
-    LZB_CUDA(cudaMemcpyAsync(c->d_in, in, (size_t)n * LZB_IN_FLOATS * sizeof(float),
-                             cudaMemcpyHostToDevice, c->stream));
-    if ((rc = lzb_ctx_forward_device(c, c->d_in, n, c->d_pol, c->d_val))) return rc;
-    LZB_CUDA(cudaMemcpyAsync(pol, c->d_pol, (size_t)n * LZB_POL_FLOATS * sizeof(float),
-                             cudaMemcpyDeviceToHost, c->stream));
-    LZB_CUDA(cudaMemcpyAsync(val, c->d_val, (size_t)n * LZB_VAL_FLOATS * sizeof(float),
-                             cudaMemcpyDeviceToHost, c->stream));
-    return lzb_ctx_sync(c);
+    return run_host(c, in, nullptr, n, false, 1.0f, pol, val);
+}
+
+int lzb_ctx_forward_packed(lzb_ctx* c, const unsigned int* planes, int n, float* pol, float* val) {
+    return run_host(c, nullptr, planes, n, false, 1.0f, pol, val);
+}
+
+int lzb_ctx_forward_heads(lzb_ctx* c, const float* in, int n, float softmax_temp, float* policy,
+                          float* winrate) {
+    return run_host(c, in, nullptr, n, true, softmax_temp, policy, winrate);
+}
+
+int lzb_ctx_forward_heads_packed(lzb_ctx* c, const unsigned int* planes, int n, float softmax_temp,
+                                 float* policy, float* winrate) {
+    return run_host(c, nullptr, planes, n, true, softmax_temp, policy, winrate);
 }
 
 int lzb_ctx_forward_heads_device(lzb_ctx* c, const float* in_dev, int n, float softmax_temp,
                                  float* policy_dev, float* winrate_dev) {
     int rc = check_ctx(c, n);
     if (rc) return rc;
-    if (!c->pipe->heads.present) return fail(LZB_ERR_ARG, "head weights were not pushed");
-    if (!(softmax_temp > 0.f)) return fail(LZB_ERR_ARG, "softmax temperature must be positive");
-    if (!policy_dev || !winrate_dev) return fail(LZB_ERR_ARG, "null buffer");
-    if ((rc = lzb_ctx_forward_device(c, in_dev, n, c->d_pol, c->d_val))) return rc;
-    const Heads& h = c->pipe->heads;
-    {
-        LaunchScope scope(c, kClassHead);
-        policy_head_kernel<<<n * kPolicySlices, 384, 0, c->stream>>>(c->d_pol, h.bn_pol_mean, h.bn_pol_invstd,
-                                                     h.ip_pol_wT, h.ip_pol_b, 1.0f / softmax_temp,
-                                                     policy_dev);
-    }
-    {
-        LaunchScope scope(c, kClassHead);
-        value_head_kernel<<<n * kValueSlices, 256, 0, c->stream>>>(c->d_val, h.bn_val_mean, h.bn_val_invstd,
-                                                    h.ip1_val_wT, h.ip1_val_b, h.ip2_val_w,
-                                                    h.ip2_val_b, winrate_dev);
-    }
-    LZB_CUDA(cudaGetLastError());
-    return LZB_OK;
-}
-
-int lzb_ctx_forward_heads(lzb_ctx* c, const float* in, int n, float softmax_temp, float* policy,
-                          float* winrate) {
-    int rc = check_ctx(c, n);
-    if (rc) return rc;
-    if (!in || !policy || !winrate) return fail(LZB_ERR_ARG, "null buffer");
+    if ((rc = check_heads(c, softmax_temp))) return rc;
+    if (!in_dev || !policy_dev || !winrate_dev) return fail(LZB_ERR_ARG, "null buffer");
     LZB_CUDA(enter_device(c->pipe->device));
-    LZB_CUDA(cudaMemcpyAsync(c->d_in, in, (size_t)n * LZB_IN_FLOATS * sizeof(float),
-                             cudaMemcpyHostToDevice, c->stream));
-    if ((rc = lzb_ctx_forward_heads_device(c, c->d_in, n, softmax_temp, c->d_policy, c->d_winrate))) {
-        return rc;
-    }
-    LZB_CUDA(cudaMemcpyAsync(policy, c->d_policy, (size_t)n * LZB_MOVES * sizeof(float),
-                             cudaMemcpyDeviceToHost, c->stream));
-    LZB_CUDA(cudaMemcpyAsync(winrate, c->d_winrate, (size_t)n * sizeof(float),
-                             cudaMemcpyDeviceToHost, c->stream));
-    return lzb_ctx_sync(c);
+    Job job = {};
+    job.in.f32 = in_dev;
+    job.heads = true;
+    job.out0 = policy_dev;
+    job.out1 = winrate_dev;
+    job.inv_temp = 1.0f / softmax_temp;
+    return enqueue(c, job, n);
 }
 
 // ---------------------------------------------------------------------------
@@ -1583,51 +1714,6 @@ int lzb_conv3x3_static(int device, const float* in_dev, int n, int c_in, int cha
     nhwc_to_nchw_kernel<float><<<128, 256, 0, stream>>>(X, out_dev, n, channels, Cp);
     LZB_CUDA(cudaGetLastError());
     return LZB_OK;
-}
-
-namespace {
-// Copy n bit-packed positions to the device and expand them into c->d_in.
-int stage_packed(lzb_ctx* c, const unsigned int* planes, int n) {
-    LZB_CUDA(cudaMemcpyAsync(c->d_packed, planes, (size_t)n * LZB_PACKED_WORDS * sizeof(unsigned int),
-                             cudaMemcpyHostToDevice, c->stream));
-    {
-        LaunchScope scope(c, kClassInput);
-        lzb::unpack_planes_kernel<<<c->pipe->sm_count * 2, 256, 0, c->stream>>>(c->d_packed, c->d_in, n);
-    }
-    LZB_CUDA(cudaGetLastError());
-    return LZB_OK;
-}
-}  // namespace
-
-int lzb_ctx_forward_packed(lzb_ctx* c, const unsigned int* planes, int n, float* pol, float* val) {
-    int rc = check_ctx(c, n);
-    if (rc) return rc;
-    if (!planes || !pol || !val) return fail(LZB_ERR_ARG, "null buffer");
-    LZB_CUDA(enter_device(c->pipe->device));
-    if ((rc = stage_packed(c, planes, n))) return rc;
-    if ((rc = lzb_ctx_forward_device(c, c->d_in, n, c->d_pol, c->d_val))) return rc;
-    LZB_CUDA(cudaMemcpyAsync(pol, c->d_pol, (size_t)n * LZB_POL_FLOATS * sizeof(float),
-                             cudaMemcpyDeviceToHost, c->stream));
-    LZB_CUDA(cudaMemcpyAsync(val, c->d_val, (size_t)n * LZB_VAL_FLOATS * sizeof(float),
-                             cudaMemcpyDeviceToHost, c->stream));
-    return lzb_ctx_sync(c);
-}
-
-int lzb_ctx_forward_heads_packed(lzb_ctx* c, const unsigned int* planes, int n, float softmax_temp,
-                                 float* policy, float* winrate) {
-    int rc = check_ctx(c, n);
-    if (rc) return rc;
-    if (!planes || !policy || !winrate) return fail(LZB_ERR_ARG, "null buffer");
-    LZB_CUDA(enter_device(c->pipe->device));
-    if ((rc = stage_packed(c, planes, n))) return rc;
-    if ((rc = lzb_ctx_forward_heads_device(c, c->d_in, n, softmax_temp, c->d_policy, c->d_winrate))) {
-        return rc;
-    }
-    LZB_CUDA(cudaMemcpyAsync(policy, c->d_policy, (size_t)n * LZB_MOVES * sizeof(float),
-                             cudaMemcpyDeviceToHost, c->stream));
-    LZB_CUDA(cudaMemcpyAsync(winrate, c->d_winrate, (size_t)n * sizeof(float),
-                             cudaMemcpyDeviceToHost, c->stream));
-    return lzb_ctx_sync(c);
 }
 
 int lzb_ctx_debug_wait_probe(lzb_ctx* c, int limit_ms) {

@@ -13,6 +13,7 @@
 // out_transform_fused_bn_in OpenCL kernels (src/kernels/convolve3.opencl:109-452)
 // and follow the arithmetic of src/CPUPipe.cpp:63-183, 212-284, 352-377.
 #pragma once
+#include "input_view.cuh"
 #include "winograd_math.cuh"
 
 namespace lzb {
@@ -72,13 +73,12 @@ __device__ __forceinline__ void zero_halo(float2* board, int warp, int lane, int
 }
 
 // ---------------------------------------------------------------------------
-// Input planes of the network: in[n][18][361] fp32 (as the engine builds them,
-// src/Network.cpp:935-966) -> V[36][Pa][64], channels 18..63 zero.
+// Input planes of the network -> V[36][Pa][64], channels 18..63 zero.
 // One warp per tile, one lane per channel pair.
 // ---------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(256) first_in_transform_kernel(
-    const float* __restrict__ in, T* __restrict__ V, int Pa, int P) {
+    const InputView in, T* __restrict__ V, int Pa, int P) {
     using P2 = Pair<T>;
     const int lane = threadIdx.x & 31;
     const int p = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -87,8 +87,6 @@ __global__ void __launch_bounds__(256) first_in_transform_kernel(
     const int by = tile / kTilesPerSide, bx = tile % kTilesPerSide;
     const int c0 = 2 * lane;
     const bool live = c0 < kInputPlanes;   // 18 is even: pairs never straddle
-    const float* pl0 = in + ((size_t)n * kInputPlanes + (live ? c0 : 0)) * kSq;
-    const float* pl1 = pl0 + kSq;
 
     float2 t1[6][6];
 #pragma unroll
@@ -99,7 +97,7 @@ __global__ void __launch_bounds__(256) first_in_transform_kernel(
         for (int r = 0; r < 6; r++) {
             const int y = 4 * by - 1 + r;
             const bool inside = live && x >= 0 && x < kBoard && y >= 0 && y < kBoard;
-            vin[r] = inside ? make_float2(pl0[y * kBoard + x], pl1[y * kBoard + x])
+            vin[r] = inside ? make_float2(in.at(n, c0, y * kBoard + x), in.at(n, c0 + 1, y * kBoard + x))
                             : make_float2(0.f, 0.f);
         }
         apply_bt<Pair<T>::exact>(vout, vin);
@@ -239,46 +237,6 @@ __global__ void __launch_bounds__(XformShape<T>::warps * 32, XformShape<T>::ctas
 }
 
 // ---------------------------------------------------------------------------
-// The two 1x1 head convolutions (policy: 2 outputs, value: 1 output):
-//   out[o][s] = sum_c w[o][c] * X[n][s][c]          (src/CPUPipe.cpp:301-350)
-// One warp per board cell, lanes stride over channel pairs.  w is [3][Cp]
-// fp32: rows 0,1 policy, row 2 value.  Outputs are fp32 planes in the layout
-// ForwardPipe::forward returns: pol[n][2][361], val[n][361].
-// ---------------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(256) head_conv_kernel(
-    const T* __restrict__ X, const float* __restrict__ w, int Cp, int cells,
-    float* __restrict__ pol, float* __restrict__ val) {
-    using P2 = Pair<T>;
-    const int lane = threadIdx.x & 31;
-    const int cell = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (cell >= cells) return;
-    const T* x = X + (size_t)cell * Cp;
-    float a0 = 0.f, a1 = 0.f, a2 = 0.f;
-    for (int c = 2 * lane; c < Cp; c += 64) {
-        const float2 v = P2::to_f2(*reinterpret_cast<const typename P2::type*>(x + c));
-        const float2 w0 = *reinterpret_cast<const float2*>(w + c);
-        const float2 w1 = *reinterpret_cast<const float2*>(w + Cp + c);
-        const float2 w2 = *reinterpret_cast<const float2*>(w + 2 * Cp + c);
-        a0 += w0.x * v.x + w0.y * v.y;
-        a1 += w1.x * v.x + w1.y * v.y;
-        a2 += w2.x * v.x + w2.y * v.y;
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        a0 += __shfl_xor_sync(0xffffffffu, a0, off);
-        a1 += __shfl_xor_sync(0xffffffffu, a1, off);
-        a2 += __shfl_xor_sync(0xffffffffu, a2, off);
-    }
-    if (lane == 0) {
-        const int n = cell / kSq, s = cell % kSq;
-        pol[((size_t)n * 2 + 0) * kSq + s] = a0;
-        pol[((size_t)n * 2 + 1) * kSq + s] = a1;
-        val[(size_t)n * kSq + s] = a2;
-    }
-}
-
-// ---------------------------------------------------------------------------
 // Weight repack at upload time: U32[36][c_in][K] fp32 (engine layout,
 // src/Network.cpp:215) -> U[36][Kp][Cin_p] of type T, zero padded, input
 // channel innermost so that both contraction operands are K-major.
@@ -326,18 +284,6 @@ __global__ void transform_f_kernel(const float* __restrict__ f, float* __restric
                 for (int m = 0; m < 3; m++) acc = nf_add(acc, nf_mul(gf[xi][m], G[nu][m]));
                 U32[((size_t)(xi * 6 + nu) * c_in + c) * K + k] = acc;
             }
-    }
-}
-
-// Bit-packed planes [n][18][12] words -> fp32 planes [n][18][361] of 0 / 1.
-__global__ void unpack_planes_kernel(const unsigned int* __restrict__ packed, float* __restrict__ out,
-                                     int n) {
-    const size_t total = (size_t)n * kInputPlanes * kSq;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total;
-         i += (size_t)gridDim.x * blockDim.x) {
-        const int s = i % kSq;
-        const size_t plane = i / kSq;
-        out[i] = (packed[plane * 12 + (s >> 5)] >> (s & 31)) & 1u ? 1.0f : 0.0f;
     }
 }
 
