@@ -29,6 +29,7 @@
 #include "conv_direct.cuh"
 #include "conv_direct2.cuh"
 #include "conv_tower.cuh"
+#include "gemm_f32x3.cuh"
 #include "gemm_simt.cuh"
 #include "gemm_tcgen05.cuh"
 #include "head_kernels.cuh"
@@ -146,12 +147,13 @@ int make_weight_map(CUtensorMap* map, int precision, void* base, uint64_t rows, 
 }
 
 struct Layer {
-    void* U = nullptr;          // [36][Kp][cin_p] storage type
+    void* U = nullptr;          // [36][Kp][cin_p] storage type; fp32: [36][Kp][3][cin_p] bf16 planes
     float* mean = nullptr;      // [Kp]
     float* invstd = nullptr;    // [Kp]
     int cin_p = 0;
     bool present = false;
-    CUtensorMap tmU;
+    CUtensorMap tmU;            // Winograd modes: box 64 x Kp; fp32 (three planes): box 64 x 64
+    CUtensorMap tmU128;         // fp32: box 64 x 128
     void* Wd = nullptr;         // direct path: [9][Kp][cinw] storage type
     int cinw = 0;               // input-channel extent of Wd: cin_p x weight planes
     int achunks = 0;            // 64-channel chunks of the activation tensor this layer reads
@@ -234,6 +236,7 @@ struct lzb_ctx {
     int* d_err = nullptr;
     int* h_err = nullptr;  // pinned
     CUtensorMap tmV_first, tmV;
+    CUtensorMap tmV32_first, tmV32;  // fp32: boxes of 32 rows
     // direct path: padded cell-major activations
     int Qa = 0;            // rows allocated in IN / X / H
     void *IN = nullptr, *H = nullptr;
@@ -258,6 +261,14 @@ int upload_layer_t(lzb_pipe* p, Layer& L, const float* U32_dev, int c_in) {
     const size_t n = (size_t)kPoints * p->Cp * L.cin_p;
     LZB_CUDA(cudaMalloc(&L.U, n * sizeof(T)));
     repack_u_kernel<T><<<1024, 256>>>(U32_dev, static_cast<T*>(L.U), c_in, p->channels, L.cin_p, p->Cp);
+    LZB_CUDA(cudaGetLastError());
+    return LZB_OK;
+}
+
+int upload_layer_f32(lzb_pipe* p, Layer& L, const float* U32_dev, int c_in) {
+    const size_t n = (size_t)kPoints * p->Cp * L.cin_p * 3;
+    LZB_CUDA(cudaMalloc(&L.U, n * sizeof(__nv_bfloat16)));
+    repack_u3_kernel<<<1024, 256>>>(U32_dev, static_cast<__nv_bfloat16*>(L.U), c_in, p->channels, L.cin_p, p->Cp);
     LZB_CUDA(cudaGetLastError());
     return LZB_OK;
 }
@@ -319,28 +330,36 @@ struct LaunchScope {
     }
 };
 
-// fp32: FFMA contraction.
-int launch_gemm_f32(lzb_ctx* c, const Layer& L, int P) {
+// fp32: contraction as three bf16 planes (gemm_f32x3.cuh), persistent CTAs.
+// Items of 128 output channels, or of 64 where the SMs could take twice as many
+// (an MMA of N = 64 takes 49 cycles, one of N = 128 65: not worth it otherwise).
+bool gemm_f32_narrow(const lzb_pipe* p, int nblk) {
+    return p->Cp % 128 != 0 || 2 * kPoints * (p->Cp / 128) * nblk <= p->sm_count;
+}
+int launch_gemm_f32(lzb_ctx* c, const Layer& L, int P, bool first) {
     lzb_pipe* p = c->pipe;
+    const int nblk = (P + tc::kBlockM - 1) / tc::kBlockM;
+    const bool narrow = gemm_f32_narrow(p, nblk);
+    const int items = kPoints * (p->Cp / (narrow ? 64 : 128)) * nblk;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(std::min(items, p->sm_count));
+    cfg.blockDim = dim3(f3::kF3Threads);
+    cfg.dynamicSmemBytes = narrow ? f3::Shape<64>::smem : f3::Shape<128>::smem;
+    cfg.stream = c->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaError_t le;
     {
         LaunchScope scope(c, kClassContraction);
-        // 128-row tiles (V and M have Pa rows, a multiple of 128; rows beyond P
-        // are scratch), 128 output channels per tile where they divide evenly;
-        // persistent CTAs, two per SM
-        const int bn = p->Cp % 128 == 0 ? 128 : 64;
-        const int row_tiles = round_up(P, kSimtBigM) / kSimtBigM;
-        const int tiles = row_tiles * (p->Cp / bn) * kPoints;
-        const int grid = tiles < 2 * p->sm_count ? tiles : 2 * p->sm_count;
-        if (bn == 128) {
-            gemm_f32_big_kernel<128><<<grid, 256, 0, c->stream>>>(
-                static_cast<const float*>(c->V), static_cast<const float*>(L.U),
-                static_cast<float*>(c->M), c->Pa, L.cin_p, p->Cp, row_tiles);
-        } else {
-            gemm_f32_big_kernel<64><<<grid, 256, 0, c->stream>>>(
-                static_cast<const float*>(c->V), static_cast<const float*>(L.U),
-                static_cast<float*>(c->M), c->Pa, L.cin_p, p->Cp, row_tiles);
-        }
+        le = cudaLaunchKernelEx(&cfg, narrow ? f3::gemm_f32x3_kernel<64> : f3::gemm_f32x3_kernel<128>,
+                                first ? c->tmV_first : c->tmV, first ? c->tmV32_first : c->tmV32,
+                                narrow ? L.tmU : L.tmU128, static_cast<float*>(c->M), c->Pa, P, p->Cp, L.cin_p, nblk,
+                                c->d_err);
     }
+    LZB_CUDA(le);
     LZB_CUDA(cudaGetLastError());
     return LZB_OK;
 }
@@ -380,18 +399,17 @@ int contraction(lzb_ctx* c, const Layer& L, int P, bool first) {
     return launch_gemm_tc<T>(c, L, P, first);
 }
 template <>
-int contraction<float>(lzb_ctx* c, const Layer& L, int P, bool) {
-    return launch_gemm_f32(c, L, P);
+int contraction<float>(lzb_ctx* c, const Layer& L, int P, bool first) {
+    return launch_gemm_f32(c, L, P, first);
 }
 
 template <typename T>
-int launch_xform(lzb_ctx* c, const Layer& L, int nb, const T* R, T* X_out, T* V) {
+using VType = typename TileOut<T, PipeV<T>::split>::type;
+
+template <typename T>
+int launch_xform(lzb_ctx* c, const Layer& L, int nb, const T* R, T* X_out, VType<T>* V) {
     lzb_pipe* p = c->pipe;
-    const dim3 grid(p->Cp / kChanPerCta, nb);
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(XformShape<T>::warps * 32);
-    cfg.dynamicSmemBytes = kXformSmem;
     cfg.stream = c->stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -401,8 +419,18 @@ int launch_xform(lzb_ctx* c, const Layer& L, int nb, const T* R, T* X_out, T* V)
     cudaError_t le;
     {
         LaunchScope scope(c, kClassTransform);
-        le = cudaLaunchKernelEx(&cfg, xform_kernel<T>, static_cast<const T*>(c->M), c->Pa, p->Cp,
-                                (const float*)L.mean, (const float*)L.invstd, R, X_out, V);
+        if constexpr (std::is_same<T, float>::value) {
+            cfg.gridDim = dim3(p->Cp / kXf32Chan, nb);
+            cfg.blockDim = dim3(kXf32Threads);
+            le = cudaLaunchKernelEx(&cfg, xform_f32_kernel, static_cast<const float*>(c->M), c->Pa, p->Cp,
+                                    (const float*)L.mean, (const float*)L.invstd, R, X_out, V);
+        } else {
+            cfg.gridDim = dim3(p->Cp / kChanPerCta, nb);
+            cfg.blockDim = dim3(XformShape<T>::warps * 32);
+            cfg.dynamicSmemBytes = kXformSmem;
+            le = cudaLaunchKernelEx(&cfg, xform_kernel<T>, static_cast<const T*>(c->M), c->Pa, p->Cp,
+                                    (const float*)L.mean, (const float*)L.invstd, R, X_out, V);
+        }
     }
     LZB_CUDA(le);
     LZB_CUDA(cudaGetLastError());
@@ -470,12 +498,12 @@ template <typename T>
 int run_tower(lzb_ctx* c, const Job& job, int nb) {
     lzb_pipe* p = c->pipe;
     const int P = nb * kTilesPerPos;
-    T* V = static_cast<T*>(c->V);
+    VType<T>* V = static_cast<VType<T>*>(c->V);
     T* X = static_cast<T*>(c->X);
     int rc;
     {
         LaunchScope scope(c, kClassInput);
-        first_in_transform_kernel<T><<<(P + 7) / 8, 256, 0, c->stream>>>(job.in, V, c->Pa, P);
+        first_in_transform_kernel<T, PipeV<T>::split><<<(P + 7) / 8, 256, 0, c->stream>>>(job.in, V, c->Pa, P);
     }
     LZB_CUDA(cudaGetLastError());
     if ((rc = contraction<T>(c, p->layers[0], P, true))) return rc;
@@ -690,9 +718,7 @@ int check_ctx(lzb_ctx* c, int n) {
 }
 
 int set_smem_attrs() {
-    LZB_CUDA(cudaFuncSetAttribute(xform_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  kXformSmem));
-    LZB_CUDA(cudaFuncSetAttribute(in_transform_kernel<float>,
+    LZB_CUDA(cudaFuncSetAttribute(in_transform_kernel<float, false>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   kXformSmem));
     LZB_CUDA(cudaFuncSetAttribute(xform_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -700,12 +726,16 @@ int set_smem_attrs() {
     LZB_CUDA(cudaFuncSetAttribute(xform_kernel<__nv_bfloat16>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   kXformSmem));
-    LZB_CUDA(cudaFuncSetAttribute(in_transform_kernel<__half>,
+    LZB_CUDA(cudaFuncSetAttribute(in_transform_kernel<__half, false>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   kXformSmem));
-    LZB_CUDA(cudaFuncSetAttribute(in_transform_kernel<__nv_bfloat16>,
+    LZB_CUDA(cudaFuncSetAttribute(in_transform_kernel<__nv_bfloat16, false>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   kXformSmem));
+    LZB_CUDA(cudaFuncSetAttribute(f3::gemm_f32x3_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  f3::Shape<64>::smem));
+    LZB_CUDA(cudaFuncSetAttribute(f3::gemm_f32x3_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  f3::Shape<128>::smem));
     LZB_CUDA(cudaFuncSetAttribute(tc::gemm_tc_kernel<__half>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, tc::kSmemBytes));
     LZB_CUDA(cudaFuncSetAttribute(tc::gemm_tc_kernel<__nv_bfloat16>,
@@ -799,6 +829,12 @@ int debug_conv_direct_t(lzb_ctx* c, int layer, const float* in, int n, const flo
     return rc ? rc : rc2;
 }
 
+// fp32 layers are contracted here by the FFMA kernel, which adds the channels in
+// ascending order like the engine's CPU pipe: a layer can then be compared with it
+// to the last places.  (Pipes contract on the tensor cores, gemm_f32x3.cuh, closer
+// to the exact sums than either: over 256 channels the CPU pipe's own rounding, a
+// layer's largest error 2.8e-6 of its largest output, is more than the 2e-6 this
+// diagnostic is held to.)
 template <typename T>
 int debug_conv_t(lzb_ctx* c, int layer, const float* in, int n, const float* residual, float* out) {
     lzb_pipe* p = c->pipe;
@@ -806,7 +842,7 @@ int debug_conv_t(lzb_ctx* c, int layer, const float* in, int n, const float* res
     const int P = n * kTilesPerPos;
     const int C = p->channels;
     const size_t plane_floats = (size_t)n * C * kSq;
-    T* V = static_cast<T*>(c->V);
+    T* V = static_cast<T*>(c->V);      // plain elements of T
     T* X = static_cast<T*>(c->X);
     float* stage = nullptr;    // fp32 NCHW staging on the device
     LZB_CUDA(cudaMalloc(&stage, sizeof(float) * (plane_floats > (size_t)n * LZB_IN_FLOATS
@@ -818,16 +854,27 @@ int debug_conv_t(lzb_ctx* c, int layer, const float* in, int n, const float* res
     };
     if (layer == 0) {
         guard(cudaMemcpyAsync(stage, in, sizeof(float) * n * LZB_IN_FLOATS, cudaMemcpyHostToDevice, c->stream), "copy in");
-        first_in_transform_kernel<T><<<(P + 7) / 8, 256, 0, c->stream>>>(InputView{stage, nullptr}, V, c->Pa, P);
+        first_in_transform_kernel<T, false><<<(P + 7) / 8, 256, 0, c->stream>>>(InputView{stage, nullptr}, V, c->Pa, P);
     } else {
         guard(cudaMemcpyAsync(stage, in, sizeof(float) * plane_floats, cudaMemcpyHostToDevice, c->stream), "copy in");
         nchw_to_nhwc_kernel<T><<<512, 256, 0, c->stream>>>(stage, X, n, C, p->Cp);
         const dim3 grid(p->Cp / kChanPerCta, n);
-        in_transform_kernel<T><<<grid, kXformThreads, kXformSmem, c->stream>>>(
-            X, V, c->Pa, p->Cp);
+        in_transform_kernel<T, false><<<grid, kXformThreads, kXformSmem, c->stream>>>(X, V, c->Pa, p->Cp);
     }
     guard(cudaGetLastError(), "input transform");
-    if (rc == LZB_OK) rc = contraction<T>(c, L, P, layer == 0);
+    float* U32 = nullptr;
+    if constexpr (std::is_same<T, float>::value) {
+        const size_t rows = (size_t)kPoints * p->Cp;
+        guard(cudaMalloc(&U32, rows * L.cin_p * sizeof(float)), "filters");
+        if (rc == LZB_OK) {
+            merge_u3_kernel<<<512, 256, 0, c->stream>>>(static_cast<const __nv_bfloat16*>(L.U), U32, rows, L.cin_p);
+            const dim3 grid(round_up(P, kSimtTile) / kSimtTile, p->Cp / kSimtTile, kPoints);
+            gemm_f32_kernel<<<grid, 256, 0, c->stream>>>(V, U32, static_cast<float*>(c->M), c->Pa, L.cin_p, p->Cp);
+            guard(cudaGetLastError(), "contraction");
+        }
+    } else {
+        if (rc == LZB_OK) rc = contraction<T>(c, L, P, layer == 0);
+    }
     const T* R = nullptr;
     if (rc == LZB_OK && residual) {
         guard(cudaMemcpyAsync(stage, residual, sizeof(float) * plane_floats, cudaMemcpyHostToDevice, c->stream), "copy residual");
@@ -841,6 +888,7 @@ int debug_conv_t(lzb_ctx* c, int layer, const float* in, int n, const float* res
         guard(cudaMemcpyAsync(out, stage, sizeof(float) * plane_floats, cudaMemcpyDeviceToHost, c->stream), "copy out");
     }
     int rc2 = lzb_ctx_sync(c);
+    cudaFree(U32);
     cudaFree(stage);
     return rc ? rc : rc2;
 }
@@ -970,7 +1018,7 @@ int install_conv(lzb_pipe* p, int layer, const float* src, int c_in, const float
                 rc = p->precision == LZB_FP16 ? upload_layer_direct_t<__half>(p, L, u_dev, c_in)
                                               : upload_layer_direct_t<__nv_bfloat16>(p, L, u_dev, c_in);
             } else if (p->precision == LZB_FP32) {
-                rc = upload_layer_t<float>(p, L, u_dev, c_in);
+                rc = upload_layer_f32(p, L, u_dev, c_in);
             } else if (p->precision == LZB_FP16) {
                 rc = upload_layer_t<__half>(p, L, u_dev, c_in);
             } else {
@@ -1021,7 +1069,13 @@ int install_conv(lzb_pipe* p, int layer, const float* src, int c_in, const float
             L.split_ok[ns] = (rc == LZB_OK);
         }
         if (rc) return rc;
-    } else if (p->precision != LZB_FP32) {
+    } else if (p->precision == LZB_FP32) {
+        const uint64_t rows = (uint64_t)kPoints * p->Cp, cols = (uint64_t)3 * L.cin_p;
+        rc = make_map_2d(&L.tmU, LZB_BF16, L.U, rows, cols, 64);
+        if (!rc && p->Cp % 128 == 0) rc = make_map_2d(&L.tmU128, LZB_BF16, L.U, rows, cols, 128);
+        else L.tmU128 = L.tmU;
+        if (rc) return rc;
+    } else {
         rc = make_map_2d(&L.tmU, p->precision, L.U, (uint64_t)kPoints * p->Cp, L.cin_p, p->Cp);
         if (rc) return rc;
     }
@@ -1290,16 +1344,13 @@ static int default_micro_batch(const lzb_pipe* p, int cap) {
             if ((groups * cand) % p->sm_count == 0) { n = cand; break; }
         }
     } else {
-        // fp32: the FFMA contraction runs tiles of 128 rows x 128 (or 64) channels,
-        // two CTAs per SM; take the count, from 64 down to 48, whose tiles fill
-        // their last wave best (61 positions at 256 channels: 864 tiles = 2.9 waves
-        // of 296, where 64 positions make 936 = 3.2)
-        const int col_tiles = p->Cp / (p->Cp % 128 == 0 ? 128 : 64);
-        const int slots = 2 * p->sm_count;
+        // fp32: of the counts from 64 down to 40 (V and M of 50 positions at 256 channels
+        // are 116 MB), the one whose items (128 rows x 128 channels) fill their last
+        // wave best
         double best = 0.0;
-        for (int cand = kDefaultMicroBatch; cand >= 48; cand--) {
-            const int tiles = round_up(cand * kTilesPerPos, kSimtBigM) / kSimtBigM * col_tiles * kPoints;
-            const int waves = (tiles + slots - 1) / slots;
+        for (int cand = kDefaultMicroBatch; cand >= 40; cand--) {
+            const int items = round_up(cand * kTilesPerPos, tc::kBlockM) / tc::kBlockM * ((p->Cp + 127) / 128) * kPoints;
+            const int waves = (items + p->sm_count - 1) / p->sm_count;
             const double rate = static_cast<double>(cand) / waves;     // positions per wave
             if (rate > best * 1.02) { best = rate; n = cand; }
         }
@@ -1341,7 +1392,7 @@ int lzb_ctx_create(lzb_ctx** out, lzb_pipe* p, int max_batch) {
         c->micro = default_micro_batch(p, c->micro_cap);
         c->Pa = round_up(c->micro_cap * kTilesPerPos, 128);
         const size_t vm = (size_t)kPoints * c->Pa * p->Cp * p->elt;
-        alloc(&c->V, vm);
+        alloc(&c->V, p->precision == LZB_FP32 ? vm / 4 * 6 : vm);     // fp32: three bf16 planes
         alloc(&c->M, vm);
         alloc(&c->X, (size_t)c->micro_cap * kSq * p->Cp * p->elt);
     }
@@ -1390,7 +1441,17 @@ int lzb_ctx_create(lzb_ctx** out, lzb_pipe* p, int max_batch) {
             lzb_ctx_destroy(c);
             return rc;
         }
-    } else if (p->precision != LZB_FP32) {
+    } else if (p->precision == LZB_FP32) {
+        const uint64_t rows = (uint64_t)kPoints * c->Pa;
+        int rc = make_map_2d(&c->tmV_first, LZB_BF16, c->V, rows, 3 * 64, tc::kBlockM);
+        if (!rc) rc = make_map_2d(&c->tmV32_first, LZB_BF16, c->V, rows, 3 * 64, 32);
+        if (!rc) rc = make_map_2d(&c->tmV, LZB_BF16, c->V, rows, (uint64_t)3 * p->Cp, tc::kBlockM);
+        if (!rc) rc = make_map_2d(&c->tmV32, LZB_BF16, c->V, rows, (uint64_t)3 * p->Cp, 32);
+        if (rc) {
+            lzb_ctx_destroy(c);
+            return rc;
+        }
+    } else {
         int rc = make_map_2d(&c->tmV_first, p->precision, c->V, (uint64_t)kPoints * c->Pa, 64, tc::kBlockM);
         if (!rc) rc = make_map_2d(&c->tmV, p->precision, c->V, (uint64_t)kPoints * c->Pa, p->Cp, tc::kBlockM);
         if (rc) {
@@ -1645,13 +1706,8 @@ int static_scratch_for(int device, unsigned char** out) {
             return fail(LZB_ERR_CUDA, std::string("cudaGetSymbolAddress(g_static_scratch): ") +
                                           cudaGetErrorString(e));
         }
-        e = cudaFuncSetAttribute(lzb::xform_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 kXformSmem);
-        if (e == cudaSuccess) {
-            e = cudaFuncSetAttribute(lzb::in_transform_kernel<float>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     kXformSmem);
-        }
+        e = cudaFuncSetAttribute(lzb::in_transform_kernel<float, false>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, kXformSmem);
         if (e != cudaSuccess) {
             return fail(LZB_ERR_CUDA, std::string("kernel attribute set-up: ") + cudaGetErrorString(e));
         }
@@ -1701,7 +1757,7 @@ int lzb_conv3x3_static(int device, const float* in_dev, int n, int c_in, int cha
     nchw_to_nhwc_kernel<float><<<128, 256, 0, stream>>>(in_dev, X, n, c_in, Cp);
     const dim3 tgrid(Cp / kChanPerCta, n);
     const size_t tsmem = kXformSmem;
-    in_transform_kernel<float><<<tgrid, kXformThreads, tsmem, stream>>>(X, V, kStaticRows, Cp);
+    in_transform_kernel<float, false><<<tgrid, kXformThreads, tsmem, stream>>>(X, V, kStaticRows, Cp);
     const dim3 ggrid(round_up(P, kSimtTile) / kSimtTile, Cp / kSimtTile, kPoints);
     gemm_f32_kernel<<<ggrid, 256, 0, stream>>>(V, U, M, kStaticRows, Cp, Cp);
     const float* R = nullptr;
@@ -1709,8 +1765,8 @@ int lzb_conv3x3_static(int device, const float* in_dev, int n, int c_in, int cha
         nchw_to_nhwc_kernel<float><<<128, 256, 0, stream>>>(residual_dev, X, n, channels, Cp);
         R = X;
     }
-    xform_kernel<float><<<tgrid, XformShape<float>::warps * 32, tsmem, stream>>>(M, kStaticRows, Cp, bn, bn + 64, R, X,
-                                                                  nullptr);
+    xform_f32_kernel<<<dim3(Cp / kXf32Chan, n), kXf32Threads, 0, stream>>>(M, kStaticRows, Cp, bn, bn + 64, R, X,
+                                                                          nullptr);
     nhwc_to_nchw_kernel<float><<<128, 256, 0, stream>>>(X, out_dev, n, channels, Cp);
     LZB_CUDA(cudaGetLastError());
     return LZB_OK;

@@ -5,7 +5,8 @@
 // Device layouts (T = float, __half or __nv_bfloat16; Cp = channels rounded up
 // to a multiple of 64, extra channels are zero):
 //   activations  X[n][361][Cp]        (board cell major, channel minor)
-//   V[36][Pa][Cp]   transformed input tiles,  row p = position * 25 + tile
+//   V[36][Pa][Cp]   transformed input tiles,  row p = position * 25 + tile; in fp32
+//                   V[36][Pa][3][Cp], three bf16 planes (gemm_f32x3.cuh)
 //   M[36][Pa][Cp]   contraction results, same row index
 // Pa = rows allocated (a multiple of 128).
 //
@@ -13,6 +14,7 @@
 // out_transform_fused_bn_in OpenCL kernels (src/kernels/convolve3.opencl:109-452)
 // and follow the arithmetic of src/CPUPipe.cpp:63-183, 212-284, 352-377.
 #pragma once
+#include "gemm_f32x3.cuh"
 #include "input_view.cuh"
 #include "winograd_math.cuh"
 
@@ -24,20 +26,43 @@ constexpr int kXformWarps = 8;
 constexpr int kXformThreads = kXformWarps * 32;
 // The fused transform runs one warp per tile in the 16-bit modes (25 warps: all
 // 25 tiles of a position have their loads in flight at once; the kernel is
-// bound by L2 latency, not by arithmetic) and 8 warps in fp32, whose 124 KB
-// board leaves room for one CTA per SM anyway.
+// bound by L2 latency, not by arithmetic).  fp32 has a kernel of its own,
+// xform_f32_kernel.
 template <typename T> struct XformShape { static constexpr int warps = 25; static constexpr int ctas = 1; };
-template <> struct XformShape<float> { static constexpr int warps = 8; static constexpr int ctas = 1; };
 constexpr int kChanPerCta = 64;               // one warp covers 32 channel pairs
+
+// How transformed tiles are stored: as elements of T, or (kSplit, fp32) as three
+// bf16 planes beside each other in a row.  Two channels at offset `off` of row
+// `row`, rows of C channels.
+template <typename T, bool kSplit> struct TileOut {
+    using type = T;
+    static __device__ __forceinline__ void store(T* V, size_t row, int C, int off, float2 v) {
+        using P2 = Pair<T>;
+        *reinterpret_cast<typename P2::type*>(V + row * C + off) = P2::from_f2(v);
+    }
+};
+template <> struct TileOut<float, true> {
+    using type = __nv_bfloat16;
+    static __device__ __forceinline__ void store(__nv_bfloat16* V, size_t row, int C, int off, float2 v) {
+        __nv_bfloat162 p0, p1, p2;
+        f3::split3(v.x, p0.x, p1.x, p2.x);
+        f3::split3(v.y, p0.y, p1.y, p2.y);
+        __nv_bfloat16* dst = V + row * 3 * C + off;
+        *reinterpret_cast<__nv_bfloat162*>(dst) = p0;
+        *reinterpret_cast<__nv_bfloat162*>(dst + C) = p1;
+        *reinterpret_cast<__nv_bfloat162*>(dst + 2 * C) = p2;
+    }
+};
+// The storage of V in a pipe of type T.
+template <typename T> struct PipeV { static constexpr bool split = false; };
+template <> struct PipeV<float> { static constexpr bool split = true; };
 
 // B^T d B of the 6x6 patch of tile (by, bx), read from a zero-haloed board in
 // shared memory, written to V rows of point t = xi*6 + nu.
-template <typename T>
-__device__ __forceinline__ void tile_in_transform(const float2* board,
-                                                  int lane, int by, int bx,
-                                                  T* V, size_t v_row_stride_pts,
-                                                  size_t v_off) {
-    using P2 = Pair<T>;
+template <typename T, bool kSplit>
+__device__ __forceinline__ void tile_in_transform(const float2* board, int lane, int by, int bx,
+                                                  typename TileOut<T, kSplit>::type* V, int Pa, int p,
+                                                  int Cp, int k) {
     float2 t1[6][6];
 #pragma unroll
     for (int col = 0; col < 6; col++) {
@@ -56,9 +81,7 @@ __device__ __forceinline__ void tile_in_transform(const float2* board,
         apply_bt<Pair<T>::exact>(vout, t1[xi]);
 #pragma unroll
         for (int nu = 0; nu < 6; nu++) {
-            auto* dst = reinterpret_cast<typename P2::type*>(
-                V + (size_t)(xi * 6 + nu) * v_row_stride_pts + v_off);
-            *dst = P2::from_f2(vout[nu]);
+            TileOut<T, kSplit>::store(V, (size_t)(xi * 6 + nu) * Pa + p, Cp, k, vout[nu]);
         }
     }
 }
@@ -76,10 +99,9 @@ __device__ __forceinline__ void zero_halo(float2* board, int warp, int lane, int
 // Input planes of the network -> V[36][Pa][64], channels 18..63 zero.
 // One warp per tile, one lane per channel pair.
 // ---------------------------------------------------------------------------
-template <typename T>
+template <typename T, bool kSplit>
 __global__ void __launch_bounds__(256) first_in_transform_kernel(
-    const InputView in, T* __restrict__ V, int Pa, int P) {
-    using P2 = Pair<T>;
+    const InputView in, typename TileOut<T, kSplit>::type* __restrict__ V, int Pa, int P) {
     const int lane = threadIdx.x & 31;
     const int p = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (p >= P) return;
@@ -110,9 +132,7 @@ __global__ void __launch_bounds__(256) first_in_transform_kernel(
         apply_bt<Pair<T>::exact>(vout, t1[xi]);
 #pragma unroll
         for (int nu = 0; nu < 6; nu++) {
-            auto* dst = reinterpret_cast<typename P2::type*>(
-                V + ((size_t)(xi * 6 + nu) * Pa + p) * 64 + c0);
-            *dst = P2::from_f2(vout[nu]);
+            TileOut<T, kSplit>::store(V, (size_t)(xi * 6 + nu) * Pa + p, 64, c0, vout[nu]);
         }
     }
 }
@@ -123,9 +143,9 @@ __global__ void __launch_bounds__(256) first_in_transform_kernel(
 // the tower this step is the tail of xform_kernel.
 // grid (Cp/64, n), block 256.
 // ---------------------------------------------------------------------------
-template <typename T>
+template <typename T, bool kSplit>
 __global__ void __launch_bounds__(kXformThreads) in_transform_kernel(
-    const T* __restrict__ X, T* __restrict__ V, int Pa, int Cp) {
+    const T* __restrict__ X, typename TileOut<T, kSplit>::type* __restrict__ V, int Pa, int Cp) {
     using P2 = Pair<T>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     auto* board = reinterpret_cast<float2*>(smem_raw);
@@ -140,8 +160,7 @@ __global__ void __launch_bounds__(kXformThreads) in_transform_kernel(
     __syncthreads();
     for (int tile = warp; tile < kTilesPerPos; tile += kXformWarps) {
         const int p = n * kTilesPerPos + tile;
-        tile_in_transform<T>(board, lane, tile / kTilesPerSide, tile % kTilesPerSide, V,
-                             (size_t)Pa * Cp, (size_t)p * Cp + k);
+        tile_in_transform<T, kSplit>(board, lane, tile / kTilesPerSide, tile % kTilesPerSide, V, Pa, p, Cp, k);
     }
 }
 
@@ -231,8 +250,112 @@ __global__ void __launch_bounds__(XformShape<T>::warps * 32, XformShape<T>::ctas
     __syncthreads();
     for (int tile = warp; tile < kTilesPerPos; tile += XformShape<T>::warps) {
         const int p = n * kTilesPerPos + tile;
-        tile_in_transform<T>(board, lane, tile / kTilesPerSide, tile % kTilesPerSide, V,
-                             pt_stride, (size_t)p * Cp + k);
+        tile_in_transform<T, false>(board, lane, tile / kTilesPerSide, tile % kTilesPerSide, V, Pa, p, Cp, k);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// The same step in fp32 (V as three bf16 planes, or null).  A CTA owns one position
+// and 16 channels: eight lanes of two channels for each of the 25 tiles, so that
+// one pass of 200 threads takes the whole plane and a single position at 256
+// channels already fills 16 CTAs (with 64 channels per CTA and 8 warps walking
+// over the tiles it was 4 CTAs of 25 us).  A row segment of a CTA is 64 bytes of M
+// and 32 of each plane of V: whole sectors.  All 36 loads of a thread are in flight
+// at once.  Board cells are 80 bytes apart, so that the two tiles of a half warp
+// (four cells apart) use different banks.
+// grid (Cp/16, n), block 200.  Values and order of operations are those of
+// xform_kernel with Pair<float>: multiplies and adds as the CPU pipe has them.
+// ---------------------------------------------------------------------------
+constexpr int kXf32Chan = 16;
+constexpr int kXf32Threads = kTilesPerPos * (kXf32Chan / 2);
+constexpr int kXf32Cell = 10;                 // float2 per board cell: 8 used
+
+__global__ void __launch_bounds__(kXf32Threads, 2) xform_f32_kernel(
+    const float* M, int Pa, int Cp, const float* __restrict__ bn_mean, const float* __restrict__ bn_invstd,
+    const float* R, float* X_out, __nv_bfloat16* __restrict__ V) {
+    __shared__ float2 board[kBoardCells * kXf32Cell];
+    const int tile = threadIdx.x >> 3, lane = threadIdx.x & 7;
+    const int by = tile / kTilesPerSide, bx = tile % kTilesPerSide;
+    const int n = blockIdx.y, k = blockIdx.x * kXf32Chan + 2 * lane;
+
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (V != nullptr) {
+        for (int cell = tile; cell < kBoardCells; cell += kTilesPerPos) {
+            const int r = cell / kBoardPad, c = cell % kBoardPad;
+            if (r == 0 || r > kBoard || c == 0 || c > kBoard) board[cell * kXf32Cell + lane] = make_float2(0.f, 0.f);
+        }
+    }
+    const float2 mean = *reinterpret_cast<const float2*>(bn_mean + k);
+    const float2 scale = *reinterpret_cast<const float2*>(bn_invstd + k);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+
+    const float* msrc = M + (size_t)(n * kTilesPerPos + tile) * Cp + k;
+    const size_t pt_stride = (size_t)Pa * Cp;
+    float2 temp[4][6];
+    {
+        float2 m[36];
+#pragma unroll
+        for (int t = 0; t < 36; t++) m[t] = __ldcg(reinterpret_cast<const float2*>(msrc + t * pt_stride));
+#pragma unroll
+        for (int nu = 0; nu < 6; nu++) {
+            const float2 col[6] = {m[nu], m[6 + nu], m[12 + nu], m[18 + nu], m[24 + nu], m[30 + nu]};
+            float2 o4[4];
+            apply_at<true>(o4, col);
+#pragma unroll
+            for (int i = 0; i < 4; i++) temp[i][nu] = o4[i];
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int y = 4 * by + i;
+        float2 r4[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int x = 4 * bx + j;
+            r4[j] = (R != nullptr && y < kBoard && x < kBoard)
+                        ? *reinterpret_cast<const float2*>(R + ((size_t)n * kSq + y * kBoard + x) * Cp + k)
+                        : make_float2(0.f, 0.f);
+        }
+        float2 o4[4];
+        apply_at<true>(o4, temp[i]);
+        if (y >= kBoard) continue;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int x = 4 * bx + j;
+            if (x >= kBoard) continue;
+            // max(0, invstd * (v - mean) [+ residual]), src/CPUPipe.cpp:352-377
+            float2 v = make_float2(op_mul<true>(scale.x, op_add<true>(o4[j].x, -mean.x)),
+                                   op_mul<true>(scale.y, op_add<true>(o4[j].y, -mean.y)));
+            if (R != nullptr) v = add2<true>(v, r4[j]);
+            v.x = fmaxf(v.x, 0.f);
+            v.y = fmaxf(v.y, 0.f);
+            if (X_out != nullptr) {
+                *reinterpret_cast<float2*>(X_out + ((size_t)n * kSq + y * kBoard + x) * Cp + k) = v;
+            }
+            if (V != nullptr) board[((y + 1) * kBoardPad + x + 1) * kXf32Cell + lane] = v;
+        }
+    }
+    if (V == nullptr) return;
+    __syncthreads();
+    float2 t1[6][6];
+#pragma unroll
+    for (int col = 0; col < 6; col++) {
+        float2 vin[6], vout[6];
+#pragma unroll
+        for (int r = 0; r < 6; r++) vin[r] = board[((4 * by + r) * kBoardPad + 4 * bx + col) * kXf32Cell + lane];
+        apply_bt<true>(vout, vin);
+#pragma unroll
+        for (int r = 0; r < 6; r++) t1[r][col] = vout[r];
+    }
+    const int p = n * kTilesPerPos + tile;
+#pragma unroll
+    for (int xi = 0; xi < 6; xi++) {
+        float2 vout[6];
+        apply_bt<true>(vout, t1[xi]);
+#pragma unroll
+        for (int nu = 0; nu < 6; nu++) {
+            TileOut<float, true>::store(V, (size_t)(xi * 6 + nu) * Pa + p, Cp, k, vout[nu]);
+        }
     }
 }
 
@@ -241,6 +364,28 @@ __global__ void __launch_bounds__(XformShape<T>::warps * 32, XformShape<T>::ctas
 // src/Network.cpp:215) -> U[36][Kp][Cin_p] of type T, zero padded, input
 // channel innermost so that both contraction operands are K-major.
 // ---------------------------------------------------------------------------
+// Three bf16 planes per row, U[36][Kp][3][Cin_p] (gemm_f32x3.cuh).
+__global__ void repack_u3_kernel(const float* __restrict__ U32, __nv_bfloat16* __restrict__ U, int c_in, int K,
+                                 int Cin_p, int Kp) {
+    const size_t total = (size_t)kPoints * Kp * Cin_p;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total;
+         i += (size_t)gridDim.x * blockDim.x) {
+        const int c = i % Cin_p;
+        const int k = (i / Cin_p) % Kp;
+        const int t = i / ((size_t)Cin_p * Kp);
+        const float v = (c < c_in && k < K) ? U32[((size_t)t * c_in + c) * K + k] : 0.f;
+        __nv_bfloat16* dst = U + ((size_t)t * Kp + k) * 3 * Cin_p + c;
+        f3::split3(v, dst[0], dst[Cin_p], dst[2 * Cin_p]);
+    }
+}
+// ... and back: the sum of the planes is the fp32 value they were split from.
+__global__ void merge_u3_kernel(const __nv_bfloat16* __restrict__ U, float* __restrict__ out, size_t rows, int Cin_p) {
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < rows * Cin_p;
+         i += (size_t)gridDim.x * blockDim.x) {
+        const __nv_bfloat16* src = U + (i / Cin_p) * 3 * Cin_p + i % Cin_p;
+        out[i] = (__bfloat162float(src[0]) + __bfloat162float(src[Cin_p])) + __bfloat162float(src[2 * Cin_p]);
+    }
+}
 template <typename T>
 __global__ void repack_u_kernel(const float* __restrict__ U32, T* __restrict__ U, int c_in,
                                 int K, int Cin_p, int Kp) {
