@@ -18,21 +18,24 @@
 // it is 1.4e-6 at 256.
 //
 // V is [36 * Pa rows][3 * Cin] and U [36 * Kp rows][3 * Cin], plane-major within a
-// row.  One work item is (t, slice of N output channels, block of 128 rows);
-// items are numbered row block innermost, so that neighbouring CTAs share U in L2.
-// A pipeline stage is one 64-channel chunk: three V tiles and three U tiles, each
-// plane pair with a "full" barrier of its own, because x0y0 can start while the
-// other planes are on their way.  N = 128 normally, 64 where that gives the SMs
-// more items than N = 128 has (small batches).
+// row.  One work item is (t, slice of N output channels, block of rows); items are
+// numbered row block innermost, so that neighbours share U in L2.  Batches of more
+// than 128 rows run on CTA pairs (tcgen05 cta_group::2, 256 rows, each CTA staging
+// half of the U tile: 72 KB instead of 96 KB per 24 MMAs, and L2 is what the large
+// ones are bound by); smaller ones on single CTAs with N = 64, so that the 36 points
+// of one position fill the SMs.
 //
-// Roles as in gemm_tcgen05.cuh with eight epilogue warps.  The small accumulator
-// alternates between two places; the two x0y0 ones are free again as soon as the
-// epilogue has read them, which it does first.
+// The operand ring has eight slots, one plane of V and U each, three to a 64-channel
+// chunk; x0y0 can start while the other planes are on their way.  Roles as in
+// gemm_tcgen05.cuh with eight epilogue warps, which leave through shared memory and
+// TMA (a lane's 256 bytes of a row as direct stores took 2,600 cycles an item).  The
+// small accumulator alternates between two places; the two x0y0 ones are free again
+// as soon as the epilogue has read them, which it does first.
 //
-// What bounds it: at 256 x 256 channels the MMAs (96 of 128 x 128 x 16 per item at
-// 65 cycles) against 96 KB of operands per 24 of them, 61 bytes a cycle and SM.
+// What bounds it: 256 channels, N = 128: 96 MMAs of 65 cycles an item against 288 KB
+// of operands per CTA, some 40 bytes a cycle and SM from L2.
 #pragma once
-#include "gemm_tcgen05.cuh"
+#include "conv_direct2.cuh"
 
 namespace lzb {
 namespace f3 {
@@ -41,13 +44,11 @@ using namespace tc;
 
 constexpr int kF3Threads = 320;                        // producer, MMA, 8 epilogue warps
 constexpr uint32_t kATile = kBlockM * 128;             // 16 KB: one plane of 128 rows x 64 channels
-template <int N> struct Shape {
-    static constexpr uint32_t b_tile = N * 128;
-    static constexpr uint32_t stage = 3 * (kATile + b_tile);
-    static constexpr int stages = N == 64 ? 3 : 2;
-    static constexpr uint32_t smem = stages * stage + kBarBytes + 1024;
-};
-static_assert(Shape<64>::smem <= 227 * 1024 && Shape<128>::smem <= 227 * 1024, "shared memory of one CTA");
+constexpr int kF3Slots = 8;
+constexpr uint32_t kF3SlotBytes = kATile + 64 * 128;   // and the U rows this CTA stages (at most 64)
+constexpr uint32_t kF3OutBytes = 32 * 128;             // one epilogue warp: 32 rows x 32 channels
+constexpr uint32_t kF3Smem = kF3Slots * kF3SlotBytes + 8 * kF3OutBytes + kBarBytes + 1024;
+static_assert(kF3Smem <= 227 * 1024, "shared memory of one CTA");
 
 constexpr int kErrF3Producer = 601;
 constexpr int kErrF3Mma = 602;
@@ -62,178 +63,219 @@ __device__ __forceinline__ void split3(float v, __nv_bfloat16& p0, __nv_bfloat16
 }
 
 // tmV : [36 * Pa][3 * Cin], box 64 x 128; tmV32 : the same, box 64 x 32 (the last
-// rows of a small batch); tmU : [36 * Kp][3 * Cin], box 64 x N.  nblk row blocks of
-// 128 covering P rows.
-template <int N>
+// rows of a batch); tmU : [36 * Kp][3 * Cin], box 64 x the U rows of one CTA; tmM :
+// [36 * Pa][Kp] fp32, box 32 x 32, 128-byte swizzle.  P rows, nblk blocks of 128 (or
+// of 256, for a pair); rows of M from P to the end of a block of 32 are scratch.
+template <int N, bool kPair>
 __global__ void __launch_bounds__(kF3Threads, 1) gemm_f32x3_kernel(
     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmV32,
-    const __grid_constant__ CUtensorMap tmU, float* M, int Pa, int P, int Kp, int Cin, int nblk, int* err) {
-    using S = Shape<N>;
+    const __grid_constant__ CUtensorMap tmU, const __grid_constant__ CUtensorMap tmM, int Pa, int P, int Kp,
+    int Cin, int nblk, int* err) {
+    constexpr int kCtas = kPair ? 2 : 1;
+    constexpr int kURows = N / kCtas;                  // U rows this CTA stages
+    constexpr uint32_t kBTile = kURows * 128;
+    static_assert(kURows <= 64, "slot size");
     extern __shared__ unsigned char smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
     unsigned char* smem = smem_raw + (base - raw);
-    unsigned char* bar_mem = smem + S::stages * S::stage;
+    unsigned char* stage_out = smem + kF3Slots * kF3SlotBytes;
+    unsigned char* bar_mem = stage_out + 8 * kF3OutBytes;
     const uint32_t bars = smem_u32(bar_mem);
-    auto full_bar = [&](int s, int plane) { return bars + 8u * (s * 3 + plane); };
-    auto empty_bar = [&](int s) { return bars + 8u * (12 + s); };
-    auto tfull_bar = [&](int a) { return bars + 8u * (16 + a); };       // all accumulators of an item
-    auto sfree_bar = [&](int a) { return bars + 8u * (18 + a); };       // small accumulator a
-    const uint32_t mfree_bar = bars + 8u * 20;                           // both x0y0 accumulators
+    auto full_bar = [&](int s) { return bars + 8u * s; };               // the leader's are used
+    auto empty_bar = [&](int s) { return bars + 8u * (8 + s); };        // every CTA
+    auto tfull_bar = [&](int a) { return bars + 8u * (16 + a); };       // every CTA: an item's accumulators
+    auto sfree_bar = [&](int a) { return bars + 8u * (18 + a); };       // the leader's: small accumulator a
+    const uint32_t mfree_bar = bars + 8u * 20;                           // the leader's: both x0y0 accumulators
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bar_mem + 8 * 24);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(bar_mem + 8 * 24 + 8);
 
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = kPair ? dc2::cluster_ctarank() : 0u;
     if (threadIdx.x == 0) {
-        for (int s = 0; s < S::stages; s++) {
-            for (int k = 0; k < 3; k++) mbar_init(full_bar(s, k), 1);
+        for (int s = 0; s < kF3Slots; s++) {
+            mbar_init(full_bar(s), kCtas);
             mbar_init(empty_bar(s), 1);
         }
         for (int a = 0; a < 2; a++) {
             mbar_init(tfull_bar(a), 1);
-            mbar_init(sfree_bar(a), 8);
+            mbar_init(sfree_bar(a), 8 * kCtas);
         }
-        mbar_init(mfree_bar, 8);
+        mbar_init(mfree_bar, 8 * kCtas);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                         smem_u32(const_cast<uint32_t*>(tmem_slot))),
-                     "r"(4u * N)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if constexpr (kPair) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                             smem_u32(const_cast<uint32_t*>(tmem_slot))), "r"(4u * N) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                             smem_u32(const_cast<uint32_t*>(tmem_slot))), "r"(4u * N) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
     }
     tcgen05_fence_before();
     __syncthreads();
+    if constexpr (kPair) dc2::cluster_sync_all();      // the peer's barriers are initialised
     tcgen05_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     // columns: [x0y0 first half][x0y0 second half][small 0][small 1], N each
     const int chunks = Cin / kChunkK, first_half = (chunks + 1) / 2;
     const int slices = Kp / N, items = kPoints * slices * nblk;
-    const int item_begin = static_cast<int>(static_cast<long long>(blockIdx.x) * items / gridDim.x);
-    const int item_end = static_cast<int>(static_cast<long long>(blockIdx.x + 1) * items / gridDim.x);
+    const int workers = gridDim.x / kCtas, worker = blockIdx.x / kCtas;
+    const int item_begin = static_cast<int>(static_cast<long long>(worker) * items / workers);
+    const int item_end = static_cast<int>(static_cast<long long>(worker + 1) * items / workers);
+    // first row of this CTA's block; rows of it that exist (none: the CTA of a pair
+    // beyond the last row still loads one box, so that its barriers complete)
+    auto block_row = [&](int item) { return (item % nblk) * kBlockM * kCtas + static_cast<int>(rank) * kBlockM; };
+    auto boxes_of = [&](int row) {                      // boxes of 32 rows; 4: the whole block
+        const int b = (P - row + 31) / 32;
+        return b > 4 ? 4 : (b < 1 ? 1 : b);
+    };
 
     if (warp == 0) {
         // ------------------------------------------------ TMA producer
         if (elect_one()) {
-            int stage = 0;
+            const uint32_t lead = kPair ? dc2::map_to_cta(bars, 0) : bars;
+            int slot = 0;
             uint32_t phase = 0;
             bool ok = true, waited = false;
-            // U does not depend on the previous kernel: the first stages' tiles are
-            // requested before this kernel waits for V
-            const int ahead = item_begin < item_end ? (chunks < S::stages ? chunks : S::stages) : 0;
-            auto load_u = [&](int item, int c, int s) {
+            auto load = [&](uint32_t dst, const CUtensorMap* map, int c, int r, uint32_t bar) {
+                if constexpr (kPair) dc2::tma_load_2d_pair(dst, map, c, r, bar);
+                else tma_load_2d(dst, map, c, r, bar);
+            };
+            // the slot's byte count and its U tile, which does not depend on the kernel
+            // before this one
+            auto begin_slot = [&](int item, int c, int k, int s) {
                 const int ts = item / nblk;                    // t * slices + slice
-                const int row = (ts / slices) * Kp + (ts % slices) * N;
-                for (int k = 0; k < 3; k++) {
-                    tma_load_2d(base + s * S::stage + 3 * kATile + k * S::b_tile, &tmU, k * Cin + c * kChunkK, row,
-                                full_bar(s, k));
-                }
+                const uint32_t bytes = static_cast<uint32_t>(boxes_of(block_row(item))) * 32u * 128u + kBTile;
+                const uint32_t bar = lead + 8u * s;
+                if constexpr (kPair) dc2::mbar_expect_tx_cluster(bar, bytes);
+                else mbar_expect_tx(bar, bytes);
+                load(base + s * kF3SlotBytes + kATile, &tmU, k * Cin + c * kChunkK,
+                     (ts / slices) * Kp + (ts % slices) * N + static_cast<int>(rank) * kURows, bar);
             };
-            auto expect = [&](int item, int s) {
-                const int left = P - (item % nblk) * kBlockM;
-                const uint32_t a = left >= kBlockM ? kATile : static_cast<uint32_t>((left + 31) / 32) * 32u * 128u;
-                for (int k = 0; k < 3; k++) mbar_expect_tx(full_bar(s, k), a + S::b_tile);
-            };
-            for (int c = 0; c < ahead; ++c) {
-                expect(item_begin, c);
-                load_u(item_begin, c, c);
-            }
+            // the first slots' U tiles are requested before this kernel waits for V
+            const int total = 3 * chunks;                      // slots of one item
+            const int ahead = item_begin < item_end ? (total < kF3Slots ? total : kF3Slots) : 0;
+            for (int i = 0; i < ahead; ++i) begin_slot(item_begin, i / 3, i % 3, i);
             for (int item = item_begin; item < item_end && ok; ++item) {
-                const int t = item / nblk / slices, blk = item % nblk;
-                const int left = P - blk * kBlockM, row = t * Pa + blk * kBlockM;
-                for (int c = 0; c < chunks; ++c) {
-                    if (item != item_begin || c >= ahead) {
-                        ok = mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, err, kErrF3Producer);
+                const int row = block_row(item), boxes = boxes_of(row);
+                const int row0 = (item / nblk / slices) * Pa + (row < P ? row : 0);
+                for (int i = 0; i < total; ++i) {
+                    const int c = i / 3, k = i % 3;
+                    if (item != item_begin || i >= ahead) {
+                        ok = mbar_wait(empty_bar(slot), phase ^ 1u, abort_flag, err, kErrF3Producer);
                         if (!ok) break;
-                        expect(item, stage);
-                        load_u(item, c, stage);
+                        begin_slot(item, c, k, slot);
                     }
                     if (!waited) {
                         asm volatile("griddepcontrol.wait;" ::: "memory");
                         waited = true;
                     }
-                    for (int k = 0; k < 3; k++) {
-                        const uint32_t dst = base + stage * S::stage + k * kATile;
-                        if (left >= kBlockM) {
-                            tma_load_2d(dst, &tmV, k * Cin + c * kChunkK, row, full_bar(stage, k));
-                        } else {
-                            for (int r = 0; r < left; r += 32) {
-                                tma_load_2d(dst + r * 128, &tmV32, k * Cin + c * kChunkK, row + r,
-                                            full_bar(stage, k));
-                            }
+                    const uint32_t dst = base + slot * kF3SlotBytes;
+                    if (boxes == 4) {
+                        load(dst, &tmV, k * Cin + c * kChunkK, row0, lead + 8u * slot);
+                    } else {
+                        for (int r = 0; r < boxes; ++r) {
+                            load(dst + r * 4096u, &tmV32, k * Cin + c * kChunkK, row0 + 32 * r, lead + 8u * slot);
                         }
                     }
-                    if (++stage == S::stages) { stage = 0; phase ^= 1u; }
+                    if (++slot == kF3Slots) { slot = 0; phase ^= 1u; }
                 }
             }
         }
     } else if (warp == 1) {
-        // ------------------------------------------------ MMA issuer
-        if (elect_one()) {
+        // ------------------------------------------------ MMA issuer (a pair's leader)
+        if (rank == 0 && elect_one()) {
             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(N >> 3) << 17) |
-                                   (static_cast<uint32_t>(kBlockM >> 4) << 24);
-            int stage = 0;
+                                   (static_cast<uint32_t>((kBlockM * kCtas) >> 4) << 24);
+            int slot = 0;
             uint32_t phase = 0;
             bool ok = true;
             int local = 0;
             const uint64_t d0 = umma_desc_sw128(base);
+            auto first = [&](uint32_t d, uint64_t a, uint64_t b) {
+                if constexpr (kPair) dc2::tcgen05_mma_f16_pair<false>(d, a, b, idesc);
+                else tcgen05_mma_f16<false>(d, a, b, idesc);
+            };
+            auto mma = [&](uint32_t d, uint64_t a, uint64_t b) {
+                if constexpr (kPair) dc2::tcgen05_mma_f16_pair<true>(d, a, b, idesc);
+                else tcgen05_mma_f16<true>(d, a, b, idesc);
+            };
+            auto mma4 = [&](uint32_t d, uint64_t a, uint64_t b) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) mma(d, a + 2u * k, b + 2u * k);
+            };
+            auto commit = [&](uint32_t bar) {
+                if constexpr (kPair) dc2::tcgen05_commit_pair(bar);
+                else tcgen05_commit(bar);
+            };
             for (int item = item_begin; item < item_end && ok; ++item, ++local) {
                 const int acc = local & 1;
                 const uint32_t t_small = tmem_base + static_cast<uint32_t>((2 + acc) * N);
                 ok = mbar_wait(sfree_bar(acc), ((local >> 1) & 1u) ^ 1u, abort_flag, err, kErrF3Mma);
+                if (ok) ok = mbar_wait(mfree_bar, (local & 1u) ^ 1u, abort_flag, err, kErrF3Mma);
                 for (int c = 0; c < chunks && ok; ++c) {
                     const uint32_t t_main = tmem_base + (c < first_half ? 0u : static_cast<uint32_t>(N));
-                    const uint64_t s16 = static_cast<uint64_t>(stage) * (S::stage >> 4);
-                    auto a = [&](int k) { return d0 + s16 + static_cast<uint64_t>(k) * (kATile >> 4); };
-                    auto b = [&](int k) {
-                        return d0 + s16 + (3 * kATile >> 4) + static_cast<uint64_t>(k) * (S::b_tile >> 4);
-                    };
-                    if (c == 0) ok = mbar_wait(mfree_bar, (local & 1u) ^ 1u, abort_flag, err, kErrF3Mma);
-                    if (ok) ok = mbar_wait(full_bar(stage, 0), phase, abort_flag, err, kErrF3Mma);
+                    uint64_t a[3], b[3];
+                    int s[3];
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) {
+                        ok = ok && mbar_wait(full_bar(slot), phase, abort_flag, err, kErrF3Mma);
+                        s[k] = slot;
+                        a[k] = d0 + static_cast<uint64_t>(slot) * (kF3SlotBytes >> 4);
+                        b[k] = a[k] + (kATile >> 4);
+                        if (++slot == kF3Slots) { slot = 0; phase ^= 1u; }
+                        if (!ok) break;
+                        tcgen05_fence_after();
+                        if (k == 0) {
+                            if (c == 0 || c == first_half) first(t_main, a[0], b[0]);
+                            else mma(t_main, a[0], b[0]);
+#pragma unroll
+                            for (int j = 1; j < 4; ++j) mma(t_main, a[0] + 2u * j, b[0] + 2u * j);
+                        } else if (k == 1) {
+                            if (c == 0) first(t_small, a[1], b[1]);
+                            else mma(t_small, a[1], b[1]);
+#pragma unroll
+                            for (int j = 1; j < 4; ++j) mma(t_small, a[1] + 2u * j, b[1] + 2u * j);
+                            mma4(t_small, a[0], b[1]);
+                            mma4(t_small, a[1], b[0]);
+                        } else {
+                            mma4(t_small, a[0], b[2]);
+                            mma4(t_small, a[2], b[0]);
+                        }
+                    }
                     if (!ok) break;
-                    tcgen05_fence_after();
-                    if (c == 0 || c == first_half) tcgen05_mma_f16<false>(t_main, a(0), b(0), idesc);
-                    else tcgen05_mma_f16<true>(t_main, a(0), b(0), idesc);
 #pragma unroll
-                    for (int k = 1; k < 4; ++k) tcgen05_mma_f16<true>(t_main, a(0) + 2u * k, b(0) + 2u * k, idesc);
-                    ok = mbar_wait(full_bar(stage, 1), phase, abort_flag, err, kErrF3Mma);
-                    if (!ok) break;
-                    if (c == 0) tcgen05_mma_f16<false>(t_small, a(1), b(1), idesc);
-                    else tcgen05_mma_f16<true>(t_small, a(1), b(1), idesc);
-#pragma unroll
-                    for (int k = 1; k < 4; ++k) tcgen05_mma_f16<true>(t_small, a(1) + 2u * k, b(1) + 2u * k, idesc);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) tcgen05_mma_f16<true>(t_small, a(0) + 2u * k, b(1) + 2u * k, idesc);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) tcgen05_mma_f16<true>(t_small, a(1) + 2u * k, b(0) + 2u * k, idesc);
-                    ok = mbar_wait(full_bar(stage, 2), phase, abort_flag, err, kErrF3Mma);
-                    if (!ok) break;
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) tcgen05_mma_f16<true>(t_small, a(0) + 2u * k, b(2) + 2u * k, idesc);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) tcgen05_mma_f16<true>(t_small, a(2) + 2u * k, b(0) + 2u * k, idesc);
-                    tcgen05_commit(empty_bar(stage));
-                    if (++stage == S::stages) { stage = 0; phase ^= 1u; }
+                    for (int k = 0; k < 3; ++k) commit(empty_bar(s[k]));
                 }
-                tcgen05_commit(tfull_bar(acc));
+                commit(tfull_bar(acc));
             }
         }
     } else {
-        // ------------------------------------------------ epilogue (warps 2..9)
+        // ------------------------------------------------ epilogue (warps 2..9 of every CTA)
         const int qd = warp & 3;
         constexpr int kCols = N / 2;                   // channels of this warp
         const int col0 = ((warp - 2) >> 2) * kCols;
         const uint32_t lanes = static_cast<uint32_t>(qd * 32) << 16;
+        unsigned char* stg = stage_out + (warp - 2) * kF3OutBytes;
+        const uint32_t stg_addr = smem_u32(stg);
+        const uint32_t lead = kPair ? dc2::map_to_cta(bars, 0) : bars;
+        auto arrive = [&](uint32_t bar) {
+            if constexpr (kPair) dc2::mbar_arrive_cluster(lead + (bar - bars));
+            else mbar_arrive(bar);
+        };
         bool waited = false;
         int local = 0;
         for (int item = item_begin; item < item_end; ++item, ++local) {
             const int acc = local & 1;
             const int ts = item / nblk, t = ts / slices;
-            const int p = (item % nblk) * kBlockM + qd * 32 + lane;
+            const int p = block_row(item) + qd * 32;   // first row of this warp
             bool ok = true;
             if (lane == 0) ok = mbar_wait(tfull_bar(acc), (local >> 1) & 1u, abort_flag, err, kErrF3Epilogue);
             ok = __shfl_sync(0xffffffffu, ok, 0);
@@ -256,7 +298,7 @@ __global__ void __launch_bounds__(kF3Threads, 1) gemm_f32x3_kernel(
             }
             tcgen05_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(mfree_bar);
+            if (lane == 0) arrive(mfree_bar);
 #pragma unroll
             for (int j = 0; j < kCols; j += 32) {
                 uint32_t r0[32];
@@ -267,32 +309,39 @@ __global__ void __launch_bounds__(kF3Threads, 1) gemm_f32x3_kernel(
             }
             tcgen05_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(sfree_bar(acc));
+            if (lane == 0) arrive(sfree_bar(acc));
             if (!waited) {
                 // M may still be read by the kernel before this one
                 asm volatile("griddepcontrol.wait;" ::: "memory");
                 waited = true;
             }
             if (p < P) {
-                float* dst = M + (static_cast<size_t>(t) * Pa + p) * Kp + (ts % slices) * N + col0;
-                // whole 32-byte sectors per lane and store
 #pragma unroll
-                for (int j = 0; j < kCols; j += 8) {
-                    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst + j),
-                                 "f"(sum[j]), "f"(sum[j + 1]), "f"(sum[j + 2]), "f"(sum[j + 3]), "f"(sum[j + 4]),
-                                 "f"(sum[j + 5]), "f"(sum[j + 6]), "f"(sum[j + 7])
-                                 : "memory");
+                for (int j = 0; j < kCols; j += 32) {
+                    dc::wait_staged_tile_read(lane);
+                    // 16-byte word v of row r at slot v ^ (r & 7): the 128-byte swizzle
+#pragma unroll
+                    for (int v = 0; v < 8; ++v) {
+                        *reinterpret_cast<float4*>(stg + lane * 128 + ((v ^ (lane & 7)) << 4)) =
+                            make_float4(sum[j + 4 * v], sum[j + 4 * v + 1], sum[j + 4 * v + 2], sum[j + 4 * v + 3]);
+                    }
+                    dc::store_staged_tile(&tmM, stg_addr, (ts % slices) * N + col0 + j, t * Pa + p, lane);
                 }
             }
         }
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     }
 
     tcgen05_fence_before();
     __syncthreads();
+    if constexpr (kPair) dc2::cluster_sync_all();      // neither CTA retires while its peer can touch it
     if (warp == 1) {
         __syncwarp();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(4u * N)
-                     : "memory");
+        if constexpr (kPair) {
+            asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(4u * N) : "memory");
+        } else {
+            asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(4u * N) : "memory");
+        }
     }
 }
 

@@ -21,7 +21,8 @@
 // fetched four at a time behind the activations, the heads of one position took
 // 25 us; together with the copies that followed them they were a third of a small
 // evaluation.  With more positions than clusters fit the GPU at once a cluster
-// takes several and reads the 1.4 MB of weights once for all of them.
+// takes several at a time: it reads the 1.4 MB of weights once for all of them, and
+// each of its CTAs finishes another position.
 #pragma once
 #include "conv_direct.cuh"
 #include "winograd_math.cuh"
@@ -147,15 +148,18 @@ struct HeadWeights {
         *ip1_val_wT /*[361][256]*/, *ip1_val_b, *ip2_val_w, *ip2_val_b;
 };
 
-// grid: clusters of kHeadCtas, each takes positions first, first + clusters, ...
-template <typename T, bool kCells>
+// grid: clusters of kHeadCtas.  A cluster takes its positions G = kHeadGroup at a
+// time, first group at G * cluster, and CTA g of the cluster finishes position g of
+// a group (its value head is finished by the next CTA, so that with one position
+// the two heads end side by side).
+template <typename T, bool kCells, int kHeadGroup>
 __global__ void __cluster_dims__(kHeadCtas, 1, 1) __launch_bounds__(kHeadThreads)
     heads_kernel(const T* X, const float* __restrict__ w, int Cp, int n, int ldx, int lo_off, int lo_e5m2,
                  const HeadWeights h, float inv_temp, float* __restrict__ policy, float* __restrict__ winrate,
                  const int* err, int* err_out) {
-    __shared__ float x[3][kHeadCells];
-    __shared__ float part_pol[2 * kHeadCtas][kMoves];       // used in the first CTA of the cluster
-    __shared__ float part_val[kHeadCtas][kValueHidden];     // ... in the second
+    __shared__ float x[3][kHeadCells][kHeadGroup];
+    __shared__ float part_pol[2 * kHeadCtas][kMoves];       // of the position this CTA finishes
+    __shared__ float part_val[kHeadCtas][kValueHidden];
     __shared__ float scratch[32];
     const int rank = static_cast<int>(head_cluster_rank());
     const int s0 = rank * kHeadCells;
@@ -168,36 +172,50 @@ __global__ void __cluster_dims__(kHeadCtas, 1, 1) __launch_bounds__(kHeadThreads
     const int outs = plane < 2 ? kMoves : kValueHidden;
     const float* wsrc = plane < 2 ? h.ip_pol_wT + (size_t)(plane * kSq + s0) * kMoves + o
                                   : h.ip1_val_wT + (size_t)s0 * kValueHidden + o;
-    constexpr int kHeld = 26;        // weights held in registers; the rest come from L1 / L2 later
+    constexpr int kHeld = kHeadGroup == 1 ? 26 : 18;        // weights held in registers; the rest come from L2 later
     float wr[kHeld];
 #pragma unroll
     for (int i = 0; i < kHeld; i++) wr[i] = owns ? wsrc[i * outs] : 0.f;
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (err_out != nullptr && blockIdx.x == 0 && t == 0) *err_out = *err;
-    for (int pos = blockIdx.x / kHeadCtas; pos < n; pos += gridDim.x / kHeadCtas) {
-        for (int s = warp; s < cells; s += warps) {
-            const float3 r = head_conv_cell<T>(X + head_row<kCells>(pos, s0 + s) * ldx, w, Cp, lo_off, lo_e5m2, lane);
+    const int stride = static_cast<int>(gridDim.x / kHeadCtas) * kHeadGroup;
+    for (int first = static_cast<int>(blockIdx.x / kHeadCtas) * kHeadGroup; first < n; first += stride) {
+        const int group = n - first < kHeadGroup ? n - first : kHeadGroup;
+        for (int i = warp; i < cells * group; i += warps) {
+            const int g = i / cells, s = i - g * cells;
+            const float3 r =
+                head_conv_cell<T>(X + head_row<kCells>(first + g, s0 + s) * ldx, w, Cp, lo_off, lo_e5m2, lane);
             if (lane < 3) {
                 const float raw = lane == 0 ? r.x : (lane == 1 ? r.y : r.z);
                 const float m = lane < 2 ? h.bn_pol_mean[lane] : h.bn_val_mean[0];
                 const float is = lane < 2 ? h.bn_pol_invstd[lane] : h.bn_val_invstd[0];
-                x[lane][s] = fmaxf(nf_mul(is, nf_add(raw, -m)), 0.f);
+                x[lane][s][g] = fmaxf(nf_mul(is, nf_add(raw, -m)), 0.f);
             }
         }
         __syncthreads();
         if (owns) {
-            const float* xp = x[plane];
-            float acc = 0.f;
+            const float* xp = &x[plane][0][0];
+            float acc[kHeadGroup] = {};
 #pragma unroll
-            for (int i = 0; i < kHeld; i++) acc = fmaf(wr[i], xp[i], acc);
-#pragma unroll 8
-            for (int i = kHeld; i < cells; i++) acc = fmaf(wsrc[i * outs], xp[i], acc);
-            if (plane < 2) store_to_cta(&part_pol[2 * rank + plane][o], 0, acc);
-            else store_to_cta(&part_val[rank][o], 1, acc);
+            for (int i = 0; i < kHeld; i++) {
+#pragma unroll
+                for (int g = 0; g < kHeadGroup; g++) acc[g] = fmaf(wr[i], xp[i * kHeadGroup + g], acc[g]);
+            }
+#pragma unroll 7
+            for (int i = kHeld; i < cells; i++) {
+                const float wv = wsrc[i * outs];
+#pragma unroll
+                for (int g = 0; g < kHeadGroup; g++) acc[g] = fmaf(wv, xp[i * kHeadGroup + g], acc[g]);
+            }
+#pragma unroll
+            for (int g = 0; g < kHeadGroup; g++) {
+                if (plane < 2) store_to_cta(&part_pol[2 * rank + plane][o], g, acc[g]);
+                else store_to_cta(&part_val[rank][o], (g + 1) % kHeadCtas, acc[g]);
+            }
         }
         __syncthreads();                  // every warp whole again before the aligned cluster barrier
         head_cluster_sync();              // all partial sums have arrived
-        if (rank == 0) {
+        if (rank < group) {
             float logit = -INFINITY;
             if (t < kMoves) {
                 float acc = 0.f;
@@ -208,8 +226,10 @@ __global__ void __cluster_dims__(kHeadCtas, 1, 1) __launch_bounds__(kHeadThreads
             const float mx = block_reduce(logit, scratch, true);
             const float e = t < kMoves ? expf((logit - mx) * inv_temp) : 0.f;
             const float denom = block_reduce(e, scratch, false);
-            if (t < kMoves) policy[(size_t)pos * kMoves + t] = e / denom;
-        } else if (rank == 1) {
+            if (t < kMoves) policy[(size_t)(first + rank) * kMoves + t] = e / denom;
+        }
+        const int vg = (rank + kHeadCtas - 1) % kHeadCtas;      // whose value head this CTA finishes
+        if (vg < group) {
             float v = 0.f;
             if (t < kValueHidden) {
                 float acc = 0.f;
@@ -218,11 +238,11 @@ __global__ void __cluster_dims__(kHeadCtas, 1, 1) __launch_bounds__(kHeadThreads
                 v = h.ip2_val_w[t] * fmaxf(h.ip1_val_b[t] + acc, 0.f);
             }
             const float sum = block_reduce(v, scratch, false);
-            if (t == 0) winrate[pos] = (1.0f + tanhf(h.ip2_val_b[0] + sum)) / 2.0f;
+            if (t == 0) winrate[first + vg] = (1.0f + tanhf(h.ip2_val_b[0] + sum)) / 2.0f;
         }
-        if (pos + static_cast<int>(gridDim.x / kHeadCtas) < n) {
+        if (first + stride < n) {
             __syncthreads();
-            head_cluster_sync();          // the sums are read: the next position may overwrite them
+            head_cluster_sync();          // the sums are read: the next group may overwrite them
         }
     }
 }

@@ -97,21 +97,22 @@ EncodeTiledFn encode_tiled_fn() {
 // maps use boxes of 64 columns (128 bytes) x box_rows under the 128-byte swizzle
 // the UMMA descriptors expect; the output maps of the convolution kernel use
 // 32 x 32 boxes under the 64-byte swizzle.
-// precision < 0: a byte tensor (e5m2 planes).  pitch_bytes 0: rows are dense.
+// precision < 0: a byte tensor (e5m2 planes); LZB_FP32: fp32 elements.  pitch_bytes 0: rows are dense.
 int make_map_2d(CUtensorMap* map, int precision, void* base, uint64_t rows, uint64_t cols,
                 uint32_t box_rows, uint32_t box_cols = 64,
                 CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B, uint64_t pitch_bytes = 0) {
     EncodeTiledFn fn = encode_tiled_fn();
     if (!fn) return fail(LZB_ERR_CUDA, "cuTensorMapEncodeTiled entry point not available");
-    const uint64_t elt = precision < 0 ? 1 : 2;
+    const uint64_t elt = precision < 0 ? 1 : (precision == LZB_FP32 ? 4 : 2);
     const cuuint64_t dims[2] = {cols, rows};
     const cuuint64_t strides[1] = {pitch_bytes ? pitch_bytes : cols * elt};
     const cuuint32_t box[2] = {box_cols, box_rows};
     const cuuint32_t estr[2] = {1, 1};
     const CUtensorMapDataType dt =
-        precision < 0 ? CU_TENSOR_MAP_DATA_TYPE_UINT8
-                      : (precision == LZB_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
-                                               : CU_TENSOR_MAP_DATA_TYPE_FLOAT16);
+        precision < 0             ? CU_TENSOR_MAP_DATA_TYPE_UINT8
+        : precision == LZB_FP32   ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
+        : precision == LZB_BF16   ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
+                                  : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
     CUresult r = fn(map, dt, 2, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                     swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -153,7 +154,7 @@ struct Layer {
     int cin_p = 0;
     bool present = false;
     CUtensorMap tmU;            // Winograd modes: box 64 x Kp; fp32 (three planes): box 64 x 64
-    CUtensorMap tmU128;         // fp32: box 64 x 128
+    CUtensorMap tmU32;          // fp32: box 64 x 32
     void* Wd = nullptr;         // direct path: [9][Kp][cinw] storage type
     int cinw = 0;               // input-channel extent of Wd: cin_p x weight planes
     int achunks = 0;            // 64-channel chunks of the activation tensor this layer reads
@@ -206,6 +207,7 @@ struct lzb_pipe {
     // the kernel are resident at once (0: not used).
     lzb::dct::TowerLayer* tower_table[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     int tower_pairs = 0;
+    int head_clusters = 1;      // clusters of the head kernel resident at once
     std::atomic<bool> tower_refused{false};      // a cooperative launch of it failed once: not tried again
     float* head_w = nullptr;   // [3][Cp] fp32
     bool head_convs = false;
@@ -237,6 +239,7 @@ struct lzb_ctx {
     int* h_err = nullptr;  // pinned
     CUtensorMap tmV_first, tmV;
     CUtensorMap tmV32_first, tmV32;  // fp32: boxes of 32 rows
+    CUtensorMap tmM;                 // fp32: 32 x 32 output stores
     // direct path: padded cell-major activations
     int Qa = 0;            // rows allocated in IN / X / H
     void *IN = nullptr, *H = nullptr;
@@ -330,34 +333,37 @@ struct LaunchScope {
     }
 };
 
-// fp32: contraction as three bf16 planes (gemm_f32x3.cuh), persistent CTAs.
-// Items of 128 output channels, or of 64 where the SMs could take twice as many
-// (an MMA of N = 64 takes 49 cycles, one of N = 128 65: not worth it otherwise).
-bool gemm_f32_narrow(const lzb_pipe* p, int nblk) {
-    return p->Cp % 128 != 0 || 2 * kPoints * (p->Cp / 128) * nblk <= p->sm_count;
-}
+// fp32: contraction as three bf16 planes (gemm_f32x3.cuh), persistent CTAs: pairs,
+// with 128 output channels per item where the channels divide, from 129 rows on;
+// single CTAs with 64 channels below (36 points x 4 slices of 256 channels = 144
+// items for 148 SMs, and a pair's second CTA would have no rows).
 int launch_gemm_f32(lzb_ctx* c, const Layer& L, int P, bool first) {
     lzb_pipe* p = c->pipe;
-    const int nblk = (P + tc::kBlockM - 1) / tc::kBlockM;
-    const bool narrow = gemm_f32_narrow(p, nblk);
-    const int items = kPoints * (p->Cp / (narrow ? 64 : 128)) * nblk;
+    const bool pair = P > tc::kBlockM, wide = pair && p->Cp % 128 == 0;
+    const int rows = pair ? 2 * tc::kBlockM : tc::kBlockM, nblk = (P + rows - 1) / rows;
+    const int items = kPoints * (p->Cp / (wide ? 128 : 64)) * nblk;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(std::min(items, p->sm_count));
+    cfg.gridDim = dim3(pair ? 2 * std::min(items, p->sm_count / 2) : std::min(items, p->sm_count));
     cfg.blockDim = dim3(f3::kF3Threads);
-    cfg.dynamicSmemBytes = narrow ? f3::Shape<64>::smem : f3::Shape<128>::smem;
+    cfg.dynamicSmemBytes = f3::kF3Smem;
     cfg.stream = c->stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = pair ? 2 : 1;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
+    auto kernel = wide ? f3::gemm_f32x3_kernel<128, true>
+                       : (pair ? f3::gemm_f32x3_kernel<64, true> : f3::gemm_f32x3_kernel<64, false>);
     cudaError_t le;
     {
         LaunchScope scope(c, kClassContraction);
-        le = cudaLaunchKernelEx(&cfg, narrow ? f3::gemm_f32x3_kernel<64> : f3::gemm_f32x3_kernel<128>,
-                                first ? c->tmV_first : c->tmV, first ? c->tmV32_first : c->tmV32,
-                                narrow ? L.tmU : L.tmU128, static_cast<float*>(c->M), c->Pa, P, p->Cp, L.cin_p, nblk,
-                                c->d_err);
+        // U rows a CTA stages: half of N for a pair
+        le = cudaLaunchKernelEx(&cfg, kernel, first ? c->tmV_first : c->tmV, first ? c->tmV32_first : c->tmV32,
+                                pair && !wide ? L.tmU32 : L.tmU, c->tmM, c->Pa, P, p->Cp, L.cin_p, nblk, c->d_err);
     }
     LZB_CUDA(le);
     LZB_CUDA(cudaGetLastError());
@@ -476,10 +482,17 @@ int launch_heads(lzb_ctx* c, const Job& job, int nb, int ldx, int lo_off, int lo
             const Heads& h = p->heads;
             const HeadWeights hw = {h.bn_pol_mean, h.bn_pol_invstd, h.ip_pol_wT, h.ip_pol_b, h.bn_val_mean,
                                     h.bn_val_invstd, h.ip1_val_wT, h.ip1_val_b, h.ip2_val_w, h.ip2_val_b};
-            // one CTA per SM: more positions than clusters fit share a cluster's weights
-            cfg.gridDim = dim3(kHeadCtas * std::min(nb, p->sm_count / kHeadCtas));
+            // as many clusters as are resident at once (a CTA takes an SM); the fewest
+            // positions per cluster and round that give every position a place
+            const int per_cluster = (nb + p->head_clusters - 1) / p->head_clusters;
+            const int group = per_cluster <= 1 ? 1 : (per_cluster <= 2 ? 2 : (per_cluster <= 4 ? 4 : 8));
+            auto kernel = heads_kernel<T, kCells, 1>;
+            if (group == 2) kernel = heads_kernel<T, kCells, 2>;
+            if (group == 4) kernel = heads_kernel<T, kCells, 4>;
+            if (group == 8) kernel = heads_kernel<T, kCells, 8>;
+            cfg.gridDim = dim3(kHeadCtas * std::min((nb + group - 1) / group, p->head_clusters));
             cfg.blockDim = dim3(kHeadThreads);
-            le = cudaLaunchKernelEx(&cfg, heads_kernel<T, kCells>, X, (const float*)p->head_w, p->Cp, nb, ldx, lo_off,
+            le = cudaLaunchKernelEx(&cfg, kernel, X, (const float*)p->head_w, p->Cp, nb, ldx, lo_off,
                                     lo_e5m2, hw, job.inv_temp, job.out0, job.out1, (const int*)c->d_err, job.err_out);
         } else {
             cfg.gridDim = dim3((nb * kSq + 31) / 32);
@@ -732,10 +745,14 @@ int set_smem_attrs() {
     LZB_CUDA(cudaFuncSetAttribute(in_transform_kernel<__nv_bfloat16, false>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   kXformSmem));
-    LZB_CUDA(cudaFuncSetAttribute(f3::gemm_f32x3_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  f3::Shape<64>::smem));
-    LZB_CUDA(cudaFuncSetAttribute(f3::gemm_f32x3_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  f3::Shape<128>::smem));
+    {
+        const void* variants[] = {(const void*)f3::gemm_f32x3_kernel<64, false>,
+                                  (const void*)f3::gemm_f32x3_kernel<64, true>,
+                                  (const void*)f3::gemm_f32x3_kernel<128, true>};
+        for (const void* k : variants) {
+            LZB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, f3::kF3Smem));
+        }
+    }
     LZB_CUDA(cudaFuncSetAttribute(tc::gemm_tc_kernel<__half>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, tc::kSmemBytes));
     LZB_CUDA(cudaFuncSetAttribute(tc::gemm_tc_kernel<__nv_bfloat16>,
@@ -769,8 +786,20 @@ int set_smem_attrs() {
     return LZB_OK;
 }
 
-// How many CTA pairs of the one-launch tower the device holds at once (0 if the
-// question fails: it is then not used).
+// How many clusters of the head kernel the device holds at once.
+int head_resident_clusters() {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kHeadCtas);
+    cfg.blockDim = dim3(kHeadThreads);
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, heads_kernel<float, false, 8>, &cfg) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return 1;
+    }
+    return n > 0 ? n : 1;
+}
+// How many CTA pairs of the one-launch tower it holds (0 if the question fails: it is
+// then not used).
 int tower_resident_pairs() {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2);
@@ -1072,8 +1101,7 @@ int install_conv(lzb_pipe* p, int layer, const float* src, int c_in, const float
     } else if (p->precision == LZB_FP32) {
         const uint64_t rows = (uint64_t)kPoints * p->Cp, cols = (uint64_t)3 * L.cin_p;
         rc = make_map_2d(&L.tmU, LZB_BF16, L.U, rows, cols, 64);
-        if (!rc && p->Cp % 128 == 0) rc = make_map_2d(&L.tmU128, LZB_BF16, L.U, rows, cols, 128);
-        else L.tmU128 = L.tmU;
+        if (!rc) rc = make_map_2d(&L.tmU32, LZB_BF16, L.U, rows, cols, 32);
         if (rc) return rc;
     } else {
         rc = make_map_2d(&L.tmU, p->precision, L.U, (uint64_t)kPoints * p->Cp, L.cin_p, p->Cp);
@@ -1191,6 +1219,7 @@ int lzb_pipe_create(lzb_pipe** out, int device, int channels, int blocks, int pr
     p->elt = precision == LZB_FP32 ? 4 : 2;
     p->sm_count = prop.multiProcessorCount;
     if (p->pairs) p->tower_pairs = tower_resident_pairs();
+    p->head_clusters = head_resident_clusters();
     p->layers.resize(1 + 2 * blocks);
     *out = p;
     return LZB_OK;
@@ -1344,13 +1373,13 @@ static int default_micro_batch(const lzb_pipe* p, int cap) {
             if ((groups * cand) % p->sm_count == 0) { n = cand; break; }
         }
     } else {
-        // fp32: of the counts from 64 down to 40 (V and M of 50 positions at 256 channels
-        // are 116 MB), the one whose items (128 rows x 128 channels) fill their last
-        // wave best
+        // fp32: of the counts from 64 down to 40, the one whose items (256 rows x 128
+        // channels, CTA pairs) fill their last wave best
         double best = 0.0;
+        const int pairs = p->sm_count / 2;
         for (int cand = kDefaultMicroBatch; cand >= 40; cand--) {
-            const int items = round_up(cand * kTilesPerPos, tc::kBlockM) / tc::kBlockM * ((p->Cp + 127) / 128) * kPoints;
-            const int waves = (items + p->sm_count - 1) / p->sm_count;
+            const int items = round_up(cand * kTilesPerPos, 256) / 256 * ((p->Cp + 127) / 128) * kPoints;
+            const int waves = (items + pairs - 1) / pairs;
             const double rate = static_cast<double>(cand) / waves;     // positions per wave
             if (rate > best * 1.02) { best = rate; n = cand; }
         }
@@ -1447,6 +1476,7 @@ int lzb_ctx_create(lzb_ctx** out, lzb_pipe* p, int max_batch) {
         if (!rc) rc = make_map_2d(&c->tmV32_first, LZB_BF16, c->V, rows, 3 * 64, 32);
         if (!rc) rc = make_map_2d(&c->tmV, LZB_BF16, c->V, rows, (uint64_t)3 * p->Cp, tc::kBlockM);
         if (!rc) rc = make_map_2d(&c->tmV32, LZB_BF16, c->V, rows, (uint64_t)3 * p->Cp, 32);
+        if (!rc) rc = make_map_2d(&c->tmM, LZB_FP32, c->M, rows, p->Cp, 32, 32);
         if (rc) {
             lzb_ctx_destroy(c);
             return rc;

@@ -43,14 +43,23 @@ template <typename T, bool kSplit> struct TileOut {
 };
 template <> struct TileOut<float, true> {
     using type = __nv_bfloat16;
+    static __device__ __forceinline__ float2 widen(__nv_bfloat162 v) {
+        const uint32_t u = *reinterpret_cast<const uint32_t*>(&v);
+        return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xFFFF0000u));
+    }
+    static __device__ __forceinline__ void split(float2 v, __nv_bfloat162 (&p)[3]) {
+        p[0] = __float22bfloat162_rn(v);
+        const float2 r1 = sub_packed(v, widen(p[0]));          // exact, as is the next one
+        p[1] = __float22bfloat162_rn(r1);
+        p[2] = __float22bfloat162_rn(sub_packed(r1, widen(p[1])));
+    }
     static __device__ __forceinline__ void store(__nv_bfloat16* V, size_t row, int C, int off, float2 v) {
-        __nv_bfloat162 p0, p1, p2;
-        f3::split3(v.x, p0.x, p1.x, p2.x);
-        f3::split3(v.y, p0.y, p1.y, p2.y);
+        __nv_bfloat162 p[3];
+        split(v, p);
         __nv_bfloat16* dst = V + row * 3 * C + off;
-        *reinterpret_cast<__nv_bfloat162*>(dst) = p0;
-        *reinterpret_cast<__nv_bfloat162*>(dst + C) = p1;
-        *reinterpret_cast<__nv_bfloat162*>(dst + 2 * C) = p2;
+        *reinterpret_cast<__nv_bfloat162*>(dst) = p[0];
+        *reinterpret_cast<__nv_bfloat162*>(dst + C) = p[1];
+        *reinterpret_cast<__nv_bfloat162*>(dst + 2 * C) = p[2];
     }
 };
 // The storage of V in a pipe of type T.
@@ -289,13 +298,16 @@ __global__ void __launch_bounds__(kXf32Threads, 2) xform_f32_kernel(
     const float2 scale = *reinterpret_cast<const float2*>(bn_invstd + k);
     asm volatile("griddepcontrol.wait;" ::: "memory");
 
-    const float* msrc = M + (size_t)(n * kTilesPerPos + tile) * Cp + k;
-    const size_t pt_stride = (size_t)Pa * Cp;
+    // byte offsets of 32 bits from the kernel's pointers (V is the largest tensor, 36 x
+    // 6400 rows of 6 Cp bytes): one add per access
+    const unsigned char* mb = reinterpret_cast<const unsigned char*>(M);
+    const uint32_t m0 = static_cast<uint32_t>((n * kTilesPerPos + tile) * Cp + k) * 4u;
+    const uint32_t pt_stride = static_cast<uint32_t>(Pa * Cp) * 4u;
     float2 temp[4][6];
     {
         float2 m[36];
 #pragma unroll
-        for (int t = 0; t < 36; t++) m[t] = __ldcg(reinterpret_cast<const float2*>(msrc + t * pt_stride));
+        for (int t = 0; t < 36; t++) m[t] = __ldcg(reinterpret_cast<const float2*>(mb + (m0 + t * pt_stride)));
 #pragma unroll
         for (int nu = 0; nu < 6; nu++) {
             const float2 col[6] = {m[nu], m[6 + nu], m[12 + nu], m[18 + nu], m[24 + nu], m[30 + nu]};
@@ -324,8 +336,7 @@ __global__ void __launch_bounds__(kXf32Threads, 2) xform_f32_kernel(
             const int x = 4 * bx + j;
             if (x >= kBoard) continue;
             // max(0, invstd * (v - mean) [+ residual]), src/CPUPipe.cpp:352-377
-            float2 v = make_float2(op_mul<true>(scale.x, op_add<true>(o4[j].x, -mean.x)),
-                                   op_mul<true>(scale.y, op_add<true>(o4[j].y, -mean.y)));
+            float2 v = mul_packed(scale, sub_packed(o4[j], mean));
             if (R != nullptr) v = add2<true>(v, r4[j]);
             v.x = fmaxf(v.x, 0.f);
             v.y = fmaxf(v.y, 0.f);
@@ -347,14 +358,23 @@ __global__ void __launch_bounds__(kXf32Threads, 2) xform_f32_kernel(
 #pragma unroll
         for (int r = 0; r < 6; r++) t1[r][col] = vout[r];
     }
-    const int p = n * kTilesPerPos + tile;
+    unsigned char* vb = reinterpret_cast<unsigned char*>(V);
+    const uint32_t plane = static_cast<uint32_t>(Cp) * 2u, v_stride = static_cast<uint32_t>(Pa) * 3u * plane;
+    uint32_t off = static_cast<uint32_t>(n * kTilesPerPos + tile) * 3u * plane + static_cast<uint32_t>(k) * 2u;
+    unsigned char* vb1 = vb + plane;
+    unsigned char* vb2 = vb + 2 * static_cast<size_t>(plane);
 #pragma unroll
     for (int xi = 0; xi < 6; xi++) {
         float2 vout[6];
         apply_bt<true>(vout, t1[xi]);
 #pragma unroll
         for (int nu = 0; nu < 6; nu++) {
-            TileOut<float, true>::store(V, (size_t)(xi * 6 + nu) * Pa + p, Cp, k, vout[nu]);
+            __nv_bfloat162 pl[3];
+            TileOut<float, true>::split(vout[nu], pl);
+            *reinterpret_cast<__nv_bfloat162*>(vb + off) = pl[0];
+            *reinterpret_cast<__nv_bfloat162*>(vb1 + off) = pl[1];
+            *reinterpret_cast<__nv_bfloat162*>(vb2 + off) = pl[2];
+            off += v_stride;
         }
     }
 }

@@ -21,8 +21,6 @@ constexpr int kTilesPerPos = 25;   // P
 constexpr int kPoints = 36;        // alpha^2
 constexpr float kSq2 = 1.4142135623730951f;
 
-__device__ __forceinline__ float2 operator-(float2 a) { return make_float2(-a.x, -a.y); }
-
 // Two flavours of every operation: kExact keeps multiplies and adds apart
 // (__fmul_rn/__fadd_rn are never contracted into FMAs), so that the fp32 path
 // reproduces the CPU pipe's transform values bit for bit; the other flavour
@@ -36,14 +34,41 @@ template <bool kExact> __device__ __forceinline__ float op_add(float a, float b)
 }
 __device__ __forceinline__ float nf_mul(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ float nf_add(float a, float b) { return __fadd_rn(a, b); }
+// Both channels in one instruction (sm_100 packed fp32; the two results are rounded
+// like two separate operations, and nothing is contracted).
+__device__ __forceinline__ unsigned long long f2_bits(float2 v) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(v.x), "f"(v.y));
+    return r;
+}
+__device__ __forceinline__ float2 f2_from(unsigned long long r) {
+    float2 v;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(r));
+    return v;
+}
+__device__ __forceinline__ float2 add_packed(float2 a, float2 b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));
+    return f2_from(r);
+}
+__device__ __forceinline__ float2 sub_packed(float2 a, float2 b) {
+    unsigned long long r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));
+    return f2_from(r);
+}
+__device__ __forceinline__ float2 mul_packed(float2 a, float2 b) {
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));
+    return f2_from(r);
+}
 template <bool kExact> __device__ __forceinline__ float2 mul2(float2 a, float s) {
-    return make_float2(op_mul<kExact>(a.x, s), op_mul<kExact>(a.y, s));
+    return kExact ? mul_packed(a, make_float2(s, s)) : make_float2(a.x * s, a.y * s);
 }
 template <bool kExact> __device__ __forceinline__ float2 add2(float2 a, float2 b) {
-    return make_float2(op_add<kExact>(a.x, b.x), op_add<kExact>(a.y, b.y));
+    return kExact ? add_packed(a, b) : make_float2(a.x + b.x, a.y + b.y);
 }
 template <bool kExact> __device__ __forceinline__ float2 sub2(float2 a, float2 b) {
-    return make_float2(op_add<kExact>(a.x, -b.x), op_add<kExact>(a.y, -b.y));
+    return kExact ? sub_packed(a, b) : make_float2(a.x - b.x, a.y - b.y);
 }
 
 // o = B^T i, factored as in src/CPUPipe.cpp:88-106.
@@ -53,11 +78,11 @@ __device__ __forceinline__ void apply_bt(float2 (&o)[6], const float2 (&i)[6]) {
     float2 b = add2<kExact>(mul2<kExact>(i[2], -2.0f), i[4]);
     o[0] = add2<kExact>(add2<kExact>(i[0], mul2<kExact>(i[2], -5.0f / 2.0f)), i[4]);
     o[1] = add2<kExact>(a, b);
-    o[2] = add2<kExact>(-a, b);
+    o[2] = sub2<kExact>(b, a);
     float2 a2 = add2<kExact>(mul2<kExact>(i[3], kSq2), mul2<kExact>(i[1], -kSq2 / 2.0f));
     float2 b2 = add2<kExact>(mul2<kExact>(i[2], -1.0f / 2.0f), i[4]);
     o[3] = add2<kExact>(a2, b2);
-    o[4] = add2<kExact>(-a2, b2);
+    o[4] = sub2<kExact>(b2, a2);
     o[5] = add2<kExact>(add2<kExact>(i[1], mul2<kExact>(i[3], -5.0f / 2.0f)), i[5]);
 }
 
