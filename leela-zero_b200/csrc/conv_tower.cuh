@@ -181,9 +181,11 @@ struct UnitWalk {
 // the e5m2 plane from byte 0, the hi8 plane from byte Kp).  X, H : the two
 // activation tensors, ldr elements of T per cell row.  input : the network input, converted here into IN (64 channels of T per cell row,
 // channels 24 .. 63 zero beforehand).  ntiles row tiles (three per position),
-// nsplit slices.  counts : [n_layers + 1][tile_cap] words, row l for the tiles
-// layer l reads, zero when the kernel starts; counts_next : the same for the next
-// run on this context, cleared here.
+// nsplit slices.  count_sets : two sets of [n_layers + 1][tile_cap] words, row l for
+// the tiles layer l reads.  *run, the number of runs so far, says which set is this
+// run's (all zero when the kernel starts); the other one is cleared here for the
+// next run.  The number lies on the device and is raised by the head kernel, so
+// that a captured run can be replayed.
 template <typename T, int kPlanes>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTowerThreads, 1) conv_tower_kernel(
     const __grid_constant__ CUtensorMap tmIN, const __grid_constant__ CUtensorMap tmX,
@@ -191,8 +193,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTowerThreads, 1) co
     const __grid_constant__ CUtensorMap tmHl, const __grid_constant__ CUtensorMap tmXo,
     const __grid_constant__ CUtensorMap tmHo, const __grid_constant__ CUtensorMap tmXlo,
     const __grid_constant__ CUtensorMap tmHlo, const TowerLayer* __restrict__ layers, int n_layers,
-    const InputView input, T* IN, T* X, T* H, int ntiles, int Kp, int nsplit, int ldr, uint32_t* counts,
-    uint32_t* counts_next, int tile_cap, int* err) {
+    const InputView input, T* IN, T* X, T* H, int ntiles, int Kp, int nsplit, int ldr,
+    uint32_t* count_sets, const uint32_t* run, int tile_cap, int* err) {
     extern __shared__ unsigned char smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
@@ -226,6 +228,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTowerThreads, 1) co
     const int fit = static_cast<int>(kTowerRingBytes / stage_bytes);
     const int nstages = fit < kTowerMaxStages ? fit : kTowerMaxStages;
 
+    const uint32_t odd = __ldcg(run) & 1u;
+    const int set_words = (n_layers + 1) * tile_cap;
+    uint32_t* counts = count_sets + (odd ? set_words : 0);
+    uint32_t* counts_next = count_sets + (odd ? 0 : set_words);
+
     if (threadIdx.x == 0) {
         for (int i = 0; i < kTowerMaxStages; i++) {
             mbar_init(bfull_bar(i), 2);      // one arrive.expect_tx per CTA of the pair
@@ -244,7 +251,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTowerThreads, 1) co
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    for (int i = blockIdx.x * kTowerThreads + threadIdx.x; i < (n_layers + 1) * tile_cap; i += gridDim.x * kTowerThreads) {
+    for (int i = blockIdx.x * kTowerThreads + threadIdx.x; i < set_words; i += gridDim.x * kTowerThreads) {
         counts_next[i] = 0u;
     }
     if (warp == 1) {

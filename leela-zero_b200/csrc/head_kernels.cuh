@@ -112,13 +112,17 @@ __device__ __forceinline__ size_t head_row(int n, int s) {
 
 // Raw head planes pol[n][2][361], val[n][361] (which may be page-locked host memory):
 // 32 board cells per CTA, four per warp, written as whole rows of 128 bytes.
-// err_out, if given, receives *err.
+// err_out, if given, receives *err; run, if given, counts the tower run that ends here.
 template <typename T, bool kCells>
 __global__ void __launch_bounds__(256) head_planes_kernel(const T* X, const float* __restrict__ w, int Cp, int n,
                                                           float* __restrict__ pol, float* __restrict__ val, int ldx,
-                                                          int lo_off, int lo_e5m2, const int* err, int* err_out) {
+                                                          int lo_off, int lo_e5m2, const int* err, int* err_out,
+                                                          uint32_t* run) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (err_out != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *err_out = *err;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        if (err_out != nullptr) *err_out = *err;
+        if (run != nullptr) *run += 1u;
+    }
     __shared__ float out[3][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int first = blockIdx.x * 32;
@@ -156,7 +160,10 @@ template <typename T, bool kCells, int kHeadGroup>
 __global__ void __cluster_dims__(kHeadCtas, 1, 1) __launch_bounds__(kHeadThreads)
     heads_kernel(const T* X, const float* __restrict__ w, int Cp, int n, int ldx, int lo_off, int lo_e5m2,
                  const HeadWeights h, float inv_temp, float* __restrict__ policy, float* __restrict__ winrate,
-                 const int* err, int* err_out) {
+                 const int* err, int* err_out, uint32_t* run) {
+    // a CTA's shared memory may be written from the cluster once that CTA runs: every
+    // thread says so here and looks before its first remote store
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     __shared__ float x[3][kHeadCells][kHeadGroup];
     __shared__ float part_pol[2 * kHeadCtas][kMoves];       // of the position this CTA finishes
     __shared__ float part_val[kHeadCtas][kValueHidden];
@@ -177,7 +184,11 @@ __global__ void __cluster_dims__(kHeadCtas, 1, 1) __launch_bounds__(kHeadThreads
 #pragma unroll
     for (int i = 0; i < kHeld; i++) wr[i] = owns ? wsrc[i * outs] : 0.f;
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (err_out != nullptr && blockIdx.x == 0 && t == 0) *err_out = *err;
+    if (blockIdx.x == 0 && t == 0) {
+        if (err_out != nullptr) *err_out = *err;
+        if (run != nullptr) *run += 1u;
+    }
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
     const int stride = static_cast<int>(gridDim.x / kHeadCtas) * kHeadGroup;
     for (int first = static_cast<int>(blockIdx.x / kHeadCtas) * kHeadGroup; first < n; first += stride) {
         const int group = n - first < kHeadGroup ? n - first : kHeadGroup;

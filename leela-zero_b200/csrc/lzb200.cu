@@ -231,10 +231,12 @@ struct lzb_ctx {
     unsigned int* h_packed = nullptr;   // page-locked
     float* h_out = nullptr;             // page-locked
     // One-launch tower: arrival counters of the tiles, two sets of [layers + 1][tile_cap]
-    // words used in turn (a run clears the other set); null: a launch per layer
+    // words used in turn (a run clears the other set), and a word that counts the runs;
+    // null: a launch per layer
     uint32_t* tile_counts = nullptr;
     int tile_cap = 0;
-    uint32_t tower_runs = 0;
+    size_t tile_count_words() const { return (size_t)2 * (2 + 2 * pipe->blocks) * tile_cap; }
+    uint32_t* tower_runs() const { return tile_counts + tile_count_words(); }
     int* d_err = nullptr;
     int* h_err = nullptr;  // pinned
     CUtensorMap tmV_first, tmV;
@@ -463,9 +465,9 @@ struct Job {
 // The last launch of an evaluation: 1x1 head convolutions, and the heads where the
 // job wants them.  Programmatic launch: its blocks are placed as soon as there is
 // room (the tower leaves SMs free in small batches) and fetch their weights while
-// the tower still runs.
+// the tower still runs.  run: the context's count of tower runs, raised here, or null.
 template <typename T, bool kCells>
-int launch_heads(lzb_ctx* c, const Job& job, int nb, int ldx, int lo_off, int lo_e5m2) {
+int launch_heads(lzb_ctx* c, const Job& job, int nb, int ldx, int lo_off, int lo_e5m2, uint32_t* run) {
     lzb_pipe* p = c->pipe;
     cudaLaunchConfig_t cfg = {};
     cfg.stream = c->stream;
@@ -493,12 +495,13 @@ int launch_heads(lzb_ctx* c, const Job& job, int nb, int ldx, int lo_off, int lo
             cfg.gridDim = dim3(kHeadCtas * std::min((nb + group - 1) / group, p->head_clusters));
             cfg.blockDim = dim3(kHeadThreads);
             le = cudaLaunchKernelEx(&cfg, kernel, X, (const float*)p->head_w, p->Cp, nb, ldx, lo_off,
-                                    lo_e5m2, hw, job.inv_temp, job.out0, job.out1, (const int*)c->d_err, job.err_out);
+                                    lo_e5m2, hw, job.inv_temp, job.out0, job.out1, (const int*)c->d_err, job.err_out,
+                                    run);
         } else {
             cfg.gridDim = dim3((nb * kSq + 31) / 32);
             cfg.blockDim = dim3(256);
             le = cudaLaunchKernelEx(&cfg, head_planes_kernel<T, kCells>, X, (const float*)p->head_w, p->Cp, nb,
-                                    job.out0, job.out1, ldx, lo_off, lo_e5m2, (const int*)c->d_err, job.err_out);
+                                    job.out0, job.out1, ldx, lo_off, lo_e5m2, (const int*)c->d_err, job.err_out, run);
         }
     }
     LZB_CUDA(le);
@@ -530,7 +533,7 @@ int run_tower(lzb_ctx* c, const Job& job, int nb) {
         const bool last = (b + 1 == p->blocks);
         if ((rc = launch_xform<T>(c, l2, nb, X, X, last ? nullptr : V))) return rc;
     }
-    return launch_heads<T, false>(c, job, nb, p->Cp, 0, 0);
+    return launch_heads<T, false>(c, job, nb, p->Cp, 0, 0, nullptr);
 }
 
 template <typename T>
@@ -641,9 +644,6 @@ int launch_tower(lzb_ctx* c, const InputView& in, int nb, bool* refused) {
     const int ntiles = dct::kTilesPerPos128 * nb, npairs = (ntiles + 1) / 2;
     const int ns = tower_slices(p, npairs);
     const int n_layers = static_cast<int>(p->layers.size());
-    const size_t words = static_cast<size_t>(n_layers + 1) * c->tile_cap;
-    uint32_t* counts = c->tile_counts + (c->tower_runs & 1u) * words;
-    uint32_t* counts_next = c->tile_counts + ((c->tower_runs & 1u) ^ 1u) * words;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * std::min(npairs * ns, p->tower_pairs));
     cfg.blockDim = dim3(dct::kTowerThreads);
@@ -663,8 +663,9 @@ int launch_tower(lzb_ctx* c, const InputView& in, int nb, bool* refused) {
     LaunchScope scope(c, kClassContraction, n_layers);
     cudaError_t le = cudaLaunchKernelEx(
         &cfg, kernel, c->tmIN, c->tmX, c->tmH, bytes ? c->tmXl : c->tmX, bytes ? c->tmHl : c->tmH, c->tmXo, c->tmHo,
-        bytes ? c->tmXlo : c->tmXo, bytes ? c->tmHlo : c->tmHo, (const dct::TowerLayer*)p->tower_table[ns], n_layers, in, static_cast<T*>(c->IN), static_cast<T*>(c->X),
-        static_cast<T*>(c->H), ntiles, p->Cp, ns, p->row_bytes() / p->elt, counts, counts_next, c->tile_cap, c->d_err);
+        bytes ? c->tmXlo : c->tmXo, bytes ? c->tmHlo : c->tmHo, (const dct::TowerLayer*)p->tower_table[ns], n_layers, in,
+        static_cast<T*>(c->IN), static_cast<T*>(c->X), static_cast<T*>(c->H), ntiles, p->Cp, ns, p->row_bytes() / p->elt,
+        c->tile_counts, (const uint32_t*)c->tower_runs(), c->tile_cap, c->d_err);
     if (le == cudaSuccess) le = cudaGetLastError();
     *refused = le != cudaSuccess;
     if (*refused) {
@@ -672,8 +673,6 @@ int launch_tower(lzb_ctx* c, const InputView& in, int nb, bool* refused) {
         (void)cudaGetLastError();
         p->tower_refused = true;
         c->launches--;
-    } else {
-        c->tower_runs++;
     }
     return LZB_OK;
 }
@@ -706,9 +705,14 @@ int run_tower_direct(lzb_ctx* c, const Job& job, int nb) {
             }
         }
     }
-    return launch_heads<T, true>(c, job, nb, p->row_bytes() / p->elt,
-                                 (p->aplanes == 2 || (p->aplanes == 3 && p->layers.back().out_lo)) ? p->Cp : 0,
-                                 p->aplanes == 3 ? 1 : 0);
+    rc = launch_heads<T, true>(c, job, nb, p->row_bytes() / p->elt,
+                               (p->aplanes == 2 || (p->aplanes == 3 && p->layers.back().out_lo)) ? p->Cp : 0,
+                               p->aplanes == 3 ? 1 : 0, per_layer ? nullptr : c->tower_runs());
+    // nobody counted this run: the next one uses the same counters, which must be zero
+    if (rc && !per_layer) {
+        cudaMemsetAsync(c->tile_counts, 0, c->tile_count_words() * sizeof(uint32_t), c->stream);
+    }
+    return rc;
 }
 
 int run_tower_any(lzb_ctx* c, const Job& job, int nb) {
@@ -1318,6 +1322,7 @@ int lzb_pipe_finalize(lzb_pipe* p) {
         if (!p->layers[l].present) return fail(LZB_ERR_ARG, "layer " + std::to_string(l) + " missing");
     }
     if (!p->head_convs) return fail(LZB_ERR_ARG, "head convolutions missing");
+    if (p->finalized) return LZB_OK;
     // records of the one-launch tower (conv_tower.cuh), for each number of slices
     for (int ns = 1; ns <= 4 && p->tower_pairs > 0; ns++) {
         // a channel slice must be a multiple of 64 (two epilogue warps x 32 columns)
@@ -1397,6 +1402,12 @@ int lzb_ctx_create(lzb_ctx** out, lzb_pipe* p, int max_batch) {
     c->pipe = p;
     c->max_batch = max_batch;
     c->micro_cap = max_batch < kMaxMicroBatch ? max_batch : kMaxMicroBatch;
+    if (p->precision == LZB_FP32) {
+        // xform_f32_kernel reaches V, 6 bytes an element, with 32-bit offsets: 256
+        // positions of up to 3,072 channels, fewer of wider networks
+        const long long most = (1ll << 32) / (6ll * kPoints * p->Cp) / 128 * 128 / kTilesPerPos;
+        c->micro_cap = static_cast<int>(std::max(1ll, std::min<long long>(c->micro_cap, most)));
+    }
     cudaError_t e = cudaSuccess;
     auto alloc = [&](void** ptr, size_t bytes) {
         if (e == cudaSuccess) e = cudaMalloc(ptr, bytes);
@@ -1415,7 +1426,7 @@ int lzb_ctx_create(lzb_ctx** out, lzb_pipe* p, int max_batch) {
         const char* tf = getenv("LZB_TILE_FLAGS");
         if (p->tower_pairs > 0 && !(tf != nullptr && atoi(tf) == 0)) {
             c->tile_cap = (dct::kTilesPerPos128 * c->micro_cap + 1) / 2;
-            alloc((void**)&c->tile_counts, (size_t)2 * (2 + 2 * p->blocks) * c->tile_cap * sizeof(uint32_t));
+            alloc((void**)&c->tile_counts, (c->tile_count_words() + 1) * sizeof(uint32_t));
         }
     } else {
         c->micro = default_micro_batch(p, c->micro_cap);
@@ -1547,8 +1558,7 @@ int collect_error(lzb_ctx* c) {
     *c->h_err = 0;
     cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream);
     if (c->tile_counts != nullptr) {
-        cudaMemsetAsync(c->tile_counts, 0, (size_t)2 * (2 + 2 * c->pipe->blocks) * c->tile_cap * sizeof(uint32_t),
-                        c->stream);
+        cudaMemsetAsync(c->tile_counts, 0, c->tile_count_words() * sizeof(uint32_t), c->stream);
     }
     return fail(LZB_ERR_DEVICE_WAIT, "a kernel gave up a bounded wait (code " + std::to_string(code) + ")");
 }

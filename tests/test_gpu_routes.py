@@ -1,0 +1,192 @@
+"""The kernels behind one evaluation at the sizes where their routes change:
+row-tile remainders and channel slices of the one-launch tower, single CTAs and
+CTA pairs of the fp32 contraction, positions per cluster of the head kernel,
+positions read in place or copied, bits or fp32 planes, and a captured run."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def W(lzb):
+    return lzb.weights
+
+
+def _same(a, b):
+    return all(np.array_equal(x, y) for x, y in zip(a, b))
+
+
+@pytest.mark.parametrize("filters", [32, 96, 192, 256])
+@pytest.mark.parametrize("mode", ["fp16", "bf16", "fp16x2", "fp16x3", "bf16x3"])
+def test_tower_gives_the_bits_of_a_launch_per_layer(lzb, W, monkeypatch, mode, filters):
+    """One position is three row tiles (an odd count: the last pair works on a
+    copy), 25 positions are just more units than CTA pairs; the number of slices
+    falls from 4 to 1 along these batches.  Every output is the same sum in the
+    same order as with a launch per layer, whatever batch came before it on the
+    context."""
+    net = W.synthetic_network(5, filters, 2200 + filters, calibrated=True)
+    x = W.synthetic_positions(80, 1200)
+    pipe = lzb.Pipe(net, mode)
+    monkeypatch.setenv("LZB_TILE_FLAGS", "0")
+    layers = pipe.context(80)
+    monkeypatch.delenv("LZB_TILE_FLAGS")
+    tower = pipe.context(80)
+    for n in (1, 2, 80, 3, 11, 25, 37, 1, 49):
+        assert _same(tower.forward(x[:n]), layers.forward(x[:n])), n
+    before = tower.launches
+    tower.forward(x)
+    assert tower.launches - before == 2          # the tower, the head planes
+    pipe.close()
+
+
+def _forward64(net, x):
+    """Raw head planes in 64 bits: direct convolutions with the network's filters."""
+    import torch
+    t = lambda a: torch.from_numpy(np.asarray(a, dtype=np.float64))
+    y = t(x).reshape(-1, 18, 19, 19)
+    res = None
+    for l, f in enumerate(net["filters"]):
+        z = torch.nn.functional.conv2d(y, t(f), padding=1)
+        z = (z - t(net["bn_mean"][l])[None, :, None, None]) * t(net["bn_invstd"][l])[None, :, None, None]
+        if l > 0 and l % 2 == 0:
+            z = z + res
+        y = z.clamp_min(0)
+        if l % 2 == 0:
+            res = y
+    flat = y.reshape(y.shape[0], y.shape[1], 361)
+    pol = torch.einsum("kc,ncs->nks", t(net["pol_w"]).reshape(2, -1), flat)
+    val = torch.einsum("c,ncs->ns", t(net["val_w"]).reshape(-1), flat)
+    return pol.numpy(), val.numpy()
+
+
+@pytest.mark.parametrize("filters", [40, 64, 128, 192, 320])
+def test_fp32_contraction_is_closer_to_64_bits_than_the_fma_chain(lzb, oracle, W, filters):
+    """Rows of a batch: 25 and 125 (single CTAs), 150 (a pair whose second CTA
+    has 22 rows), 275 and 525 (pairs whose second CTA has none), 2000 (cut into
+    micro-batches at 40 positions and more).  The oracle does the same Winograd
+    arithmetic with its contractions as one chain of fp32 additions; three bf16
+    planes must not be further from the 64-bit result than that (5 % for the
+    rounding of the transforms, which both share)."""
+    import torch
+    net = W.synthetic_network(2, filters, 2300 + filters, calibrated=True)
+    x = W.synthetic_positions(80, 1300)
+    ctx = lzb.Pipe(net, "fp32").context(80)
+    got = [np.asarray(a).reshape(80, -1) for a in ctx.forward(x)]
+    for n in (1, 5, 6, 11, 21):
+        part = [np.asarray(a).reshape(n, -1) for a in ctx.forward(x[:n])]
+        # a position's sums do not depend on its neighbours or on the tile shape
+        assert all(np.array_equal(p, g[:n]) for p, g in zip(part, got)), n
+    exact = [a.reshape(21, -1) for a in _forward64(net, x[:21])]
+    chain = [np.asarray(a).reshape(21, -1) for a in oracle.cpu_pipe(net).forward(x[:21])]
+    for g, c, e in zip(got, chain, exact):
+        ours, theirs = np.linalg.norm(g[:21] - e), np.linalg.norm(c - e)
+        assert ours <= 1.05 * theirs, (ours / np.linalg.norm(e), theirs / np.linalg.norm(e))
+    assert torch.isfinite(torch.from_numpy(got[0])).all()
+
+
+@pytest.mark.parametrize("mode", ["fp16", "fp32", "bf16x3"])
+def test_heads_of_several_positions_per_cluster(lzb, W, mode):
+    """1, 2, 4 and 8 positions per cluster and round, remainders in each: the
+    same additions in the same order as for a position alone."""
+    net = W.synthetic_network(1, 64, 2400, calibrated=True)
+    x = W.synthetic_positions(301, 1400)
+    ctx = lzb.Pipe(net, mode).context(301)
+    alone = [ctx.forward_heads(x[i:i + 1]) for i in range(0, 301, 7)]
+    policy = np.concatenate([a[0] for a in alone])
+    win = np.concatenate([a[1] for a in alone])
+    for n in (2, 15, 19, 29, 41, 75, 130, 149, 256, 301):
+        p, w = ctx.forward_heads(x[:n])
+        k = (n + 6) // 7
+        assert np.array_equal(p[::7], policy[:k]) and np.array_equal(w[::7], win[:k]), n
+
+
+@pytest.mark.parametrize("mode", ["fp16x2", "fp32"])
+def test_positions_as_bits_and_as_planes(lzb, W, mode):
+    """0 / 1 planes travel as bits, read in place up to 32 positions and copied
+    above, 1,024 at a time; anything else travels as fp32.  The same planes on
+    the device are read as fp32: equal bits out."""
+    import torch
+    net = W.synthetic_network(1, 64, 2500, calibrated=True)
+    x = W.synthetic_positions(1030, 1500)
+    ctx = lzb.Pipe(net, mode).context(1030)
+    dev = torch.from_numpy(x).cuda()
+    pol = torch.empty((1030, 2, 361), device="cuda")
+    val = torch.empty((1030, 361), device="cuda")
+    torch.cuda.synchronize()
+
+    def planes(src, n):
+        src = src.contiguous()
+        torch.cuda.synchronize()
+        ctx.forward_device(src.data_ptr(), n, pol.data_ptr(), val.data_ptr())
+        ctx.sync()
+        return pol[:n].cpu().numpy(), val[:n].cpu().numpy()
+
+    for n in (1, 32, 33, 1024, 1030):
+        want = planes(dev, n)
+        a = ctx.forward(x[:n])
+        b = ctx.forward_packed(lzb.pack_positions(x[:n]))
+        # page-locked buffers on both sides are copied from and to directly
+        locked = torch.from_numpy(lzb.pack_positions(x[:n]).view(np.int32)).pin_memory()
+        to = torch.empty((n, 722)).pin_memory(), torch.empty((n, 361)).pin_memory()
+        lzb.check(lzb.lib().lzb_ctx_forward_packed(ctx.h, locked.data_ptr(), n, to[0].data_ptr(), to[1].data_ptr()))
+        c = to[0].numpy().copy(), to[1].numpy().copy()
+        to[0].zero_()
+        ctx.forward_ptr(x[:n].ctypes.data, n, to[0].data_ptr(), to[1].data_ptr())
+        d = to[0].numpy(), to[1].numpy()
+        for got in (a, b, c, d):
+            assert np.array_equal(np.asarray(got[0]).reshape(n, -1), want[0].reshape(n, -1)), n
+            assert np.array_equal(np.asarray(got[1]).reshape(n, -1), want[1].reshape(n, -1)), n
+    # one value of one position is neither 0 nor 1: the whole call travels as fp32
+    for value in (0.5, -1.0, 1e-30, 3.0):
+        y = x[:34].copy()
+        y[33, 17].flat[360] = value
+        want = planes(torch.from_numpy(y).cuda(), 34)
+        for n in (34, 33):
+            got = ctx.forward(y[34 - n:])
+            assert np.array_equal(np.asarray(got[0]).reshape(n, -1), want[0].reshape(34, -1)[34 - n:]), value
+
+
+@pytest.mark.parametrize("mode", ["fp16", "fp16x2", "fp32"])
+def test_a_captured_evaluation_replays(lzb, W, mode):
+    """Device-to-device evaluations enqueued under stream capture and replayed:
+    every replay, on other inputs and with plain calls in between, gives the
+    bits of a plain call."""
+    import torch
+    net = W.synthetic_network(3, 128, 2600, calibrated=True)
+    x = torch.from_numpy(W.synthetic_positions(60, 1600)).cuda().reshape(3, 20, -1)
+    ctx = lzb.Pipe(net, mode).context(20)
+    src = x[0].clone()
+    policy, win = torch.empty((20, 362), device="cuda"), torch.empty((20,), device="cuda")
+    stream = torch.cuda.ExternalStream(ctx.stream)
+
+    def enqueue():
+        ctx.forward_heads_device(src.data_ptr(), 20, 1.0, policy.data_ptr(), win.data_ptr())
+
+    def result():
+        torch.cuda.synchronize()
+        ctx.sync()
+        return policy.cpu(), win.cpu()
+
+    want = []
+    for i in range(3):
+        src.copy_(x[i])
+        torch.cuda.synchronize()
+        enqueue()
+        want.append(result())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+        enqueue()
+    for i in (0, 1, 2, 2, 1, 0):
+        src.copy_(x[i])
+        policy.zero_()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(stream):
+            graph.replay()
+        got = result()
+        assert torch.equal(got[0], want[i][0]) and torch.equal(got[1], want[i][1]), i
+        if i == 2:
+            enqueue()
+            got = result()
+            assert torch.equal(got[0], want[i][0]) and torch.equal(got[1], want[i][1]), i
+    del graph
