@@ -37,8 +37,9 @@ extern "C" {
 
 /*
  * Arithmetic of the residual tower.
- *  LZB_FP32            Winograd F(4x4,3x3), fp32 storage, FFMA contractions: the
- *                      mode that reproduces CPUPipe to 1e-4.
+ *  LZB_FP32            Winograd F(4x4,3x3), fp32 storage, contractions in fp32
+ *                      precision on the tensor cores (three bf16 planes per
+ *                      operand): the mode that reproduces CPUPipe to 1e-4.
  *  LZB_FP16, LZB_BF16  16-bit operands on the tensor cores (tcgen05), fp32
  *                      accumulation; each 3x3 layer is one implicit-GEMM
  *                      convolution with batch-norm/residual/ReLU in its epilogue.
@@ -50,9 +51,12 @@ extern "C" {
  *                      policy and winrate differences <= 0.2,
  *                      src/Network.cpp:667-690); use LZB_FP16_X2 where the
  *                      half-precision bounds must hold for every position.
- *                      (Runs on CTA pairs; the environment variable
- *                      LZB_CONV_PAIRS=0, read at lzb_pipe_create, selects the
- *                      bit-identical single-CTA kernel for diagnostics.)
+ *                      (All layers of a batch run in one cooperative launch
+ *                      of CTA pairs; LZB_TILE_FLAGS=0, read at
+ *                      lzb_ctx_create, selects a launch per layer, and
+ *                      LZB_CONV_PAIRS=0, read at lzb_pipe_create, the
+ *                      single-CTA kernel, both bit-identical, for
+ *                      diagnostics.)
  *  LZB_*_WINOGRAD      16-bit operands on the tensor cores through the Winograd
  *                      pipeline (transform, 36 batched contractions, fused
  *                      output/input transform).  3.6x fewer multiply-adds, about
@@ -76,14 +80,7 @@ extern "C" {
  *                      network with a factor of two to spare; a network with
  *                      sharper outputs may need more blocks (30 and 8 held
  *                      them on the hardest random network tried), which is
- *                      what the counts are adjustable for.  (For batches of
- *                      more than 23 positions the layers of this mode wait for
- *                      each other tile by tile rather than launch by launch;
- *                      the environment variable LZB_TILE_FLAGS=0 / 1, read at
- *                      lzb_ctx_create, switches that off / on for any of the
- *                      direct-convolution modes; LZB_TOWER_KERNEL=1 on top
- *                      of it runs all layers of such a batch in one
- *                      cooperative launch; results are bit-identical.)
+ *                      what the counts are adjustable for.
  *  LZB_FP16_X3         activations and weights both carried as two fp16 planes
  *                      (three MMAs: hi*hi + lo*hi + hi*lo): ten times closer
  *                      to fp32 than LZB_FP16 (what remains is the accumulation
