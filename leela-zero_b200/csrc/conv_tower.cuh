@@ -16,6 +16,12 @@
 // next one, without a layer boundary that everybody waits at, so that a layer of
 // 102 units costs 102 / 74 rounds and not two.
 //
+// Small batches take 64-row tiles (kRows), six to a position and three pairs: twice
+// the pairs work on a position, and an MMA of a pair over 64 channels takes 32 cycles
+// instead of 48, which is what its operands need out of shared memory (2 + 2 KB per
+// CTA instead of 4 + 2 at 128 bytes a cycle).  20 x 256, fp16: 12,400 -> 9,800 cycles
+// a layer (5 positions 335 -> 289 us with the copies); fp16x2, 1 position 460 -> 427 us.
+//
 // Dependencies.  A row tile of layer l+1 reads, through its window, the row tiles
 // i-1, i, i+1 of its own position in layer l.  Every epilogue warp adds one to
 // the counter of its (layer, tile) once its stores have completed; the producer
@@ -28,12 +34,14 @@
 // Roles (12 warps): warp 0 polls the counters and loads activation windows, warp
 // 2 loads weights, which depend on nobody and so run ahead as far as the ring
 // allows (at the next layer's weights while this layer waits for its inputs),
-// warp 1 issues the MMAs, warps 4-11 are the epilogue of conv_direct2.cuh.
+// warp 1 issues the MMAs, warps 4-11 (4-7 with 64 rows) are the epilogue of
+// conv_direct2.cuh.
 //
 // What bounds it: with one or two units per pair the chain MMAs -> epilogue ->
-// stores -> counters -> windows (about 5,000 cycles besides the MMAs: 1,600 for
-// the stores to complete, 2,000 for the counter to arrive and be seen, 1,000 for
-// the first window); with more units per pair the tensor pipe, and over seconds
+// stores -> counters -> windows (6,300 cycles besides issuing the MMAs, 20 x 256 in
+// fp16: 1,080 from the last MMA's issue to its end, 1,250 for the epilogue and its
+// stores, 1,430 for the release of the counter, 910 until it is seen, 1,500 for the
+// first window); with more units per pair the tensor pipe, and over seconds
 // the power cap.
 //
 // Every wait is bounded; a thread that gives up sets the CTA's abort flag, all
@@ -65,9 +73,14 @@ struct alignas(64) TowerLayer {
     int pad;
 };
 
-constexpr int kTowerThreads = 384;
 constexpr int kTowerEpiWarp = 4;                        // first epilogue warp
-constexpr int kTilesPerPos128 = 3;                      // row tiles of one position
+constexpr int kRowsPerPos = 384;                        // rows computed of one position's 400 cells
+// Epilogue warps and threads of a CTA with row tiles of `rows`: two warps per
+// tensor-memory quadrant, or one (a 64-row accumulator's columns are spread over two
+// quadrants, see the epilogue).
+__host__ __device__ constexpr int tower_epi_warps(int rows) { return rows == 128 ? 8 : 4; }
+__host__ __device__ constexpr int tower_threads(int rows) { return 32 * (kTowerEpiWarp + tower_epi_warps(rows)); }
+__host__ __device__ constexpr int tower_win_rows(int rows) { return rows + 2 * kWinPad; }
 constexpr int kTowerWins = 4;                           // activation windows in flight
 constexpr uint32_t kTowerRingBytes = 96 * 1024;         // weight ring
 constexpr int kTowerMaxStages = 12;
@@ -92,9 +105,11 @@ __host__ __device__ inline int tower_taps_per_stage(int n_slice) { return n_slic
 __host__ __device__ inline int tower_stage_bytes(int n_slice) {
     return tower_taps_per_stage(n_slice) * (n_slice / 2) * 128;
 }
-// First cell of row tile i.
+// First cell of row tile i of `rows` rows.
+template <int rows>
 __host__ __device__ inline int tower_tile_row(int i) {
-    return (i / kTilesPerPos128) * kCellsPerPos + kCellsPerRow + (i % kTilesPerPos128) * kTileM;
+    constexpr int per_pos = kRowsPerPos / rows;
+    return (i / per_pos) * kCellsPerPos + kCellsPerRow + (i % per_pos) * rows;
 }
 
 __device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
@@ -186,8 +201,8 @@ struct UnitWalk {
 // run's (all zero when the kernel starts); the other one is cleared here for the
 // next run.  The number lies on the device and is raised by the head kernel, so
 // that a captured run can be replayed.
-template <typename T, int kPlanes>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTowerThreads, 1) conv_tower_kernel(
+template <typename T, int kPlanes, int kRows>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(tower_threads(kRows), 1) conv_tower_kernel(
     const __grid_constant__ CUtensorMap tmIN, const __grid_constant__ CUtensorMap tmX,
     const __grid_constant__ CUtensorMap tmH, const __grid_constant__ CUtensorMap tmXl,
     const __grid_constant__ CUtensorMap tmHl, const __grid_constant__ CUtensorMap tmXo,
@@ -195,6 +210,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTowerThreads, 1) co
     const __grid_constant__ CUtensorMap tmHlo, const TowerLayer* __restrict__ layers, int n_layers,
     const InputView input, T* IN, T* X, T* H, int ntiles, int Kp, int nsplit, int ldr,
     uint32_t* count_sets, const uint32_t* run, int tile_cap, int* err) {
+    constexpr int kTilesInPos = kRowsPerPos / kRows, kEpiWarps = tower_epi_warps(kRows);
+    constexpr uint32_t kWindow = tower_win_rows(kRows) * 128u;      // bytes of a window chunk
+    static_assert(kWindow <= kWinBytes && kWindow % 1024 == 0, "window slots");
     extern __shared__ unsigned char smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
@@ -244,14 +262,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTowerThreads, 1) co
         }
         for (int a = 0; a < 2; a++) {
             mbar_init(tfull_bar(a), 1);
-            mbar_init(tempty_bar(a), 16);    // 8 epilogue warps in each CTA
+            mbar_init(tempty_bar(a), 2 * kEpiWarps);
         }
         for (int d = 0; d < kDepRing; d++) mbar_init(dep_bar(d), 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    for (int i = blockIdx.x * kTowerThreads + threadIdx.x; i < set_words; i += gridDim.x * kTowerThreads) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < set_words; i += gridDim.x * blockDim.x) {
         counts_next[i] = 0u;
     }
     if (warp == 1) {
@@ -269,8 +287,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTowerThreads, 1) co
     const int npairs = (ntiles + 1) >> 1;
     const int units = npairs * nsplit;
     const int cid = blockIdx.x >> 1, step = gridDim.x >> 1;
-    // counter value of a finished tile: 8 epilogue warps in each CTA, per slice
-    const uint32_t complete = 16u * static_cast<uint32_t>(nsplit);
+    // counter value of a finished tile: the epilogue warps of both CTAs, per slice
+    const uint32_t complete = 2u * kEpiWarps * static_cast<uint32_t>(nsplit);
     // this CTA's row tile of unit u (the last pair of an odd count works on a copy
     // of the last tile and stores nothing)
     auto tile_of = [&](int pair) {
@@ -293,25 +311,25 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTowerThreads, 1) co
             // the row tiles this window reaches: its own and, within the position, one
             // on either side, each counted with its pair
             const uint32_t* row = counts + static_cast<size_t>(w.layer) * tile_cap;
-            const int part = tile % kTilesPerPos128;
+            const int part = tile % kTilesInPos;
             const uint32_t* mine = nullptr;
             if (lane == 0) mine = row + pair;
             if (lane == 1 && part > 0) mine = row + ((tile - 1) >> 1);
-            if (lane == 2 && part < kTilesPerPos128 - 1) mine = row + ((tile + 1) >> 1);
+            if (lane == 2 && part < kTilesInPos - 1) mine = row + ((tile + 1) >> 1);
             if (!tiles_wait(mine, complete, abort_flag, err)) break;
             bool ok = true;
             if (elect_one()) {
                 mbar_arrive(dep_bar(dep));
                 // what was counted above is read below by TMA (async proxy)
                 asm volatile("fence.proxy.async.global;" ::: "memory");
-                const int m0 = tower_tile_row(tile);
+                const int m0 = tower_tile_row<kRows>(tile);
                 for (int c = 0; c < kchunks; ++c) {
                     ok = mbar_wait(wempty_bar(wb), wphase ^ 1u, abort_flag, err, kErrTowerProducer);
                     if (!ok) break;
                     const uint32_t wf = lead_bars + (wfull_bar(wb) - bars);
-                    mbar_expect_tx_cluster(wf, kWinBytes);
+                    mbar_expect_tx_cluster(wf, kWindow);
                     const bool low8 = kPlanes == 3 && c >= fchunks;     // e5m2 chunk: byte coordinates
-                    tma_load_2d_pair(win_base + wb * kWinBytes, low8 ? in_lo : in_map,
+                    tma_load_2d_pair(win_base + wb * kWindow, low8 ? in_lo : in_map,
                                      low8 ? (c - fchunks) * 128 : (c < achunks ? c : c - achunks) * kChunkK,
                                      m0 - kWinPad, wf);
                     if (++wb == kTowerWins) { wb = 0; wphase ^= 1u; }
@@ -350,7 +368,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTowerThreads, 1) co
         // ------------------------------------------------ MMA issuer (leader CTA only)
         if (leader && elect_one()) {
             const uint32_t shape = (static_cast<uint32_t>(n_slice >> 3) << 17) |
-                                   (static_cast<uint32_t>(kPairM >> 4) << 24);
+                                   (static_cast<uint32_t>((2 * kRows) >> 4) << 24);
             const uint32_t idesc = (1u << 4) | (OperandFormat<T>::value << 7) | (OperandFormat<T>::value << 10) | shape;
             // e5m2 x e5m2 -> fp32 for the chunks of an e5m2 activation plane
             const uint32_t idesc8 = (1u << 4) | (1u << 7) | (1u << 10) | shape;
@@ -372,7 +390,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTowerThreads, 1) co
                 for (int c = 0; c < kchunks && ok; ++c) {
                     ok = mbar_wait(wfull_bar(wb), wphase, abort_flag, err, kErrTowerMmaFull);
                     if (!ok) break;
-                    const uint64_t a_win = dbase + (win16 + static_cast<uint32_t>(wb) * (kWinBytes >> 4));
+                    const uint64_t a_win = dbase + (win16 + static_cast<uint32_t>(wb) * (kWindow >> 4));
                     const bool f8 = kPlanes == 3 && c >= fchunks;
                     uint64_t b_desc = 0;
                     int left = 0;                    // taps left in the current stage
@@ -416,23 +434,27 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTowerThreads, 1) co
             }
         }
     } else if (warp >= kTowerEpiWarp) {
-        // ------------------------------------------------ epilogue (warps 4..11, both CTAs)
+        // ------------------------------------------------ epilogue (warps 4.., both CTAs)
         const int ew = warp - kTowerEpiWarp;
         const int qd = warp & 3;                 // tensor-memory lane quadrant
         const int ncols = n_slice >> 1;          // channels this warp converts per unit
-        const int wcol = (ew >> 2) * ncols;
+        // Tensor memory: 128 rows per CTA are the 128 lanes, the second four warps take the
+        // second half of the columns.  Of 64 rows per CTA (MMAs with M = 128 on the pair) the
+        // first half of the columns lies in lanes 0 .. 63, the second half in lanes 64 .. 127.
+        const int wcol = (kRows == 128 ? ew >> 2 : qd >> 1) * ncols;
+        const int wrow = (kRows == 128 ? qd : qd & 1) * 32;
         unsigned char* stg_ptr = stage_out + ew * kTowerStageOut;
         const uint32_t stg = smem_u32(stg_ptr);
         unsigned char* stg_row = stg_ptr + lane * 64;
         float* s_scale = s_bn + ew * 2 * (kMaxN / 2);
         float* s_bias = s_scale + kMaxN / 2;
-        if (ew < 4) {
+        if (ew < kRows / 32) {
             // network input: this CTA's row tile of every pair it starts with, 32 cells a
-            // warp; counted like a layer's tiles (two CTAs x four warps x 2 nsplit)
+            // warp; counted like a layer's tiles (2 nsplit for each of these warps)
             for (int pair = cid; pair < npairs; pair += step) {
                 const int t = 2 * pair + static_cast<int>(rank);
                 if (t < ntiles) {
-                    const int q = tower_tile_row(t) + ew * 32 + lane;
+                    const int q = tower_tile_row<kRows>(t) + ew * 32 + lane;
                     const int c = q % kCellsPerRow, r = (q / kCellsPerRow) % 20;
                     const bool inside = c != 0 && r != 0;
                     const int s = (r - 1) * kBoard + c - 1;
@@ -440,8 +462,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTowerThreads, 1) co
 #pragma unroll
                     for (int k = 0; k < 12; ++k) {
                         const bool use = inside && 2 * k < kInputPlanes;
-                        o[k] = pack2(T(), use ? input.at(t / kTilesPerPos128, 2 * k, s) : 0.f,
-                                     use ? input.at(t / kTilesPerPos128, 2 * k + 1, s) : 0.f);
+                        o[k] = pack2(T(), use ? input.at(t / kTilesInPos, 2 * k, s) : 0.f,
+                                     use ? input.at(t / kTilesInPos, 2 * k + 1, s) : 0.f);
                     }
                     uint4* dst = reinterpret_cast<uint4*>(IN + static_cast<size_t>(q) * 64);
 #pragma unroll
@@ -460,7 +482,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTowerThreads, 1) co
             const bool live = 2 * pair + static_cast<int>(rank) < ntiles;
             const int col0 = (w.u % nsplit) * n_slice + wcol;      // first output channel of this warp
             const int acc = local & 1;
-            const int row0 = tower_tile_row(tile_of(pair)) + qd * 32;
+            const int row0 = tower_tile_row<kRows>(tile_of(pair)) + wrow;
             const int q = row0 + lane;
             const bool interior = q % kCellsPerRow != 0 && (q / kCellsPerRow) % 20 != 0;
             // batch-norm constants of this warp's channels, before anything is waited for
@@ -502,7 +524,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTowerThreads, 1) co
             if (!ok) break;
             tcgen05_fence_after();
             const uint32_t taddr0 =
-                tmem_base + (static_cast<uint32_t>(qd * 32) << 16) + static_cast<uint32_t>(acc * kMaxN + wcol);
+                tmem_base + (static_cast<uint32_t>(qd * 32) << 16) + static_cast<uint32_t>(acc * kMaxN + (kRows == 128 ? wcol : 0));
             // batch-norm etc. of the 32-channel chunk at column j of this warp, and its store(s)
             auto emit = [&](const uint32_t (&r)[32], const uint4 (&v)[4], const uint4 (&l)[4],
                             const uint4 (&e)[2], int j) {

@@ -69,6 +69,7 @@ inline int round_up(int v, int m) { return (v + m - 1) / m * m; }
 constexpr int kXformSmem = lzb::kBoardCells * 32 * 8;   // fp32 board of one position x 64 channels
 constexpr int kMaxMicroBatch = 256;      // rows of V/M allocated: 25 * 256 = 6400
 constexpr int kDefaultMicroBatch = 64;
+constexpr int kMaxSmallTiles = 48;       // positions the tower takes in 64-row tiles at most
 constexpr int kMaxStaged = 1024;         // positions of a host call staged at a time
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
@@ -245,7 +246,8 @@ struct lzb_ctx {
     // direct path: padded cell-major activations
     int Qa = 0;            // rows allocated in IN / X / H
     void *IN = nullptr, *H = nullptr;
-    CUtensorMap tmIN, tmX, tmH;      // window loads
+    CUtensorMap tmIN, tmX, tmH;      // window loads of 128-row tiles
+    CUtensorMap tmIN64, tmX64, tmH64, tmXl64, tmHl64;    // ... and of the tower's 64-row tiles
     CUtensorMap tmXo, tmHo;          // 32 x 32 output stores
     CUtensorMap tmXl, tmHl;          // e5m2 planes of X and H: 128-byte windows (LZB_FP16_X2)
     CUtensorMap tmXlo, tmHlo;        // ... and their 32 x 32 output stores
@@ -613,27 +615,45 @@ int launch_conv_direct(lzb_ctx* c, const Layer& L, int nb, const CUtensorMap& tm
     return LZB_OK;
 }
 
-// Channel slices of a tile in the one-launch tower.  An MMA of 256 x N x 16 takes
-// 44, 65, 97, 129 cycles at N = 64, 128, 192, 256 (measured), so slices shorten a
-// unit less than they multiply their number: with units to spare they pay only
-// while pairs are idle.  Cost of a layer in cycles: one unit's MMAs plus the chain
-// between layers (some 5,000 cycles), or the pairs' share of all units' MMAs,
-// whichever is longer; the fewest slices within 3 % of the best, since every
-// slice loads the activation windows again.
-int tower_slices(const lzb_pipe* p, int npairs) {
+// Rows of a CTA's tile and channel slices of a tile in the one-launch tower.
+struct TowerPlan {
+    int rows, slices;
+};
+// 64-row tiles with 64-channel slices while that makes at most 1.5 units for every
+// resident pair (2 where activations are one plane): a 128 x 64 x 16 MMA of a pair takes
+// 32 cycles instead of 48 (its operands' way out of shared memory), but its tile loads
+// twice the weights per row.  Measured, 20 x 256 in fp16, 5 / 12 / 16 positions (0.8 /
+// 1.9 / 2.6 units a pair): 296 -> 255, 326 -> 277, 322 -> 345 us; fp16x2, 8 / 12: 467 ->
+// 424, 486 -> 561; 15 x 192 fp16x2, 12 / 16 (1.5 / 1.9): 323 -> 291, 335 -> 362.
+// Else 128 rows, where an MMA of 256 x N x 16 takes 44, 65, 97, 129 cycles at N = 64,
+// 128, 192, 256: slices shorten a unit less than they multiply their number, and pay
+// only while pairs are idle.  Cost of a layer in cycles: one unit's MMAs plus the chain
+// between layers (measured 6,500, 7,500 with a second plane to store), or the pairs'
+// share of all units' MMAs, whichever is longer; the fewest slices within 3 % of the
+// best, since every slice loads the activation windows again.
+TowerPlan tower_plan(const lzb_pipe* p, int nb, int tile_cap) {
+    const int most = p->Cp / 64;                    // slices of 64 channels, at most 4 (Cp <= 256)
+    const int small_units = 3 * nb * most;
+    if (3 * nb <= tile_cap && p->tower_table[most] != nullptr &&
+        2 * small_units <= (p->aplanes == 1 ? 4 : 3) * p->tower_pairs) {
+        return {64, most};
+    }
     auto mma_cycles = [](int n) { return n <= 64 ? 44.0 : n * 0.5 + 1.0; };
-    const double mmas = 36.0 * p->layers.back().cinw / tc::kChunkK;
+    long long chunks = 0;
+    for (const Layer& L : p->layers) chunks += L.cinw / tc::kChunkK + L.lchunks;
+    const double mmas = 36.0 * chunks / p->layers.size(), chain = p->aplanes == 1 ? 6500.0 : 7500.0;
+    const int npairs = (3 * nb + 1) / 2;
     double cost[5] = {0, 0, 0, 0, 0}, best = 1e30;
     for (int ns = 1; ns <= 4; ns++) {
         if (p->tower_table[ns] == nullptr) continue;
         const double unit = mmas * mma_cycles(p->Cp / ns);
-        cost[ns] = std::max(unit + 5000.0, unit * npairs * ns / p->tower_pairs);
+        cost[ns] = std::max(unit + chain, unit * npairs * ns / p->tower_pairs);
         best = std::min(best, cost[ns]);
     }
     for (int ns = 1; ns <= 4; ns++) {
-        if (p->tower_table[ns] != nullptr && cost[ns] <= 1.03 * best) return ns;
+        if (p->tower_table[ns] != nullptr && cost[ns] <= 1.03 * best) return {128, ns};
     }
-    return 1;
+    return {128, 1};
 }
 
 // All 3x3 layers of one micro-batch in one cooperative launch.  A launch that is
@@ -641,12 +661,13 @@ int tower_slices(const lzb_pipe* p, int npairs) {
 template <typename T>
 int launch_tower(lzb_ctx* c, const InputView& in, int nb, bool* refused) {
     lzb_pipe* p = c->pipe;
-    const int ntiles = dct::kTilesPerPos128 * nb, npairs = (ntiles + 1) / 2;
-    const int ns = tower_slices(p, npairs);
+    const TowerPlan plan = tower_plan(p, nb, c->tile_cap);
+    const bool tall = plan.rows == 128;
+    const int ns = plan.slices, ntiles = dct::kRowsPerPos / plan.rows * nb, npairs = (ntiles + 1) / 2;
     const int n_layers = static_cast<int>(p->layers.size());
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * std::min(npairs * ns, p->tower_pairs));
-    cfg.blockDim = dim3(dct::kTowerThreads);
+    cfg.blockDim = dim3(dct::tower_threads(plan.rows));
     cfg.dynamicSmemBytes = dct::kTowerSmemBytes;
     cfg.stream = c->stream;
     cudaLaunchAttribute attr[1];
@@ -654,15 +675,20 @@ int launch_tower(lzb_ctx* c, const InputView& in, int nb, bool* refused) {
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    auto kernel = dct::conv_tower_kernel<T, 1>;
-    if (p->aplanes == 2) kernel = dct::conv_tower_kernel<T, 2>;
+    auto kernel = tall ? dct::conv_tower_kernel<T, 1, 128> : dct::conv_tower_kernel<T, 1, 64>;
+    if (p->aplanes == 2) kernel = tall ? dct::conv_tower_kernel<T, 2, 128> : dct::conv_tower_kernel<T, 2, 64>;
     if constexpr (std::is_same<T, __half>::value) {     // the e5m2 planes accompany fp16 only
-        if (p->aplanes == 3) kernel = dct::conv_tower_kernel<T, 3>;
+        if (p->aplanes == 3) kernel = tall ? dct::conv_tower_kernel<T, 3, 128> : dct::conv_tower_kernel<T, 3, 64>;
     }
+    // windows of the tile's height; the e5m2 ones only matter to the e5m2 variant
+    const CUtensorMap& in_map = tall ? c->tmIN : c->tmIN64;
+    const CUtensorMap& x_map = tall ? c->tmX : c->tmX64;
+    const CUtensorMap& h_map = tall ? c->tmH : c->tmH64;
     const bool bytes = p->aplanes == 3;
     LaunchScope scope(c, kClassContraction, n_layers);
     cudaError_t le = cudaLaunchKernelEx(
-        &cfg, kernel, c->tmIN, c->tmX, c->tmH, bytes ? c->tmXl : c->tmX, bytes ? c->tmHl : c->tmH, c->tmXo, c->tmHo,
+        &cfg, kernel, in_map, x_map, h_map, bytes ? (tall ? c->tmXl : c->tmXl64) : x_map,
+        bytes ? (tall ? c->tmHl : c->tmHl64) : h_map, c->tmXo, c->tmHo,
         bytes ? c->tmXlo : c->tmXo, bytes ? c->tmHlo : c->tmHo, (const dct::TowerLayer*)p->tower_table[ns], n_layers, in,
         static_cast<T*>(c->IN), static_cast<T*>(c->X), static_cast<T*>(c->H), ntiles, p->Cp, ns, p->row_bytes() / p->elt,
         c->tile_counts, (const uint32_t*)c->tower_runs(), c->tile_cap, c->d_err);
@@ -780,9 +806,13 @@ int set_smem_attrs() {
     }
     {
         const void* variants[] = {
-            (const void*)dct::conv_tower_kernel<__half, 1>, (const void*)dct::conv_tower_kernel<__half, 2>,
-            (const void*)dct::conv_tower_kernel<__half, 3>, (const void*)dct::conv_tower_kernel<__nv_bfloat16, 1>,
-            (const void*)dct::conv_tower_kernel<__nv_bfloat16, 2>};
+            (const void*)dct::conv_tower_kernel<__half, 1, 128>, (const void*)dct::conv_tower_kernel<__half, 1, 64>,
+            (const void*)dct::conv_tower_kernel<__half, 2, 128>, (const void*)dct::conv_tower_kernel<__half, 2, 64>,
+            (const void*)dct::conv_tower_kernel<__half, 3, 128>, (const void*)dct::conv_tower_kernel<__half, 3, 64>,
+            (const void*)dct::conv_tower_kernel<__nv_bfloat16, 1, 128>,
+            (const void*)dct::conv_tower_kernel<__nv_bfloat16, 1, 64>,
+            (const void*)dct::conv_tower_kernel<__nv_bfloat16, 2, 128>,
+            (const void*)dct::conv_tower_kernel<__nv_bfloat16, 2, 64>};
         for (const void* k : variants) {
             LZB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, dct::kTowerSmemBytes));
         }
@@ -807,10 +837,10 @@ int head_resident_clusters() {
 int tower_resident_pairs() {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2);
-    cfg.blockDim = dim3(dct::kTowerThreads);
+    cfg.blockDim = dim3(dct::tower_threads(128));
     cfg.dynamicSmemBytes = dct::kTowerSmemBytes;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, dct::conv_tower_kernel<__half, 3>, &cfg) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&n, dct::conv_tower_kernel<__half, 3, 128>, &cfg) != cudaSuccess) {
         (void)cudaGetLastError();
         return 0;
     }
@@ -1425,7 +1455,7 @@ int lzb_ctx_create(lzb_ctx** out, lzb_pipe* p, int max_batch) {
         // (cross-check and diagnostics).
         const char* tf = getenv("LZB_TILE_FLAGS");
         if (p->tower_pairs > 0 && !(tf != nullptr && atoi(tf) == 0)) {
-            c->tile_cap = (dct::kTilesPerPos128 * c->micro_cap + 1) / 2;
+            c->tile_cap = std::max((3 * c->micro_cap + 1) / 2, 3 * std::min(c->micro_cap, kMaxSmallTiles));
             alloc((void**)&c->tile_counts, (c->tile_count_words() + 1) * sizeof(uint32_t));
         }
     } else {
@@ -1456,13 +1486,17 @@ int lzb_ctx_create(lzb_ctx** out, lzb_pipe* p, int max_batch) {
     }
     *c->h_err = 0;
     if (p->direct) {
+        const uint32_t win64 = dct::tower_win_rows(64);
         int rc = make_map_2d(&c->tmIN, p->precision, c->IN, (uint64_t)c->Qa, 64, dc::kWinRows);
+        if (!rc) rc = make_map_2d(&c->tmIN64, p->precision, c->IN, (uint64_t)c->Qa, 64, win64);
         // 16-bit channels of a cell row (hi [+ 16-bit lo] plane) and the row pitch
         const uint64_t xp = (uint64_t)p->Cp * (p->aplanes == 2 ? 2 : 1);
         const uint64_t pitch = p->row_bytes();
         const CUtensorMapSwizzle sw128 = CU_TENSOR_MAP_SWIZZLE_128B, sw64 = CU_TENSOR_MAP_SWIZZLE_64B;
         if (!rc) rc = make_map_2d(&c->tmX, p->precision, c->X, (uint64_t)c->Qa, xp, dc::kWinRows, 64, sw128, pitch);
         if (!rc) rc = make_map_2d(&c->tmH, p->precision, c->H, (uint64_t)c->Qa, xp, dc::kWinRows, 64, sw128, pitch);
+        if (!rc) rc = make_map_2d(&c->tmX64, p->precision, c->X, (uint64_t)c->Qa, xp, win64, 64, sw128, pitch);
+        if (!rc) rc = make_map_2d(&c->tmH64, p->precision, c->H, (uint64_t)c->Qa, xp, win64, 64, sw128, pitch);
         if (!rc) rc = make_map_2d(&c->tmXo, p->precision, c->X, (uint64_t)c->Qa, xp, 32, 32, sw64, pitch);
         if (!rc) rc = make_map_2d(&c->tmHo, p->precision, c->H, (uint64_t)c->Qa, xp, 32, 32, sw64, pitch);
         if (p->aplanes == 3) {
@@ -1473,6 +1507,8 @@ int lzb_ctx_create(lzb_ctx** out, lzb_pipe* p, int max_batch) {
             const uint64_t lb = (uint64_t)p->Cp * (p->wlo_layers > 1 ? 2 : 1);
             if (!rc) rc = make_map_2d(&c->tmXl, -1, xl, (uint64_t)c->Qa, lb, dc::kWinRows, 128, sw128, pitch);
             if (!rc) rc = make_map_2d(&c->tmHl, -1, hl, (uint64_t)c->Qa, lb, dc::kWinRows, 128, sw128, pitch);
+            if (!rc) rc = make_map_2d(&c->tmXl64, -1, xl, (uint64_t)c->Qa, lb, win64, 128, sw128, pitch);
+            if (!rc) rc = make_map_2d(&c->tmHl64, -1, hl, (uint64_t)c->Qa, lb, win64, 128, sw128, pitch);
             const CUtensorMapSwizzle sw0 = CU_TENSOR_MAP_SWIZZLE_NONE;
             if (!rc) rc = make_map_2d(&c->tmXlo, -1, xl, (uint64_t)c->Qa, lb, 32, 32, sw0, pitch);
             if (!rc) rc = make_map_2d(&c->tmHlo, -1, hl, (uint64_t)c->Qa, lb, 32, 32, sw0, pitch);

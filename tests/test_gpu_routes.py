@@ -20,9 +20,9 @@ def _same(a, b):
 @pytest.mark.parametrize("filters", [32, 96, 192, 256])
 @pytest.mark.parametrize("mode", ["fp16", "bf16", "fp16x2", "fp16x3", "bf16x3"])
 def test_tower_gives_the_bits_of_a_launch_per_layer(lzb, W, monkeypatch, mode, filters):
-    """One position is three row tiles (an odd count: the last pair works on a
-    copy), 25 positions are just more units than CTA pairs; the number of slices
-    falls from 4 to 1 along these batches.  Every output is the same sum in the
+    """Up to 9 or 12 positions of 256 filters, more of narrower networks, run in
+    64-row tiles.  Above, one position is three row tiles (an odd count: the last
+    pair works on a copy) and the number of slices falls from 4 to 1.  Every output is the same sum in the
     same order as with a launch per layer, whatever batch came before it on the
     context."""
     net = W.synthetic_network(5, filters, 2200 + filters, calibrated=True)
@@ -32,7 +32,7 @@ def test_tower_gives_the_bits_of_a_launch_per_layer(lzb, W, monkeypatch, mode, f
     layers = pipe.context(80)
     monkeypatch.delenv("LZB_TILE_FLAGS")
     tower = pipe.context(80)
-    for n in (1, 2, 80, 3, 11, 25, 37, 1, 49):
+    for n in (1, 2, 80, 3, 8, 9, 12, 13, 25, 37, 1, 49):
         assert _same(tower.forward(x[:n]), layers.forward(x[:n])), n
     before = tower.launches
     tower.forward(x)
