@@ -1393,10 +1393,10 @@ int lzb_pipe_finalize(lzb_pipe* p) {
     return LZB_OK;
 }
 
-// Positions per pass through the tower.  Direct convolution: the whole batch.
-// Winograd pipeline: V and M of one micro-batch should stay in L2 (64 positions
-// x 256 channels = 2 x 29 MB in 16 bits); in the 16-bit modes the fused
-// transform runs one CTA per SM (25 warps), so the count is raised to the next
+// Positions per pass through the tower.  Direct convolution and fp32: the whole
+// batch.  16-bit Winograd pipeline: V and M of one micro-batch should stay in L2
+// (64 positions x 256 channels = 2 x 29 MB), and the fused transform runs one CTA
+// per SM (25 warps), so the count is raised to the next
 // one that makes its grid, (channels / 64) x positions, whole waves of the SMs
 // (74 for 256 channels on 148 SMs: +10 % measured against 64).
 static int default_micro_batch(const lzb_pipe* p, int cap) {
@@ -1408,16 +1408,11 @@ static int default_micro_batch(const lzb_pipe* p, int cap) {
             if ((groups * cand) % p->sm_count == 0) { n = cand; break; }
         }
     } else {
-        // fp32: of the counts from 64 down to 40, the one whose items (256 rows x 128
-        // channels, CTA pairs) fill their last wave best
-        double best = 0.0;
-        const int pairs = p->sm_count / 2;
-        for (int cand = kDefaultMicroBatch; cand >= 40; cand--) {
-            const int items = round_up(cand * kTilesPerPos, 256) / 256 * ((p->Cp + 127) / 128) * kPoints;
-            const int waves = (items + pairs - 1) / pairs;
-            const double rate = static_cast<double>(cand) / waves;     // positions per wave
-            if (rate > best * 1.02) { best = rate; n = cand; }
-        }
+        // fp32: the whole batch.  V and M of 64 positions at 256 channels are past L2 already,
+        // and fewer, larger launches fill their waves better: 77 positions of 10 x 128 in
+        // 61 + 16 / at once 1098 / 948 us, 128 of 20 x 256 in 64s 7932 / 7256, 256 of
+        // 6 x 64 in 64s 1104 / 973, 100 of 10 x 160 in 50s 2578 / 2585.
+        n = kMaxMicroBatch;
     }
     return n < cap ? n : cap;
 }

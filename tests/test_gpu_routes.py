@@ -63,8 +63,8 @@ def _forward64(net, x):
 @pytest.mark.parametrize("filters", [40, 64, 128, 192, 320])
 def test_fp32_contraction_is_closer_to_64_bits_than_the_fma_chain(lzb, oracle, W, filters):
     """Rows of a batch: 25 and 125 (single CTAs), 150 (a pair whose second CTA
-    has 22 rows), 275 and 525 (pairs whose second CTA has none), 2000 (cut into
-    micro-batches at 40 positions and more).  The oracle does the same Winograd
+    has 22 rows), 275 and 525 (pairs whose second CTA has none), 2000 (more
+    items than pairs).  The oracle does the same Winograd
     arithmetic with its contractions as one chain of fp32 additions; three bf16
     planes must not be further from the 64-bit result than that (5 % for the
     rounding of the transforms, which both share)."""
