@@ -432,7 +432,11 @@ int launch_xform(lzb_ctx* c, const Layer& L, int nb, const T* R, T* X_out, VType
         if constexpr (std::is_same<T, float>::value) {
             cfg.gridDim = dim3(p->Cp / kXf32Chan, nb);
             cfg.blockDim = dim3(kXf32Threads);
-            le = cudaLaunchKernelEx(&cfg, xform_f32_kernel, static_cast<const float*>(c->M), c->Pa, p->Cp,
+            // see the kernel: three CTAs an SM where that takes fewer waves than two
+            const int ctas = p->Cp / kXf32Chan * nb, sms = p->sm_count;
+            const bool three = (ctas + 3 * sms - 1) / (3 * sms) < (ctas + 2 * sms - 1) / (2 * sms);
+            auto kernel = three ? xform_f32_kernel<3> : xform_f32_kernel<2>;
+            le = cudaLaunchKernelEx(&cfg, kernel, static_cast<const float*>(c->M), c->Pa, p->Cp,
                                     (const float*)L.mean, (const float*)L.invstd, R, X_out, V);
         } else {
             cfg.gridDim = dim3(p->Cp / kChanPerCta, nb);
@@ -1836,8 +1840,8 @@ int lzb_conv3x3_static(int device, const float* in_dev, int n, int c_in, int cha
         nchw_to_nhwc_kernel<float><<<128, 256, 0, stream>>>(residual_dev, X, n, channels, Cp);
         R = X;
     }
-    xform_f32_kernel<<<dim3(Cp / kXf32Chan, n), kXf32Threads, 0, stream>>>(M, kStaticRows, Cp, bn, bn + 64, R, X,
-                                                                          nullptr);
+    xform_f32_kernel<2><<<dim3(Cp / kXf32Chan, n), kXf32Threads, 0, stream>>>(M, kStaticRows, Cp, bn, bn + 64, R, X,
+                                                                             nullptr);
     nhwc_to_nchw_kernel<float><<<128, 256, 0, stream>>>(X, out_dev, n, channels, Cp);
     LZB_CUDA(cudaGetLastError());
     return LZB_OK;

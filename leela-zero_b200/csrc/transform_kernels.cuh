@@ -269,9 +269,13 @@ __global__ void __launch_bounds__(XformShape<T>::warps * 32, XformShape<T>::ctas
 // one pass of 200 threads takes the whole plane and a single position at 256
 // channels already fills 16 CTAs (with 64 channels per CTA and 8 warps walking
 // over the tiles it was 4 CTAs of 25 us).  A row segment of a CTA is 64 bytes of M
-// and 32 of each plane of V: whole sectors.  All 36 loads of a thread are in flight
-// at once.  Board cells are 80 bytes apart, so that the two tiles of a half warp
+// and 32 of each plane of V: whole sectors.  Board cells are 80 bytes apart, so that the two tiles of a half warp
 // (four cells apart) use different banks.
+// kResident CTAs share an SM: two, with a thread's 36 loads in 72 registers, or three
+// (80 registers in all, loads in smaller groups) where the grid then takes fewer
+// waves of the 148 SMs.  Evaluations with two / three: 10 x 128, 40 positions (320
+// CTAs, 2 / 1 waves) 531 / 514 us, 77 (616, 3 / 2) 945 / 916; 20 x 256, 61 (976, 4 / 3)
+// 3470 / 3428, but 16 (256, 1 / 1) 1040 / 1170 and 32 (512, 2 / 2) 1900 / 1916.
 // grid (Cp/16, n), block 200.  Values and order of operations are those of
 // xform_kernel with Pair<float>: multiplies and adds as the CPU pipe has them.
 // ---------------------------------------------------------------------------
@@ -279,7 +283,8 @@ constexpr int kXf32Chan = 16;
 constexpr int kXf32Threads = kTilesPerPos * (kXf32Chan / 2);
 constexpr int kXf32Cell = 10;                 // float2 per board cell: 8 used
 
-__global__ void __launch_bounds__(kXf32Threads, 2) xform_f32_kernel(
+template <int kResident>
+__global__ void __launch_bounds__(kXf32Threads, kResident) xform_f32_kernel(
     const float* M, int Pa, int Cp, const float* __restrict__ bn_mean, const float* __restrict__ bn_invstd,
     const float* R, float* X_out, __nv_bfloat16* __restrict__ V) {
     __shared__ float2 board[kBoardCells * kXf32Cell];
