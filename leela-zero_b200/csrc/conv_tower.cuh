@@ -190,12 +190,13 @@ struct UnitWalk {
     }
 };
 
-// tmIN, tmX, tmH : activation windows (box 64 x kWinRows); tmXl, tmHl : their
-// e5m2 planes (byte maps, box 128 x kWinRows); tmXo, tmHo : output tiles (box
+// tmIN, tmX, tmH : activation windows (box 64 x tower_win_rows(kRows)); tmXl, tmHl :
+// their e5m2 planes (byte maps, box 128 x the same); tmXo, tmHo : output tiles (box
 // 32 x 32, 64-byte swizzle), tmXlo, tmHlo : byte-plane output tiles (box 32 x 32,
 // the e5m2 plane from byte 0, the hi8 plane from byte Kp).  X, H : the two
-// activation tensors, ldr elements of T per cell row.  input : the network input, converted here into IN (64 channels of T per cell row,
-// channels 24 .. 63 zero beforehand).  ntiles row tiles (three per position),
+// activation tensors, ldr elements of T per cell row.  input : the network input,
+// converted here into IN (64 channels of T per cell row, channels 24 .. 63 zero
+// beforehand).  ntiles row tiles of kRows cells (three or six per position),
 // nsplit slices.  count_sets : two sets of [n_layers + 1][tile_cap] words, row l for
 // the tiles layer l reads.  *run, the number of runs so far, says which set is this
 // run's (all zero when the kernel starts); the other one is cleared here for the

@@ -4,11 +4,13 @@
 // filters U[36][Kp][Cin_p] in the tower's storage type plus fp32 batch-norm
 // vectors, and the two 1x1 head filters.  A context holds a stream and the
 // activation buffers (V, M, X) sized for one micro-batch; a batch is pushed
-// through the whole tower one micro-batch at a time so that V and M, the two
-// large tensors every layer writes and reads once, stay resident in L2.
+// through the whole tower one micro-batch at a time (up to 256 positions; fewer in
+// the 16-bit Winograd modes, whose V and M, the two large tensors every layer
+// writes and reads once, then stay resident in L2).
 //
-// Per 3x3 layer two kernels run: the channel contractions (tcgen05 or FFMA)
-// and the fused output-transform / batch-norm / residual / ReLU / next input
+// Direct-convolution modes run all 3x3 layers in one launch (conv_tower.cuh).  In
+// the Winograd modes two kernels run per layer: the channel contractions (tcgen05;
+// fp32 operands as three bf16 planes) and the fused output-transform / batch-norm / residual / ReLU / next input
 // transform.  The sequence mirrors OpenCL_Network::forward
 // (src/OpenCL.cpp:143-329) and CPUPipe::forward (src/CPUPipe.cpp:379-428).
 #include "../../include/lzb200.h"

@@ -22,9 +22,9 @@ def _same(a, b):
 def test_tower_gives_the_bits_of_a_launch_per_layer(lzb, W, monkeypatch, mode, filters):
     """Up to 9 or 12 positions of 256 filters, more of narrower networks, run in
     64-row tiles.  Above, one position is three row tiles (an odd count: the last
-    pair works on a copy) and the number of slices falls from 4 to 1.  Every output is the same sum in the
-    same order as with a launch per layer, whatever batch came before it on the
-    context."""
+    pair works on a copy) and the number of slices falls from 4 to 1.  Every
+    output is the same sum in the same order as with a launch per layer, whatever
+    batch came before it on the context."""
     net = W.synthetic_network(5, filters, 2200 + filters, calibrated=True)
     x = W.synthetic_positions(80, 1200)
     pipe = lzb.Pipe(net, mode)
